@@ -140,18 +140,27 @@ __global__ void __launch_bounds__(256) k_gemm(GemmArgs g) {
 }
 
 // ---------------- truncated DFT along y and the mode mix ----------------
-// out[b][r][kx] = sum_y F[r][y] in[b][y][kx]
-__global__ void k_fy_fwd(const float2 *__restrict__ in, float2 *__restrict__ out, const float2 *__restrict__ F, int NB,
-                         int N, int M, int KY) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)NB * KY * M) return;
-  const int kx = idx % M, r = (idx / M) % KY;
-  const long long b = idx / ((long long)M * KY);
-  const float2 *src = in + b * N * M + kx;
-  const float2 *f = F + (size_t)r * N;
+// out[b][r][kx] = sum_y F[r][y] in[b][y][kx]; grid (blocks of 256 outputs (r, kx),
+// NB).  A block stages fy_rows rows of its in[b] at a time in shared memory: one
+// thread an output straight from global memory walked N rows 8 M bytes apart, 59
+// us against 9 at 128 x 256 rows of 12 modes.
+__host__ __device__ inline int fy_rows(int M) { return M >= 5632 ? 1 : M > 88 ? 5632 / M : 64; }  // <= 64 KB
+__global__ void __launch_bounds__(256) k_fy_fwd(const float2 *__restrict__ in, float2 *__restrict__ out,
+                                                const float2 *__restrict__ F, int N, int M, int KY) {
+  extern __shared__ float2 rows[];  // [fy_rows(M)][M]
+  const int step = fy_rows(M);
+  const int o = blockIdx.x * 256 + threadIdx.x, kx = o % M, r = o / M;
+  const float2 *src = in + (size_t)blockIdx.y * N * M, *f = F + (size_t)(r < KY ? r : 0) * N;
   float2 acc = make_float2(0.f, 0.f);
-  for (int y = 0; y < N; y++) cfma(acc, __ldg(&f[y]), src[(size_t)y * M]);
-  out[(b * KY + r) * M + kx] = acc;
+  for (int y0 = 0; y0 < N; y0 += step) {
+    const int ny = min(step, N - y0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < ny * M; e += 256) rows[e] = src[(size_t)y0 * M + e];
+    __syncthreads();
+#pragma unroll 8
+    for (int y = 0; y < ny; y++) cfma(acc, __ldg(&f[y0 + y]), rows[y * M + kx]);
+  }
+  if (r < KY) out[((size_t)blockIdx.y * KY + r) * M + kx] = acc;
 }
 
 // out[b][y][kx] = sum_r conj(F[r][y]) in[b][r][kx]
@@ -174,28 +183,30 @@ __device__ __forceinline__ float2 wround(float2 w, int bf16) {
               : w;
 }
 
-// Y[s][o][k] = sum_c R[k][o][c] X[s][c][k]
-__global__ void k_mix_fwd(const float2 *__restrict__ X, const float2 *__restrict__ R, float2 *__restrict__ Y, int S,
-                          int C, int NM, int bf16) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= S * C * NM) return;
-  const int k = idx % NM, o = (idx / NM) % C, s = idx / (NM * C);
-  float2 acc = make_float2(0.f, 0.f);
-  for (int c = 0; c < C; c++)
-    cfma(acc, wround(__ldg(&R[((size_t)k * C + o) * C + c]), bf16), X[((size_t)s * C + c) * NM + k]);
-  Y[((size_t)s * C + o) * NM + k] = acc;
-}
-
-// dX[s][c][k] = sum_o conj(R[k][o][c]) dY[s][o][k]
-__global__ void k_mix_bwd_x(const float2 *__restrict__ dY, const float2 *__restrict__ R, float2 *__restrict__ dX, int S,
-                            int C, int NM, int bf16) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= S * C * NM) return;
-  const int k = idx % NM, c = (idx / NM) % C, s = idx / (NM * C);
-  float2 acc = make_float2(0.f, 0.f);
-  for (int o = 0; o < C; o++)
-    cfma(acc, cconj(wround(__ldg(&R[((size_t)k * C + o) * C + c]), bf16)), dY[((size_t)s * C + o) * NM + k]);
-  dX[((size_t)s * C + c) * NM + k] = acc;
+// Y[s][o][k] = sum_c R[k][o][c] X[s][c][k], or with adjoint the transpose
+// Y[s][c][k] = sum_o conj(R[k][o][c]) X[s][o][k].  One block per mode k: its
+// C x C weights are contiguous, its inputs S C values NM apart; both are staged
+// in shared memory (a thread an output straight from global memory read the
+// weights 8 C^2 bytes apart between lanes: 18 and 27 us against 5 at C = 32).
+__global__ void __launch_bounds__(128) k_mix(const float2 *__restrict__ X, const float2 *__restrict__ R,
+                                             float2 *__restrict__ Y, int S, int C, int NM, int bf16, int adjoint) {
+  extern __shared__ float2 sm[];
+  float2 *w = sm, *xs = sm + C * (C + 1);  // [o][C + 1], [S][C]
+  const int k = blockIdx.x;
+  for (int e = threadIdx.x; e < C * C; e += blockDim.x)
+    w[e / C * (C + 1) + e % C] = wround(__ldg(&R[(size_t)k * C * C + e]), bf16);
+  for (int e = threadIdx.x; e < S * C; e += blockDim.x) xs[e] = X[(size_t)e * NM + k];
+  __syncthreads();
+  for (int e = threadIdx.x; e < S * C; e += blockDim.x) {
+    const int a = e % C;
+    const float2 *xr = xs + e / C * C;
+    float2 acc = make_float2(0.f, 0.f);
+    if (adjoint)
+      for (int o = 0; o < C; o++) cfma(acc, cconj(w[o * (C + 1) + a]), xr[o]);
+    else
+      for (int c = 0; c < C; c++) cfma(acc, w[a * (C + 1) + c], xr[c]);
+    Y[(size_t)e * NM + k] = acc;
+  }
 }
 
 // dR[k][o][c] += sum_s dY[s][o][k] conj(X[s][c][k])
@@ -256,14 +267,14 @@ __global__ void k_act_bwd(float *__restrict__ dv, const float *__restrict__ h, l
   if (idx < n) dv[idx] *= gelu_d(h[idx]);
 }
 
-// db[o] += sum_{s,p} d[s][o][p]; grid (C, blocks over S*P)
-__global__ void k_bias_grad(const float *__restrict__ d, float *__restrict__ db, int S, int C, int P) {
+// db[o] += sum_{s,p} d[s][o][p]; grid (C, blocks over P, S)
+__global__ void __launch_bounds__(256) k_bias_grad(const float *__restrict__ d, float *__restrict__ db, int C, int P) {
   const int o = blockIdx.x;
+  const float4 *row = (const float4 *)(d + ((size_t)blockIdx.z * C + o) * P);  // P is a multiple of 64
   float acc = 0.f;
-  for (long long e = (long long)blockIdx.y * blockDim.x + threadIdx.x; e < (long long)S * P;
-       e += (long long)gridDim.y * blockDim.x) {
-    const int s = e / P, p = e % P;
-    acc += d[((size_t)s * C + o) * P + p];
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < P / 4; e += gridDim.y * blockDim.x) {
+    const float4 v = __ldg(row + e);
+    acc += (v.x + v.y) + (v.z + v.w);
   }
   for (int w = 16; w > 0; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
   __shared__ float red[8];
@@ -580,7 +591,17 @@ void gemm(const FnoModel &F, cudaStream_t st, int batch, int M, int N, int K, co
   k_gemm<<<dim3((N + kGT - 1) / kGT, (M + kGT - 1) / kGT, batch * ksplit), 256, 0, st>>>(g);
 }
 
-int ksplit_for(long long K) { return (int)std::max<long long>(1, std::min<long long>(256, K / 4096)); }
+// K per CTA of the weight gradients, whose K is every pixel and whose M x N is one
+// tile: 1024 keeps every SM at work from 256 x 256 pixels on (4096 left 64 CTAs of
+// 64 stages each, 158 us a product of a 4-sample batch there).
+int ksplit_for(long long K) { return (int)std::max<long long>(1, std::min<long long>(256, K / 1024)); }
+
+dim3 bias_grid(int C, int P, int n) { return dim3(C, std::max(1, std::min(P / 4096, 2048 / (C * n))), n); }
+size_t mix_smem(int C, int S) { return ((size_t)C * (C + 1) + (size_t)S * C) * sizeof(float2); }
+void fy_fwd(const float2 *in, float2 *out, const FnoModel &F, int n, cudaStream_t st) {
+  k_fy_fwd<<<dim3((F.KY * F.M + 255) / 256, n * F.C), 256, (size_t)fy_rows(F.M) * F.M * sizeof(float2), st>>>(
+      in, out, F.Fy, F.N, F.M, F.KY);
+}
 
 uint64_t mix64(uint64_t &s) {
   uint64_t z = (s += 0x9E3779B97F4A7C15ull);
@@ -678,6 +699,9 @@ isg_status fno_create(isg_ctx *c, const isg_fno_opts *o) {
   if (F->tensor &&
       (e = ck(cudaFuncSetAttribute(bf::k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmem))))
     return e;
+  if ((e = ck(cudaFuncSetAttribute(k_mix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mix_smem(128, 64)))) ||
+      (e = ck(cudaFuncSetAttribute(k_fy_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * (int)sizeof(float2)))))
+    return e;  // the largest of any model: the attribute is the function's, not the context's
   const size_t act = (size_t)S * C * P;
   F->v.assign(L + 1, nullptr);
   F->h.assign(L, nullptr);
@@ -732,9 +756,8 @@ void fno_forward(isg_ctx *c, int n, int g_per_sample, cudaStream_t st) {
   for (int l = 0; l < F.L; l++) {
     const int rows = n * C * N;
     gemm(F, st, 1, rows, 2 * M, N, F.v[l], N, 1, 0, F.Ex, 2 * M, 1, 0, F.T, 2 * M, 1, 0, 0);
-    k_fy_fwd<<<blocks((long long)n * C * KY * M), 256, 0, st>>>((const float2 *)F.T, F.X[l], F.Fy, n * C, N, M, KY);
-    k_mix_fwd<<<blocks((long long)n * C * NM), 256, 0, st>>>(F.X[l], (const float2 *)(W + F.off_R[l]), F.Y, n, C, NM,
-                                                             F.tensor);
+    fy_fwd((const float2 *)F.T, F.X[l], F, n, st);
+    k_mix<<<NM, 128, mix_smem(C, n), st>>>(F.X[l], (const float2 *)(W + F.off_R[l]), F.Y, n, C, NM, F.tensor, 0);
     k_fy_inv<<<blocks((long long)n * C * N * M), 256, 0, st>>>(F.Y, (float2 *)F.Z, F.Fy, n * C, N, M, KY);
     count_launch(3);
     gemm(F, st, 1, rows, N, 2 * M, F.Z, 2 * M, 1, 0, F.Ix, N, 1, 0, F.spec, N, 1, 0, 0);
@@ -761,7 +784,7 @@ void fno_backward(isg_ctx *c, int n, cudaStream_t st) {
   const long long IP = (long long)kFnoIn * P;
   gemm(F, st, n, 2, C, P, F.dout, P, 1, 2LL * P, F.v[F.L], 1, P, CP, G + F.off_Wp, C, 1, 0, 2, ks);
   gemm(F, st, n, 2, kFnoIn, P, F.dout, P, 1, 2LL * P, F.in, 1, P, IP, G + F.off_Ws, kFnoIn, 1, 0, 2, ks);
-  k_bias_grad<<<dim3(2, 64), 256, 0, st>>>(F.dout, G + F.off_bp, n, 2, P);
+  k_bias_grad<<<bias_grid(2, P, n), 256, 0, st>>>(F.dout, G + F.off_bp, 2, P);
   count_launch();
   float *dv = F.dva, *dn = F.dvb;
   gemm(F, st, n, C, P, 2, W + F.off_Wp, 1, C, 0, F.dout, P, 1, 2LL * P, dv, P, 1, CP, 0);
@@ -771,16 +794,16 @@ void fno_backward(isg_ctx *c, int n, cudaStream_t st) {
       count_launch();
     }
     // dv now holds dh
-    k_bias_grad<<<dim3(C, 64), 256, 0, st>>>(dv, G + F.off_bw[l], n, C, P);
+    k_bias_grad<<<bias_grid(C, P, n), 256, 0, st>>>(dv, G + F.off_bw[l], C, P);
     count_launch();
     gemm(F, st, n, C, C, P, dv, P, 1, CP, F.v[l], 1, P, CP, G + F.off_W[l], C, 1, 0, 2, ks);
     const int rows = n * C * N;
     gemm(F, st, 1, rows, 2 * M, N, dv, N, 1, 0, F.Ix, 1, N, 0, F.Z, 2 * M, 1, 0, 0);
-    k_fy_fwd<<<blocks((long long)n * C * KY * M), 256, 0, st>>>((const float2 *)F.Z, F.Y, F.Fy, n * C, N, M, KY);
+    fy_fwd((const float2 *)F.Z, F.Y, F, n, st);
     k_mix_bwd_r<<<blocks((long long)NM * C * C), 256, 0, st>>>(F.Y, F.X[l], (float2 *)(G + F.off_R[l]), n, C, NM);
     // dX into the (free) layer-l spectrum buffer of the next pass: reuse T as scratch for dX
-    k_mix_bwd_x<<<blocks((long long)n * C * NM), 256, 0, st>>>(F.Y, (const float2 *)(W + F.off_R[l]),
-                                                               (float2 *)F.T, n, C, NM, F.tensor);
+    k_mix<<<NM, 128, mix_smem(C, n), st>>>(F.Y, (const float2 *)(W + F.off_R[l]), (float2 *)F.T, n, C, NM, F.tensor,
+                                           1);
     k_fy_inv<<<blocks((long long)n * C * N * M), 256, 0, st>>>((const float2 *)F.T, (float2 *)F.Z, F.Fy, n * C, N, M,
                                                                KY);
     count_launch(4);
@@ -790,7 +813,7 @@ void fno_backward(isg_ctx *c, int n, cudaStream_t st) {
   }
   // lift
   gemm(F, st, n, C, kFnoIn, P, dv, P, 1, CP, F.in, 1, P, IP, G + F.off_Wl, kFnoIn, 1, 0, 2, ks);
-  k_bias_grad<<<dim3(C, 64), 256, 0, st>>>(dv, G + F.off_bl, n, C, P);
+  k_bias_grad<<<bias_grid(C, P, n), 256, 0, st>>>(dv, G + F.off_bl, C, P);
   count_launch();
 }
 
