@@ -51,11 +51,11 @@ isg_status run_aggregateh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cu
 }
 
 isg_status run_receive(isg_ctx *c, const float2 *xb, float2 *rx, int nrhs, cudaStream_t st) {
-  return rxnear_active(c) ? rxnear_apply(c, xb, rx, nrhs, 0, st) : run_aggregate(c, xb, rx, nrhs, st);
+  return rxnear_active(c) ? rxnear_apply(c, xb, rx, nrhs, 0, nullptr, st) : run_aggregate(c, xb, rx, nrhs, st);
 }
 
 isg_status run_receiveh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cudaStream_t st) {
-  return rxnear_active(c) ? rxnear_apply(c, rx, xb, nrhs, 1, st) : run_aggregateh(c, xb, rx, nrhs, st);
+  return rxnear_active(c) ? rxnear_apply(c, rx, xb, nrhs, 1, nullptr, st) : run_aggregateh(c, xb, rx, nrhs, st);
 }
 
 }  // namespace isg
@@ -653,6 +653,8 @@ isg_status isg_receiveh(isg_ctx *c, void *x, const void *rx, int nrhs, int order
   cudaStream_t st = pick(c, stream);
   float2 *y = order == ISG_ORDER_BLOCKED ? (float2 *)x : c->wy;
   if ((e = run_receiveh(c, y, (const float2 *)rx, nrhs, st)) != ISG_OK) return e;
+  if (rxnear_active(c))  // reads the caller's order in place
+    return rxnear_apply(c, (const float2 *)x, (float2 *)rx, nrhs, 0, perm_for(c, order), st);
   from_blocked(c, y, x, nrhs, order, st);
   return cuda_check(c, cudaGetLastError(), "receiveh");
 }
@@ -661,6 +663,8 @@ int64_t isg_kernel_launches(void) { return launch_count(); }
 
 isg_status isg_time_stages(isg_ctx *c, int nrhs, int engine, int reps, double *ms) {
   isg_status e = need_gpu(c);
+  if (rxnear_active(c))  // writes the caller's order in place
+    return rxnear_apply(c, (const float2 *)rx, (float2 *)x, nrhs, 1, perm_for(c, order), st);
   if (e != ISG_OK) return e;
   if (!ms || reps < 1 || (e = check_batch(c, nrhs)) != ISG_OK) return ISG_BAD_ARG;
   if (engine == ISG_ENGINE_TENSOR && !tc_available(c)) return ISG_UNSUPPORTED;

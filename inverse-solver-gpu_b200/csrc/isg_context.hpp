@@ -93,13 +93,15 @@ isg_status run_aggregate(isg_ctx *c, const float2 *xb, float2 *rx, int nrhs, cud
 isg_status run_aggregateh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cudaStream_t st);
 const int *order_perm(const isg_ctx *c, int order);
 // The receiver operators of the inversion loop: near-field receivers (dense
+// Blocked vectors.
 // GEMMs, isg_rxnear.cu) when set, else the far-field aggregate / aggregateh.
 isg_status run_receive(isg_ctx *c, const float2 *xb, float2 *rx, int nrhs, cudaStream_t st);
 isg_status run_receiveh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cudaStream_t st);
 isg_status rxnear_setup(isg_ctx *c, double radius);
 void rxnear_destroy(isg_ctx *c);
 bool rxnear_active(const isg_ctx *c);
-isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int adjoint, cudaStream_t st);
+isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int adjoint, const int *perm,
+                        cudaStream_t st);
 int rxnear_error(isg_ctx *c);
 // Tensor-core engine (isg_tc.cu).
 isg_status tc_setup(isg_ctx *c);

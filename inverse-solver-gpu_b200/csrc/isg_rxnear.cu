@@ -15,11 +15,15 @@
 // D_re = Re(G) B and D_im = Im(G) B, and the epilogue combines
 //     forward  re = D_re[j] - D_im[R + j],  im = D_re[R + j] + D_im[j]
 //     adjoint  re = D_re[j] + D_im[R + j],  im = D_re[R + j] - D_im[j]
-// (the adjoint table stores Re and Im of go, not of its conjugate).  Each
-// K-block is converted from FP32 by all threads into the FP16 hi/lo B operand
-// while the previous block's MMAs run (double-buffered A and B).  The forward
-// GEMM has K = numunk and is split over CTAs; the partial products are summed
-// in split order by a second kernel, so results do not depend on timing.
+// (the adjoint table stores Re and Im of go, not of its conjugate).  The
+// kernel is bound by reading its table once; persistent CTAs keep four 32 KB
+// table blocks in flight while converter warps turn the right-hand sides' next
+// K-block from FP32 into the FP16 hi/lo B operand (its loads a block ahead) and
+// epilogue warps write the item before.  The caller's order is applied where
+// pixels are read or written: 8 consecutive pixels of the blocked order are one
+// leaf row, contiguous in every order.  The forward GEMM has K = numunk and is
+// split over CTAs; the partial products are summed in split order by a second
+// kernel, so results do not depend on timing.
 #include <cmath>
 #include <cstring>
 
@@ -51,14 +55,16 @@ constexpr int kRxBlock = 4 * 128 * kRxKB * 2;  // 32 KB: re hi, re lo, im hi, im
 constexpr int kRxSplit = 128 * kRxKB * 2;      // 8 KB: one FP16 split of 128 rows
 constexpr int kRxMaxN = 256;                   // 2 x 128 right-hand sides
 constexpr int kRxBBuf = kRxMaxN * kRxKB * 2 * 2;  // 32 KB: B hi then lo for N = 256
-constexpr int kRxThreads = 256;
+constexpr int kRxNA = 4;                       // table blocks in flight
+constexpr int kRxConvWarp0 = 2, kRxConvWarps = 8, kRxEpiWarp0 = kRxConvWarp0 + kRxConvWarps;  // 0: copies, 1: MMAs
+constexpr int kRxConv = 32 * kRxConvWarps, kRxThreads = 32 * (kRxEpiWarp0 + 4);
 constexpr int kErrRx = 131;
 struct RxSmem {
-  static constexpr int a = 0;                     // 2 A blocks
-  static constexpr int b = 2 * kRxBlock;          // 2 B operands
-  static constexpr int bars = b + 2 * kRxBBuf;    // afull[2], mdone[2], fin
-  static constexpr int misc = bars + 8 * 8;
-  static constexpr int total = misc + 16;
+  static constexpr int a = 0;                      // kRxNA A blocks
+  static constexpr int b = kRxNA * kRxBlock;       // 2 B operands
+  static constexpr int bars = b + 2 * kRxBBuf;     // afull, aempty [kRxNA]; bfull, bempty, tfull, tfree [2]; fin
+  static constexpr int misc = bars + (2 * kRxNA + 9) * 8;
+  static constexpr int total = misc + 16;          // TMEM base, abort flag
 };
 
 // Offset of element (row, k) of a 128 x 32 (or N x 32) K-major FP16 block in
@@ -126,13 +132,23 @@ __global__ void k_rx_pack(RxBuild B, int adjoint, int kb_total, const unsigned *
   }
 }
 
-// max |re|, |im| per right-hand side of [R][ld] complex rows (first kvalid elements)
-__global__ void k_rx_rowmax(const float2 *x, int64_t ld, int kvalid, unsigned *rowmax) {
+// max |re|, |im| per right-hand side of [R][ld] complex rows (first kvalid
+// elements); vec: rows are 16-byte aligned and kvalid is even
+__global__ void k_rx_rowmax(const float2 *x, int64_t ld, int kvalid, int vec, unsigned *rowmax) {
   const int j = blockIdx.y;
+  const float2 *r = x + (size_t)j * ld;
   float m = 0.f;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kvalid; k += gridDim.x * blockDim.x) {
-    const float2 v = x[(size_t)j * ld + k];
-    m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+  if (vec) {
+#pragma unroll 4
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kvalid / 2; k += gridDim.x * blockDim.x) {
+      const float4 v = __ldg((const float4 *)r + k);
+      m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+  } else {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kvalid; k += gridDim.x * blockDim.x) {
+      const float2 v = r[k];
+      m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+    }
   }
   const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
   if ((threadIdx.x & 31) == 0 && bits) atomicMax(&rowmax[j], bits);
@@ -144,6 +160,9 @@ struct RxGemmArgs {
   const float2 *x;    // B source: [R][ldx] complex, K index = element
   int64_t ldx;
   int kvalid, R, npad;  // valid K, right-hand sides, N = 2R padded to 16
+  int vec;              // rows of x are 16-byte aligned
+  int mt, nitems;       // row tiles; items = row tiles x K splits
+  const int *perm, *out_perm;  // caller's index of each blocked pixel: K of the forward, rows of the adjoint; or null
   const unsigned *rowmax;
   float ainv;
   int adjoint;
@@ -156,108 +175,194 @@ struct RxGemmArgs {
 
 __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
   extern __shared__ __align__(1024) char sm[];
-  uint64_t *afull = (uint64_t *)(sm + RxSmem::bars), *mdone = afull + 2, *fin = afull + 4;
+  uint64_t *afull = (uint64_t *)(sm + RxSmem::bars), *aempty = afull + kRxNA;
+  uint64_t *bfull = aempty + kRxNA, *bempty = bfull + 2, *tfull = bempty + 2, *tfree = tfull + 2, *fin = tfree + 2;
   uint32_t *tslot = (uint32_t *)(sm + RxSmem::misc);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = blockIdx.x, split = blockIdx.y;
-  const int kb0 = split * A.kb_per, kb1 = min(kb0 + A.kb_per, A.kb_total);
+  volatile int *abort = (volatile int *)(sm + RxSmem::misc + 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, R = A.R;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 5; i++) mbar_init(afull + i, 1);
+    for (int i = 0; i < 2 * kRxNA + 9; i++) mbar_init(afull + i, 1);
+    *abort = 0;
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tslot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tslot;  // D_re in columns [0, npad), D_im in [256, 256 + npad)
-  const uint32_t idesc = idesc_f16_f32(128, A.npad), sbase = smem_u32(sm);
-  const int R = A.R;
-  bool ok = true;
-  for (int kb = kb0, it = 0; kb < kb1; kb++, it++) {
-    const int b = it & 1;
-    // buffers b (A and B) are free once the MMAs of block it - 2 are done
-    if (it >= 2) ok = mbar_wait(mdone + b, ((it >> 1) - 1) & 1, A.err, kErrRx) && ok;
-    if (threadIdx.x == 0 && ok) {
-      mbar_expect_tx(afull + b, kRxBlock);
-      bulk_g2s(sm + RxSmem::a + b * kRxBlock, A.A + ((size_t)mt * A.kb_total + kb) * kRxBlock, kRxBlock, afull + b);
-    }
-    // B operand: row j = Re x_j, row R + j = Im x_j over K = kb * 32 .. + 32, scaled per RHS
-    __half *bh = (__half *)(sm + RxSmem::b + b * kRxBBuf), *bl = bh + A.npad * kRxKB;
-    for (int e = threadIdx.x; e < R * (kRxKB / 8); e += kRxThreads) {
-      const int j = e / (kRxKB / 8), c = e % (kRxKB / 8);  // 8 K-elements of RHS j
-      const float s = pow2_scale(__uint_as_float(A.rowmax[j]));
-      __align__(16) __half rh[8], rl[8], ih[8], il[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int K = kb * kRxKB + c * 8 + q;
-        const float2 v = K < A.kvalid ? A.x[(size_t)j * A.ldx + K] : make_float2(0.f, 0.f);
-        split_f16(v.x * s, rh[q], rl[q]);
-        split_f16(v.y * s, ih[q], il[q]);
-      }
-      const int o0 = rx_core_off(j, c * 8) / 2, o1 = rx_core_off(R + j, c * 8) / 2;
-      *(uint4 *)(bh + o0) = *(uint4 *)rh;
-      *(uint4 *)(bl + o0) = *(uint4 *)rl;
-      *(uint4 *)(bh + o1) = *(uint4 *)ih;
-      *(uint4 *)(bl + o1) = *(uint4 *)il;
-    }
-    // rows 2R .. npad - 1 stay zero
-    for (int e = threadIdx.x; e < (A.npad - 2 * R) * (kRxKB / 8); e += kRxThreads) {
-      const int r = 2 * R + e / (kRxKB / 8), c = e % (kRxKB / 8);
-      const int o = rx_core_off(r, c * 8) / 2;
-      *(uint4 *)(bh + o) = make_uint4(0, 0, 0, 0);
-      *(uint4 *)(bl + o) = make_uint4(0, 0, 0, 0);
-    }
-    fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      ok = mbar_wait(afull + b, (it >> 1) & 1, A.err, kErrRx) && ok;
-      tc_fence_after();
-      if (ok) {
-        const uint32_t ab = sbase + RxSmem::a + b * kRxBlock, bb = sbase + RxSmem::b + b * kRxBBuf;
-        const uint64_t brh = smem_desc(bb, 128, 512), brl = smem_desc(bb + A.npad * kRxKB * 2, 128, 512);
-#pragma unroll
-        for (int part = 0; part < 2; part++) {  // re, im of the table
-          const uint64_t ah = smem_desc(ab + part * 2 * kRxSplit, 128, 512);
-          const uint64_t al = smem_desc(ab + part * 2 * kRxSplit + kRxSplit, 128, 512);
-          const uint32_t d = tmem + (uint32_t)(part * 256);
-#pragma unroll
-          for (int ks = 0; ks < kRxKB / 16; ks++) {
-            const int acc = (kb > kb0 || ks > 0) ? 1 : 0;
-            mma_f16(d, desc_add(ah, ks * 256), desc_add(brh, ks * 256), idesc, acc);
-            mma_f16(d, desc_add(ah, ks * 256), desc_add(brl, ks * 256), idesc, 1);
-            mma_f16(d, desc_add(al, ks * 256), desc_add(brh, ks * 256), idesc, 1);
-          }
+  const uint32_t tmem = *tslot;
+  // accumulator set s: D_re at column 256 s, D_im dim columns on; one set of 2 x 256 when npad > 128
+  const int nset = A.npad <= 128 ? 2 : 1, dim = nset == 2 ? 128 : 256;
+  // item w: row tile w % mt of K split w / mt, K-blocks [kb0, kb1)
+  auto blocks = [&](int w, int &kb0, int &kb1) {
+    kb0 = (w / A.mt) * A.kb_per;
+    kb1 = min(kb0 + A.kb_per, A.kb_total);
+  };
+
+  if (warp == 0) {
+    // ---- table blocks through the ring ----
+    if (lane == 0) {
+      int ka = 0;
+      for (int w = blockIdx.x; w < A.nitems && !*abort; w += gridDim.x) {
+        int kb0, kb1;
+        blocks(w, kb0, kb1);
+        const uint8_t *src = A.A + (size_t)(w % A.mt) * A.kb_total * kRxBlock;
+        for (int kb = kb0; kb < kb1; kb++, ka++) {
+          const int i = ka % kRxNA;
+          if (!mbar_wait_or(aempty + i, ((ka / kRxNA) & 1) ^ 1, abort, A.err, kErrRx)) break;
+          mbar_expect_tx(afull + i, kRxBlock);
+          bulk_g2s(sm + RxSmem::a + i * kRxBlock, src + (size_t)kb * kRxBlock, kRxBlock, afull + i);
         }
       }
-      mma_commit(mdone + b);
+      // every copy issued has landed before the CTA exits (bounded waits)
+      for (int j = 1; j <= kRxNA && j <= ka; j++) mbar_wait(afull + (ka - j) % kRxNA, ((ka - j) / kRxNA) & 1, A.err, kErrRx);
     }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) mma_commit(fin);
-  ok = mbar_wait(fin, 0, A.err, kErrRx) && ok && kb1 > kb0;
-  tc_fence_after();
-  // epilogue: lane = table row, columns = right-hand sides; warps 0..3 and 4..7
-  // take alternate groups of 16 right-hand sides
-  const int qd = warp & 3, half = warp >> 2;
-  const int row = mt * 128 + 32 * qd + lane;
-  float2 *out = A.out + (size_t)split * A.split_stride;
-  for (int j0 = 16 * half; j0 < R; j0 += 32) {
-    __syncwarp();
-    float dre[16], dre2[16], dim[16], dim2[16];
-    tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)j0, dre);
-    tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(R + j0), dre2);
-    tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(256 + j0), dim);
-    tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(256 + R + j0), dim2);
-    if (ok && row < A.mvalid) {
+  } else if (warp == 1) {
+    // ---- MMA issue: D_re += Re(A) B, D_im += Im(A) B, three split products each ----
+    if (lane == 0) {
+      const uint32_t idesc = idesc_f16_f32(128, A.npad), sbase = smem_u32(sm);
+      int ka = 0, it = 0;
+      bool ok = true;
+      for (int w = blockIdx.x; w < A.nitems && ok; w += gridDim.x, it++) {
+        int kb0, kb1;
+        blocks(w, kb0, kb1);
+        const int set = it % nset;
+        ok = mbar_wait_or(tfree + set, ((it / nset) & 1) ^ 1, abort, A.err, kErrRx);
+        for (int kb = kb0; kb < kb1 && ok; kb++, ka++) {
+          const int i = ka % kRxNA, b = ka & 1;
+          ok = mbar_wait_or(afull + i, (ka / kRxNA) & 1, abort, A.err, kErrRx) &&
+               mbar_wait_or(bfull + b, (ka >> 1) & 1, abort, A.err, kErrRx);
+          tc_fence_after();
+          if (!ok) break;
+          const uint32_t ab = sbase + RxSmem::a + i * kRxBlock, bb = sbase + RxSmem::b + b * kRxBBuf;
+          const uint64_t brh = smem_desc(bb, 128, 512), brl = smem_desc(bb + A.npad * kRxKB * 2, 128, 512);
 #pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int j = j0 + q;
-        if (j >= R) break;
-        const float inv = A.ainv / pow2_scale(__uint_as_float(A.rowmax[j]));
-        const float re = A.adjoint ? dre[q] + dim2[q] : dre[q] - dim2[q];
-        const float im = A.adjoint ? dre2[q] - dim[q] : dre2[q] + dim[q];
-        out[(size_t)j * A.ldo + row] = make_float2(re * inv, im * inv);
+          for (int part = 0; part < 2; part++) {  // re, im of the table
+            const uint64_t ah = smem_desc(ab + part * 2 * kRxSplit, 128, 512);
+            const uint64_t al = smem_desc(ab + part * 2 * kRxSplit + kRxSplit, 128, 512);
+            const uint32_t d = tmem + (uint32_t)(set * 256 + part * dim);
+#pragma unroll
+            for (int ks = 0; ks < kRxKB / 16; ks++) {
+              mma_f16(d, desc_add(ah, ks * 256), desc_add(brh, ks * 256), idesc, (kb > kb0 || ks > 0) ? 1 : 0);
+              mma_f16(d, desc_add(ah, ks * 256), desc_add(brl, ks * 256), idesc, 1);
+              mma_f16(d, desc_add(al, ks * 256), desc_add(brh, ks * 256), idesc, 1);
+            }
+          }
+          mma_commit(aempty + i);
+          mma_commit(bempty + b);
+        }
+        if (ok) mma_commit(tfull + set);
       }
+      // every MMA issued is complete before TMEM is freed (bounded wait)
+      mma_commit(fin);
+      mbar_wait(fin, 0, A.err, kErrRx);
+    }
+  } else if (warp < kRxEpiWarp0) {
+    // ---- converters: B row j = Re x_j, row R + j = Im x_j over the K-block's 32 elements, scaled per
+    // RHS.  A unit is 8 consecutive K of one RHS; a thread has at most two, loaded a block ahead ----
+    const int ct = threadIdx.x - 32 * kRxConvWarp0, nu = 4 * R;
+    float sc[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int u = ct + q * kRxConv;
+      sc[q] = u < nu ? pow2_scale(__uint_as_float(A.rowmax[u >> 2])) : 1.f;
+    }
+    float2 v[2][8];
+    auto load = [&](int kb) {
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int u = ct + q * kRxConv, K = kb * kRxKB + (u & 3) * 8;
+        const float2 *row = A.x + (size_t)(u >> 2) * A.ldx;
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[q][e] = make_float2(0.f, 0.f);
+        if (u >= nu || K >= A.kvalid) continue;
+        const float2 *src = row + (A.perm ? A.perm[K] : K);
+        if (A.vec && K + 8 <= A.kvalid) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const float4 t = __ldg((const float4 *)src + e);
+            v[q][2 * e] = make_float2(t.x, t.y);
+            v[q][2 * e + 1] = make_float2(t.z, t.w);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; e++)
+            if (K + e < A.kvalid) v[q][e] = src[e];
+        }
+      }
+    };
+    // rows 2R .. npad - 1 stay zero
+    for (int e = ct; e < 2 * (A.npad - 2 * R) * (kRxKB / 8); e += kRxConv) {
+      const int b = e & 1, r = 2 * R + (e >> 1) / (kRxKB / 8), c = (e >> 1) % (kRxKB / 8);
+      char *bh = sm + RxSmem::b + b * kRxBBuf, *bl = bh + A.npad * kRxKB * 2;
+      *(uint4 *)(bh + rx_core_off(r, c * 8)) = make_uint4(0, 0, 0, 0);
+      *(uint4 *)(bl + rx_core_off(r, c * 8)) = make_uint4(0, 0, 0, 0);
+    }
+    int ka = 0;
+    for (int w = blockIdx.x; w < A.nitems; w += gridDim.x) {
+      int kb0, kb1;
+      blocks(w, kb0, kb1);
+      if (kb0 < kb1) load(kb0);
+      for (int kb = kb0; kb < kb1; kb++, ka++) {
+        const int b = ka & 1;
+        uint32_t rh[2][4], rl[2][4], ih[2][4], il[2][4];
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            split2u(v[q][2 * e].x * sc[q], v[q][2 * e + 1].x * sc[q], rh[q][e], rl[q][e]);
+            split2u(v[q][2 * e].y * sc[q], v[q][2 * e + 1].y * sc[q], ih[q][e], il[q][e]);
+          }
+        if (kb + 1 < kb1) load(kb + 1);
+        const bool ok = mbar_wait_or(bempty + b, ((ka >> 1) & 1) ^ 1, abort, A.err, kErrRx);
+        char *bh = sm + RxSmem::b + b * kRxBBuf, *bl = bh + A.npad * kRxKB * 2;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const int u = ct + q * kRxConv, j = u >> 2, c = u & 3;
+          if (u >= nu || !ok) continue;
+          st_shared_v4(bh + rx_core_off(j, c * 8), rh[q]);
+          st_shared_v4(bl + rx_core_off(j, c * 8), rl[q]);
+          st_shared_v4(bh + rx_core_off(R + j, c * 8), ih[q]);
+          st_shared_v4(bl + rx_core_off(R + j, c * 8), il[q]);
+        }
+        fence_proxy_async();
+        named_sync(1, kRxConv);
+        if (ct == 0) mbar_arrive(bfull + b);
+      }
+    }
+  } else {
+    // ---- epilogue: lane = table row, columns = right-hand sides ----
+    const int qd = warp & 3;
+    int it = 0;
+    for (int w = blockIdx.x; w < A.nitems; w += gridDim.x, it++) {
+      const int set = it % nset;
+      const bool ok = mbar_wait_or(tfull + set, (it / nset) & 1, abort, A.err, kErrRx);
+      __syncwarp();
+      tc_fence_after();
+      const int row = (w % A.mt) * 128 + 32 * qd + lane;
+      const bool live = ok && row < A.mvalid;
+      float2 *out = A.out + (size_t)(w / A.mt) * A.split_stride + (live && A.out_perm ? A.out_perm[row] : row);
+      const uint32_t t0 = tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(set * 256);
+      for (int j0 = 0; j0 < R; j0 += 16) {
+        __syncwarp();
+        float dre[16], dre2[16], dim1[16], dim2[16];
+        tmem_ld16(t0 + (uint32_t)j0, dre);
+        tmem_ld16(t0 + (uint32_t)(R + j0), dre2);
+        tmem_ld16(t0 + (uint32_t)(dim + j0), dim1);
+        tmem_ld16(t0 + (uint32_t)(dim + R + j0), dim2);
+        if (!live) continue;
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+          const int j = j0 + q;
+          if (j >= R) break;
+          const float inv = A.ainv / pow2_scale(__uint_as_float(A.rowmax[j]));
+          const float re = A.adjoint ? dre[q] + dim2[q] : dre[q] - dim2[q];
+          const float im = A.adjoint ? dre2[q] - dim1[q] : dre2[q] + dim1[q];
+          out[(size_t)j * A.ldo] = make_float2(re * inv, im * inv);
+        }
+      }
+      tc_fence_before();
+      named_sync(2, 128);  // the accumulator set is read out
+      if (warp == kRxEpiWarp0 && lane == 0) mbar_arrive(tfree + set);
     }
   }
   tc_fence_before();
@@ -270,6 +375,7 @@ __global__ void k_rx_sum(const float2 *part, int nsplit, size_t stride, int R, i
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= R * nrx) return;
   float2 s = make_float2(0.f, 0.f);
+#pragma unroll 16
   for (int q = 0; q < nsplit; q++) {
     const float2 v = part[q * stride + e];
     s.x += v.x;
@@ -353,10 +459,13 @@ isg_status rxnear_setup(isg_ctx *c, double radius) {
   return ISG_OK;
 }
 
-// Forward (r = go x) or adjoint (x = gh r) on blocked vectors, in batches of
-// at most 128 right-hand sides.
-isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int adjoint, cudaStream_t st) {
+// Forward (r = go x) or adjoint (x = gh r), pixel vectors in the order that perm
+// maps blocked indices to (null: blocked), in batches of at most 128 right-hand sides.
+isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int adjoint, const int *perm,
+                        cudaStream_t st) {
   RxPlan &P = *c->rx;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
   const int Rmax = std::min(c->opts.max_rhs, kRxMaxN / 2);
   for (int j0 = 0; j0 < nrhs; j0 += Rmax) {
     const int R = std::min(Rmax, nrhs - j0);
@@ -371,6 +480,10 @@ isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int
     A.kvalid = (int)ldin;
     A.R = R;
     A.npad = std::max(16, (2 * R + 15) / 16 * 16);
+    A.vec = ((uintptr_t)A.x & 15) == 0 && ldin % 2 == 0;
+    A.mt = adjoint ? P.mt_a : P.mt_f;
+    A.nitems = A.mt * nsplit;
+    A.perm = perm;
     A.rowmax = P.rowmax;
     A.ainv = P.ainv;
     A.adjoint = adjoint;
@@ -378,20 +491,23 @@ isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int
     A.mvalid = (int)ldout;
     A.err = P.err;
     if (adjoint) {
+      A.perm = nullptr;  // K runs over receivers; rows are placed by out_perm
+      A.out_perm = perm;
       A.out = out + (size_t)j0 * ldout;
       A.split_stride = 0;
     } else {
+      A.out_perm = nullptr;
       A.out = P.part;
       A.split_stride = (size_t)R * P.nrx;
     }
     cudaMemsetAsync(P.rowmax, 0, (size_t)R * sizeof(unsigned), st);
     count_launch(2);
-    k_rx_rowmax<<<dim3(std::max(1, std::min(64, (int)((ldin + 255) / 256))), R), 256, 0, st>>>(A.x, ldin, A.kvalid,
-                                                                                              P.rowmax);
-    k_rx_gemm<<<dim3(adjoint ? P.mt_a : P.mt_f, nsplit), kRxThreads, RxSmem::total, st>>>(A);
+    k_rx_rowmax<<<dim3(std::max(1, std::min(64, (int)((ldin + 2047) / 2048))), R), 256, 0, st>>>(A.x, ldin, A.kvalid,
+                                                                                                A.vec, P.rowmax);
+    k_rx_gemm<<<std::min(A.nitems, sms), kRxThreads, RxSmem::total, st>>>(A);
     if (!adjoint) {
       count_launch();
-      k_rx_sum<<<(R * P.nrx + 255) / 256, 256, 0, st>>>(P.part, nsplit, A.split_stride, R, P.nrx,
+      k_rx_sum<<<(R * P.nrx + 127) / 128, 128, 0, st>>>(P.part, nsplit, A.split_stride, R, P.nrx,
                                                         out + (size_t)j0 * P.nrx);
     }
   }
