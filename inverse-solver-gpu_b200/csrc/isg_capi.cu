@@ -369,12 +369,14 @@ isg_status isg_setup_gpu(isg_ctx *c) {
 
   const size_t R = c->opts.max_rhs, U = T.U;
   c->vec_blocks = (int)std::min<size_t>(512, std::max<size_t>(1, U / 2048));
-  c->part_blocks = std::max(c->vec_blocks, near_blocks_per_rhs(P));
+  // partial records: the vector updates' blocks, the tensor engine's 8 x 8 leaves, k_near's tiles
+  const size_t tc_tiles = (size_t)((T.nleaf + 7) / 8) * ((T.nleaf + 7) / 8);
+  const size_t parts = std::max(R * std::max<size_t>(c->vec_blocks, tc_tiles), near_partials(P, (int)R));
   if ((e = dalloc(c, &c->mul, R * P.mp)) || (e = dalloc(c, &c->loc, R * P.mp)) || (e = dalloc(c, &c->wx, R * U)) ||
       (e = dalloc(c, &c->wy, R * U)) || (e = dalloc(c, &c->wg, R * U)) || (e = dalloc(c, &c->vr, R * U)) ||
       (e = dalloc(c, &c->vrt, R * U)) || (e = dalloc(c, &c->vp, R * U)) || (e = dalloc(c, &c->vv, R * U)) ||
       (e = dalloc(c, &c->vs, R * U)) || (e = dalloc(c, &c->vt, R * U)) || (e = dalloc(c, &c->vgx, R * U)) || (e = dalloc(c, &c->levmax, 2 * R * kMaxLevels)) ||
-      (e = dalloc(c, &c->part, R * (size_t)c->part_blocks * 4 + 64)) || (e = dalloc(c, &c->state, R)) ||
+      (e = dalloc(c, &c->part, parts * 4 + 64)) || (e = dalloc(c, &c->state, R)) ||
       (e = dalloc(c, &c->active, R)) || (e = dalloc(c, &c->count, 1)))
     return e;
   c->locmax = c->levmax + R * kMaxLevels;

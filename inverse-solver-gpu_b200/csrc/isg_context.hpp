@@ -47,8 +47,7 @@ struct isg_ctx {
   float2 *vgx = nullptr;  // [R][U] g times the next matvec's input, written by the update kernels
   unsigned *levmax = nullptr;  // [R][kMaxLevels] per-level max |re|, |im| of the multipoles (FP32 bits)
   unsigned *locmax = nullptr;  // [R][kMaxLevels] the same for the locals (written by M2L)
-  double *part = nullptr;  // [R][part_blocks][4]
-  int part_blocks = 0;
+  double *part = nullptr;  // FP64 partial records [RHS][block][4]
   isg::RhsState *state = nullptr;  // [R]
   int *active = nullptr;           // [R]
   int *count = nullptr;            // active-RHS counter
@@ -93,8 +92,8 @@ isg_status run_aggregate(isg_ctx *c, const float2 *xb, float2 *rx, int nrhs, cud
 isg_status run_aggregateh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cudaStream_t st);
 const int *order_perm(const isg_ctx *c, int order);
 // The receiver operators of the inversion loop: near-field receivers (dense
-// Blocked vectors.
 // GEMMs, isg_rxnear.cu) when set, else the far-field aggregate / aggregateh.
+// Blocked vectors.
 isg_status run_receive(isg_ctx *c, const float2 *xb, float2 *rx, int nrhs, cudaStream_t st);
 isg_status run_receiveh(isg_ctx *c, float2 *xb, const float2 *rx, int nrhs, cudaStream_t st);
 isg_status rxnear_setup(isg_ctx *c, double radius);

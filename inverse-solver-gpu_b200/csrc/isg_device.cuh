@@ -172,7 +172,12 @@ struct NearArgs {
   const unsigned *inmax = nullptr;   // tensor engine: [R][kMaxLevels] whose last slot holds the input's
                                      // maximum per RHS, written by the tensor-core P2M of the same matvec
 };
-int near_blocks_per_rhs(const DevPlan &P);
+// FP64 partial records per RHS that launch_near writes for a batch of nrhs, and
+// the most records of any batch up to max_rhs.
+int near_blocks_per_rhs(const DevPlan &P, int nrhs);
+size_t near_partials(const DevPlan &P, int max_rhs);
+// Samples of a level over all its clusters and a batch.
+int64_t level_outputs(const DevPlan &P, int lvl, int nrhs);
 void launch_near(const DevPlan &P, const NearArgs &A, cudaStream_t st);
 void launch_rx_interp(const DevPlan &P, const float2 *mul, float2 *rx, int nrhs, cudaStream_t st);
 void launch_rx_anterp(const DevPlan &P, const float2 *rx, float2 *loc, int nrhs, float2 scale, cudaStream_t st);

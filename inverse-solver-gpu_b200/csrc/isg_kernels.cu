@@ -24,25 +24,39 @@ void capture_launches(int64_t *sink) { t_capture_sink = sink; }
 
 namespace {
 
-constexpr int kNearTY = 4;  // near-field tile: 4 x 8 leaves per block
-constexpr int kNearTX = 8;
-constexpr int kHaloLeaves = (kNearTY + 2) * (kNearTX + 2);
+// Largest launches of each shape, in leaves or output samples of all RHS: where
+// the stage times of the shapes cross (us, launch and event overhead of about 6
+// included).  P2M by leaves: 2048: 13.0 / 14.1 / 27.9 with 2, 8 and 32 leaves a
+// block, 4096: 20.2 / 15.3 / 27.0, 16384: 40.3 / 30.0 / 32.1.  Near field by
+// leaves: 256: 22.5 / 43.9 / 72.7 with 2 x 2, 4 x 4 and 4 x 8 leaves, 1024: 30.8 /
+// 45.0 / 75.8, 2048: 62.4 / 45.1 / 75.8, 4096: 90.6 / 62.0 / 76.3, 8192: 149 / 115
+// / 88.  All M2M levels of 1024 x 1024 x 1 (up to 425984 outputs) 70.8 direct,
+// 102.6 tiled; L2L (with M2L) of 256 x 256 x 2 (139264 leaf outputs) 61.5 / 73.5,
+// of 512 x 512 x 2 (212992 and 557056 outputs) 111 / 103.
+constexpr int64_t kP2mSmall = 2048, kP2mMid = 16384;
+constexpr int64_t kNearSmall = 1024, kNearMid = 4096;
+constexpr int64_t kM2mDirect = 500000, kL2lDirect = 200000;
 
 __device__ __forceinline__ bool inactive(const int *active, int rhs) { return active && !active[rhs]; }
 
 // P2M (kernels.cu:6-30, solve.cpp:80-92): leaf multipoles
-// mul[leaf][k] = sum_n coeff[k][n] * in[leaf*64 + n], 32 leaves per block.
-__global__ void __launch_bounds__(128) k_p2m(const float2 *__restrict__ x, const float2 *__restrict__ g,
+// mul[leaf][k] = sum_n coeff[k][n] * in[leaf*64 + n].  A block takes LB leaves
+// and a thread LT of them at one sample, walking the 64 pixels: LT sets how
+// often a coefficient read from L2 is used, LB how many blocks a grid has
+// (p2m_shape picks; the walk is one dependent chain, so a launch of few blocks
+// is as long as that chain times a block's passes over its LB / LT * ns units).
+template <int LB, int LT>
+__global__ void __launch_bounds__(288) k_p2m(const float2 *__restrict__ x, const float2 *__restrict__ g,
                                              int64_t gstride, int mode, const int *__restrict__ active,
                                              const float2 *__restrict__ coeffT, int ns, int nleaves, int U,
                                              float2 *__restrict__ mul_leaf, size_t mp) {
   const int rhs = blockIdx.y;
   if (inactive(active, rhs)) return;
-  __shared__ float2 xs[32][kBB];
-  const int leaf0 = blockIdx.x * 32;
+  __shared__ float2 xs[LB][kBB];
+  const int leaf0 = blockIdx.x * LB;
   const float2 *xr = x + (size_t)rhs * U;
   const float2 *gr = g ? g + rhs * gstride : nullptr;
-  for (int e = threadIdx.x; e < 32 * kBB; e += blockDim.x) {
+  for (int e = threadIdx.x; e < LB * kBB; e += blockDim.x) {
     const int leaf = leaf0 + e / kBB;
     float2 v = make_float2(0.f, 0.f);
     if (leaf < nleaves) {
@@ -53,18 +67,18 @@ __global__ void __launch_bounds__(128) k_p2m(const float2 *__restrict__ x, const
   }
   __syncthreads();
   float2 *out = mul_leaf + (size_t)rhs * mp;
-  for (int u = threadIdx.x; u < 8 * ns; u += blockDim.x) {
+  for (int u = threadIdx.x; u < LB / LT * ns; u += blockDim.x) {
     const int k = u % ns, lg = u / ns;
-    float2 acc[4] = {};
-#pragma unroll 8
+    float2 acc[LT] = {};
+#pragma unroll 16
     for (int n = 0; n < kBB; n++) {
       const float2 c = __ldg(&coeffT[n * ns + k]);
 #pragma unroll
-      for (int j = 0; j < 4; j++) cfma(acc[j], c, xs[lg * 4 + j][n]);
+      for (int j = 0; j < LT; j++) cfma(acc[j], c, xs[lg * LT + j][n]);
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int leaf = leaf0 + lg * 4 + j;
+    for (int j = 0; j < LT; j++) {
+      const int leaf = leaf0 + lg * LT + j;
       if (leaf < nleaves) out[(size_t)leaf * ns + k] = acc[j];
     }
   }
@@ -483,6 +497,67 @@ __global__ void __launch_bounds__(128) k_m2m_tile(TileArgs A) {
 }
 
 
+// M2M and L2L of a small launch: one thread per output sample, the taps read
+// straight from L1 / L2 (consecutive threads take consecutive samples, so the
+// loads of a warp fall on the same few lines).  The tiled kernels above stage
+// 32 or more columns per block and read each value once; a launch with fewer
+// outputs than kM2mDirect or kL2lDirect leaves most SMs without a block there
+// and is as long as one block's chain of staging, walk and write-back.  Both add
+// an output's taps in ring order, with the same roundings.
+struct DirectArgs {
+  const float2 *src;  // input level, one RHS' block every mp elements
+  float2 *dst;
+  size_t mp;
+  int n_p, ns_in, ns_out, width;
+  const int *first;    // [ns_out] first tap
+  const float *w;      // [width][ns_out]
+  const float2 *shift; // M2M shiftmul [4][ns_out], L2L shiftloc [4][ns_in]
+  const int *active;
+};
+
+__global__ void __launch_bounds__(128) k_m2m_direct(DirectArgs A) {
+  const int rhs = blockIdx.y;
+  if (inactive(A.active, rhs)) return;
+  const int o = blockIdx.x * blockDim.x + threadIdx.x, P = o / A.ns_out, k = o - P * A.ns_out;
+  if (P >= A.n_p * A.n_p) return;
+  const int py = P / A.n_p, px = P - py * A.n_p, n_c = 2 * A.n_p;
+  const float2 *c0 = A.src + (size_t)rhs * A.mp + (size_t)(2 * py * n_c + 2 * px) * A.ns_in;
+  const float2 *c[4] = {c0, c0 + A.ns_in, c0 + (size_t)n_c * A.ns_in, c0 + (size_t)(n_c + 1) * A.ns_in};
+  float2 acc[4] = {};
+  int j = A.first[k];
+#pragma unroll 10
+  for (int t = 0; t < A.width; t++) {
+    const float w = __ldg(&A.w[(size_t)t * A.ns_out + k]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) rfma(acc[q], w, c[q][j]);
+    if (++j == A.ns_in) j = 0;
+  }
+  float2 r = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < 4; q++) cfma(r, __ldg(&A.shift[q * A.ns_out + k]), acc[q]);
+  A.dst[(size_t)rhs * A.mp + o] = r;
+}
+
+__global__ void __launch_bounds__(128) k_l2l_direct(DirectArgs A) {
+  const int rhs = blockIdx.y;
+  if (inactive(A.active, rhs)) return;
+  const int o = blockIdx.x * blockDim.x + threadIdx.x, c = o / A.ns_out, k = o - c * A.ns_out, n_c = 2 * A.n_p;
+  if (c >= n_c * n_c) return;
+  const int cy = c / n_c, cx = c - cy * n_c, q = 2 * (cy & 1) + (cx & 1);
+  const float2 *z = A.src + (size_t)rhs * A.mp + (size_t)((cy >> 1) * A.n_p + (cx >> 1)) * A.ns_in;
+  const float2 *sh = A.shift + (size_t)q * A.ns_in;
+  float2 acc = make_float2(0.f, 0.f);
+  int j = A.first[k];
+#pragma unroll 10
+  for (int t = 0; t < A.width; t++) {
+    const float2 s = __ldg(&sh[j]), v = z[j];  // s v rounded as in k_l2l_tile
+    rfma(acc, __ldg(&A.w[(size_t)t * A.ns_out + k]),
+         make_float2(fmaf(-s.y, v.y, __fmul_rn(s.x, v.x)), fmaf(s.y, v.x, __fmul_rn(s.x, v.y))));
+    if (++j == A.ns_in) j = 0;
+  }
+  A.dst[(size_t)rhs * A.mp + o] = acc;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -491,30 +566,88 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // L2P (kernels.cu:32-81, solve.cpp:170-182) + near field (kernels.cu:292-319,
 // solve.cpp:199-216) + matvec epilogue (kernels.cu:402-409) + BiCGSTAB partial
-// dot products, for a tile of 4 x 8 leaves of one RHS.  The 6 x 10 halo of
-// leaves sits in shared memory; thread (t, row) owns pixel t of the 8 leaves of
-// one tile row.
-__global__ void __launch_bounds__(256) k_near(const float2 *__restrict__ x, const float2 *__restrict__ g,
-                                              int64_t gstride, int mode, const int *__restrict__ active,
-                                              const float2 *__restrict__ loc_leaf, size_t mp, int ns,
-                                              const float2 *__restrict__ nearW, const float2 *__restrict__ basisT,
-                                              float2 *__restrict__ y, int epi, int red,
-                                              const float2 *__restrict__ dot_a, double *__restrict__ part, int nleaf,
-                                              int U, int tiles_x, int tiles_total) {
+// dot products, for a tile of TY x TX leaves of one RHS.  The (TY + 2) x
+// (TX + 2) halo of leaves sits in shared memory; thread (t, row) sums pixel t
+// of the TX leaves of one tile row.  Fewer leaves per block keep more SMs at work
+// on a small launch (near_shape); a block's time there is its chain of 644
+// dependent products and its trips to L2 for the weights.  So up to 4 x 4 leaves
+// the weights, 9 * 64 + ns rows of 64, go through a ring of near_stages stages of
+// near_rows rows in shared memory that cp.async fills ahead of the row being
+// multiplied; 4 x 8 leaves, enough warps to hide the trips, read them from L1 / L2
+// (16384 leaves: 168 us, staged 174).
+// Every shape adds a pixel's terms in the same order, so the field does not
+// depend on the shape.
+__host__ __device__ constexpr int near_rows(int tx) { return tx == 2 ? 32 : 16; }
+__host__ __device__ constexpr int near_stages(int tx) { return tx == 8 ? 0 : tx == 4 ? 6 : 4; }
+
+// 8 rows of the staged walk: weights w (one row every 64) and, per leaf, 8
+// consecutive inputs (one leaf every xs, 16-byte aligned).  The loads are volatile
+// so that they are in flight before the first product, and the launch bounds leave
+// the registers for it (94 at TX 2, where the compiler otherwise kept to 34).
+template <int TX>
+struct NearRows {
+  float2 w[8];
+  float4 v[TX][4];
+  __device__ __forceinline__ void load(const float2 *wr, const float2 *x, int xs) {
+    const unsigned ws = (unsigned)__cvta_generic_to_shared(wr), xa = (unsigned)__cvta_generic_to_shared(x);
+#pragma unroll
+    for (int b = 0; b < 8; b++)
+      asm volatile("ld.volatile.shared.v2.f32 {%0, %1}, [%2];" : "=f"(w[b].x), "=f"(w[b].y) : "r"(ws + b * kBB * 8));
+#pragma unroll
+    for (int j = 0; j < TX; j++)
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[j][b].x), "=f"(v[j][b].y), "=f"(v[j][b].z), "=f"(v[j][b].w)
+                     : "r"(xa + j * xs * 8 + b * 16));
+  }
+  __device__ __forceinline__ void add(float2 (&acc)[TX]) const {
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+      for (int j = 0; j < TX; j++) {
+        cfma(acc[j], w[2 * b], make_float2(v[j][b].x, v[j][b].y));
+        cfma(acc[j], w[2 * b + 1], make_float2(v[j][b].z, v[j][b].w));
+      }
+  }
+};
+
+template <int TY, int TX>
+__global__ void __launch_bounds__(64 * TY, TX == 8 ? 0 : 2) k_near(
+    const float2 *__restrict__ x, const float2 *__restrict__ g, int64_t gstride, int mode,
+    const int *__restrict__ active, const float2 *__restrict__ loc_leaf, size_t mp, int ns,
+    const float2 *__restrict__ nearW, const float2 *__restrict__ basisT, float2 *__restrict__ y, int epi, int red,
+    const float2 *__restrict__ dot_a, double *__restrict__ part, int nleaf, int U, int tiles_x, int tiles_total) {
+  constexpr int kHalo = (TY + 2) * (TX + 2), kThreads = 64 * TY;
+  constexpr int kStages = near_stages(TX), kRows = near_rows(TX);
   const int rhs = blockIdx.y;
   if (inactive(active, rhs)) return;
-  extern __shared__ float2 sm[];
-  float2 *hx = sm;                          // [60 leaves][64]
-  float2 *ls = sm + kHaloLeaves * kBB;      // [32 leaves][ns]
+  extern __shared__ __align__(16) float2 sm[];
+  float2 *ring = sm;                              // [kStages][kRows][64]
+  float2 *hx = ring + kStages * kRows * kBB;      // [kHalo leaves][64]
+  float2 *ls = hx + kHalo * kBB;                  // [TY * TX leaves][ns]
   const int tile = blockIdx.x;
-  const int ty0 = (tile / tiles_x) * kNearTY, tx0 = (tile % tiles_x) * kNearTX;
+  const int ty0 = (tile / tiles_x) * TY, tx0 = (tile % tiles_x) * TX;
   const size_t rbase = (size_t)rhs * U;
   const float2 *gr = g ? g + rhs * gstride : nullptr;
   const bool do_near = (epi != EPI_L2P_ONLY);
+  constexpr int kNearSt = 9 * kBB / kRows;  // stages of the near field; L2P's follow
+  const int s0 = do_near ? 0 : kNearSt, s1 = kNearSt + (ns + kRows - 1) / kRows;
+  auto fill = [&](int s) {  // stage s into its ring slot, two weights per copy
+    if (s < s1) {
+      const int rows = s < kNearSt ? kRows : min(kRows, ns - (s - kNearSt) * kRows);
+      const float2 *src = s < kNearSt ? nearW + (size_t)s * kRows * kBB : basisT + (size_t)(s - kNearSt) * kRows * kBB;
+      float2 *dst = ring + (s % max(1, kStages)) * kRows * kBB;
+      for (int e = threadIdx.x; e < rows * kBB / 2; e += kThreads) cp_async16(dst + 2 * e, src + 2 * e);
+    }
+    cp_async_commit();
+  };
+  if constexpr (kStages > 0)
+    for (int s = 0; s < kStages - 1; s++) fill(s0 + s);
   if (do_near) {
-    for (int e = threadIdx.x; e < kHaloLeaves * kBB; e += blockDim.x) {
+    for (int e = threadIdx.x; e < kHalo * kBB; e += kThreads) {
       const int h = e / kBB, p = e % kBB;
-      const int ly = ty0 - 1 + h / (kNearTX + 2), lx = tx0 - 1 + h % (kNearTX + 2);
+      const int ly = ty0 - 1 + h / (TX + 2), lx = tx0 - 1 + h % (TX + 2);
       float2 v = make_float2(0.f, 0.f);
       if (ly >= 0 && ly < nleaf && lx >= 0 && lx < nleaf) {
         const size_t i = (size_t)(ly * nleaf + lx) * kBB + p;
@@ -524,46 +657,77 @@ __global__ void __launch_bounds__(256) k_near(const float2 *__restrict__ x, cons
     }
   }
   const float2 *lr = loc_leaf + (size_t)rhs * mp;
-  for (int e = threadIdx.x; e < kNearTY * kNearTX * ns; e += blockDim.x) {
+  for (int e = threadIdx.x; e < TY * TX * ns; e += kThreads) {
     const int j = e / ns, k = e % ns;
-    const int ly = ty0 + j / kNearTX, lx = tx0 + j % kNearTX;
+    const int ly = ty0 + j / TX, lx = tx0 + j % TX;
     float2 v = make_float2(0.f, 0.f);
     if (ly < nleaf && lx < nleaf) v = lr[(size_t)(ly * nleaf + lx) * ns + k];
     ls[e] = v;
   }
-  __syncthreads();
 
   const int t = threadIdx.x & (kBB - 1), row = threadIdx.x >> 6;
-  float2 acc[kNearTX];
+  float2 acc[TX];
 #pragma unroll
-  for (int j = 0; j < kNearTX; j++) acc[j] = make_float2(0.f, 0.f);
-  if (do_near) {
-    for (int s = 0; s < 9; s++) {
-      const int dr = s / 3 - 1, dc = s % 3 - 1;
-      const float2 *W = nearW + s * kBB * kBB + t;
-      const float2 *hrow = hx + ((row + 1 + dr) * (kNearTX + 2) + 1 + dc) * kBB;
+  for (int j = 0; j < TX; j++) acc[j] = make_float2(0.f, 0.f);
+  if constexpr (kStages > 0) {
+#pragma unroll 1
+    for (int s = s0; s < s1; s++) {
+      cp_async_wait_group<kStages - 2>();  // this thread's share of stage s has landed,
+      __syncthreads();                     // every thread's, and the slot of stage s - 1 is read out
+      fill(s + kStages - 1);
+      const float2 *w = ring + (s % kStages) * kRows * kBB + t;
+      if (s < kNearSt) {
+        const int sl = s * kRows / kBB, b0 = s * kRows % kBB;
+        const float2 *xv = hx + ((row + sl / 3) * (TX + 2) + sl % 3) * kBB + b0;
+        NearRows<TX> a, b;
+#pragma unroll
+        for (int r = 0; r < kRows; r += 16) {
+          a.load(w + r * kBB, xv + r, kBB);
+          b.load(w + (r + 8) * kBB, xv + r + 8, kBB);
+          a.add(acc);
+          b.add(acc);
+        }
+      } else {
+        const int k0 = (s - kNearSt) * kRows, n = min(kRows, ns - k0);
+        const float2 *xv = ls + row * TX * ns + k0;
+        int k = 0;
+        if (ns % 2 == 0)
+          for (; k + 8 <= n; k += 8) {
+            NearRows<TX> a;
+            a.load(w + k * kBB, xv + k, ns);
+            a.add(acc);
+          }
+        for (; k < n; k++) {
+          const float2 bv = w[k * kBB];
+#pragma unroll
+          for (int j = 0; j < TX; j++) cfma(acc[j], bv, xv[j * ns + k]);
+        }
+      }
+    }
+  } else {
+    __syncthreads();
+    for (int s = do_near ? 0 : 9; s < 9; s++) {
+      const float2 *W = nearW + s * kBB * kBB + t, *hrow = hx + ((row + s / 3) * (TX + 2) + s % 3) * kBB;
 #pragma unroll 4
       for (int b = 0; b < kBB; b++) {
         const float2 w = __ldg(&W[b * kBB]);
 #pragma unroll
-        for (int j = 0; j < kNearTX; j++) cfma(acc[j], w, hrow[j * kBB + b]);
+        for (int j = 0; j < TX; j++) cfma(acc[j], w, hrow[j * kBB + b]);
       }
     }
-  }
-  {
-    const float2 *lrow = ls + row * kNearTX * ns;
+    const float2 *lrow = ls + row * TX * ns;
 #pragma unroll 4
     for (int k = 0; k < ns; k++) {
       const float2 bv = __ldg(&basisT[k * kBB + t]);
 #pragma unroll
-      for (int j = 0; j < kNearTX; j++) cfma(acc[j], bv, lrow[j * ns + k]);
+      for (int j = 0; j < TX; j++) cfma(acc[j], bv, lrow[j * ns + k]);
     }
   }
 
   double r0 = 0, r1 = 0, r2 = 0;
   const int ly = ty0 + row;
 #pragma unroll
-  for (int j = 0; j < kNearTX; j++) {
+  for (int j = 0; j < TX; j++) {
     const int lx = tx0 + j;
     if (ly >= nleaf || lx >= nleaf) continue;
     const size_t i = (size_t)(ly * nleaf + lx) * kBB + t;
@@ -588,7 +752,7 @@ __global__ void __launch_bounds__(256) k_near(const float2 *__restrict__ x, cons
     }
   }
   if (red != RED_NONE) {
-    __shared__ double wsum[8][3];
+    __shared__ double wsum[kThreads / 32][3];
     r0 = warp_sum(r0);
     r1 = warp_sum(r1);
     r2 = warp_sum(r2);
@@ -601,10 +765,10 @@ __global__ void __launch_bounds__(256) k_near(const float2 *__restrict__ x, cons
     __syncthreads();
     if (threadIdx.x == 0) {
       double s0 = 0, s1 = 0, s2 = 0;
-      for (int q = 0; q < 8; q++) {
-        s0 += wsum[q][0];
-        s1 += wsum[q][1];
-        s2 += wsum[q][2];
+      for (int p = 0; p < kThreads / 32; p++) {
+        s0 += wsum[p][0];
+        s1 += wsum[p][1];
+        s2 += wsum[p][2];
       }
       double *p = part + ((size_t)rhs * tiles_total + tile) * 4;
       p[0] = s0;
@@ -658,11 +822,12 @@ __global__ void k_permute(const int *__restrict__ perm, const float2 *__restrict
 }  // namespace
 
 void launch_p2m(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
-  const int nleaves = P.nleaf * P.nleaf;
-  dim3 grid((nleaves + 31) / 32, B.nrhs);
   count_launch();
-  k_p2m<<<grid, 128, 0, st>>>(B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U,
-                              mul + P.lv[P.L - 1].off, P.mp);
+  switch (p2m_shape(P, B.nrhs)) {
+    case P2M_2_1: return p2m_as<2, 1>(P, B, mul, st);
+    case P2M_8_2: return p2m_as<8, 2>(P, B, mul, st);
+    case P2M_32_4: return p2m_as<32, 4>(P, B, mul, st);
+  }
 }
 
 static TileArgs tile_args(const float2 *src, float2 *dst, size_t mp, size_t off_in, size_t off_out, int n_p,
@@ -683,6 +848,21 @@ static TileArgs tile_args(const float2 *src, float2 *dst, size_t mp, size_t off_
   A.tb = tb;
   A.shT = shT;
   A.active = active;
+// Leaves per block and per thread of k_p2m.
+enum P2mShape { P2M_2_1, P2M_8_2, P2M_32_4 };
+static P2mShape p2m_shape(const DevPlan &P, int nrhs) {
+  const int64_t leaves = (int64_t)P.nleaf * P.nleaf * nrhs;
+  return leaves <= kP2mSmall ? P2M_2_1 : leaves <= kP2mMid ? P2M_8_2 : P2M_32_4;
+}
+
+template <int LB, int LT>
+static void p2m_as(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
+  const int nleaves = P.nleaf * P.nleaf, units = LB / LT * P.ns_leaf;
+  const int threads = LB == 32 ? 128 : std::min(288, (units + 31) / 32 * 32);
+  k_p2m<LB, LT><<<dim3((nleaves + LB - 1) / LB, B.nrhs), threads, 0, st>>>(
+      B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U, mul + P.lv[P.L - 1].off, P.mp);
+}
+
   return A;
 }
 
@@ -712,8 +892,18 @@ void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int n
   A.zeros = P.zeros;
   A.locmax = locmax;
   A.lvl = lvl;
+int64_t level_outputs(const DevPlan &P, int lvl, int nrhs) {
+  return (int64_t)P.lv[lvl].n * P.lv[lvl].n * P.lv[lvl].ns * nrhs;
+}
+
   // two sibling-group columns per thread where the level has at least four
   const int half = c.n / 2, nc = half >= 4 ? 2 : 1, bx = (half / nc * c.ns + 127) / 128;
+  if (level_outputs(P, lvl, nrhs) <= kM2mDirect) {
+    const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
+    count_launch();
+    k_m2m_direct<<<dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    return;
+  }
   // eight groups per thread when the grid stays large, fewer for small batches
   int ty = std::min(8, half);
   while (ty > 1 && (size_t)bx * ((half + ty - 1) / ty) * nrhs < 4 * 148) ty /= 2;
@@ -744,24 +934,54 @@ void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *act
   k_l2l_tile<<<dim3((A.ncols + A.cols - 1) / A.cols, c.at.tiles), A.cols * (c.at.out / kTileOut), smem, st>>>(A);
 }
 
-int near_blocks_per_rhs(const DevPlan &P) {
-  const int ty = (P.nleaf + kNearTY - 1) / kNearTY, tx = (P.nleaf + kNearTX - 1) / kNearTX;
-  return ty * tx;
+// Leaf rows and columns of a near-field tile (k_near).
+struct NearShape {
+  int ty, tx;
+};
+static NearShape near_shape(const DevPlan &P, int nrhs) {
+  const int64_t leaves = (int64_t)P.nleaf * P.nleaf * nrhs;
+  if (leaves <= kNearSmall) return {2, 2};
+  if (leaves <= kNearMid) return {4, 4};
+  return {4, 8};
+}
+
+int near_blocks_per_rhs(const DevPlan &P, int nrhs) {
+  const NearShape s = near_shape(P, nrhs);
+  return ((P.nleaf + s.ty - 1) / s.ty) * ((P.nleaf + s.tx - 1) / s.tx);
+}
+
+size_t near_partials(const DevPlan &P, int max_rhs) {
+  size_t m = 0;
+  for (int r = 1; r <= max_rhs; r++) m = std::max(m, (size_t)r * near_blocks_per_rhs(P, r));
+  return m;
+}
+
+template <int TY, int TX>
+static void near_as(const DevPlan &P, const NearArgs &A, cudaStream_t st) {
+  const int tiles_x = (P.nleaf + TX - 1) / TX, tiles = near_blocks_per_rhs(P, A.in.nrhs);
+  const size_t smem =
+      (size_t)((near_stages(TX) * near_rows(TX) + (TY + 2) * (TX + 2)) * kBB + TY * TX * P.ns_leaf) * sizeof(float2);
+  k_near<TY, TX><<<dim3(tiles, A.in.nrhs), 64 * TY, smem, st>>>(
+      A.in.x, A.in.g, A.in.gstride, A.in.mode, A.in.active, A.loc + P.lv[P.L - 1].off, P.mp, P.ns_leaf, P.nearW,
+      P.basisT, A.y, A.epi, A.red, A.dot_a, A.part, P.nleaf, P.U, tiles_x, tiles);
 }
 
 void launch_near(const DevPlan &P, const NearArgs &A, cudaStream_t st) {
-  const int tiles_x = (P.nleaf + kNearTX - 1) / kNearTX;
-  const int tiles = near_blocks_per_rhs(P);
-  const size_t smem = (size_t)(kHaloLeaves * kBB + kNearTY * kNearTX * P.ns_leaf) * sizeof(float2);
-  dim3 grid(tiles, A.in.nrhs);
   count_launch();
-  k_near<<<grid, 256, smem, st>>>(A.in.x, A.in.g, A.in.gstride, A.in.mode, A.in.active, A.loc + P.lv[P.L - 1].off,
-                                  P.mp, P.ns_leaf, P.nearW, P.basisT, A.y, A.epi, A.red, A.dot_a, A.part, P.nleaf,
-                                  P.U, tiles_x, tiles);
+  const NearShape s = near_shape(P, A.in.nrhs);
+  if (s.tx == 2) return near_as<2, 2>(P, A, st);
+  if (s.tx == 4) return near_as<4, 4>(P, A, st);
+  near_as<4, 8>(P, A, st);
 }
 
 void launch_rx_interp(const DevPlan &P, const float2 *mul, float2 *rx, int nrhs, cudaStream_t st) {
   dim3 grid((P.numrx + 127) / 128, nrhs);
+  if (level_outputs(P, lvl, nrhs) <= kL2lDirect) {
+    const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw, p.shl, active};
+    count_launch();
+    k_l2l_direct<<<dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    return;
+  }
   count_launch();
   k_rx_interp<<<grid, 128, 0, st>>>(mul + P.lv[0].off, P.mp, rx, P.numrx, P.lv[0].ns, P.hfirst, P.hw, P.ninter);
 }
@@ -797,7 +1017,9 @@ cudaError_t kernels_setup() {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e == cudaSuccess) e = allow_max_smem(k_m2m_tile, optin);
   if (e == cudaSuccess) e = allow_max_smem(k_l2l_tile, optin);
-  if (e == cudaSuccess) e = allow_max_smem(k_near, optin);
+  if (e == cudaSuccess) e = allow_max_smem(k_near<4, 8>, optin);
+  if (e == cudaSuccess) e = allow_max_smem(k_near<4, 4>, optin);
+  if (e == cudaSuccess) e = allow_max_smem(k_near<2, 2>, optin);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_m2l<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m2l_smem(1));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_m2l<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m2l_smem(1));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_m2l<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m2l_smem(2));
@@ -808,7 +1030,10 @@ cudaError_t kernels_setup() {
 cudaError_t aggregate_kernels_load() {
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, k_permute);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<2, 1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<8, 2>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<32, 4>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_direct);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_tile);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_rx_interp);
   return e;

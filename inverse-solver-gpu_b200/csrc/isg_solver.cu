@@ -417,7 +417,7 @@ struct BicgsRun {
     kind = hermitian ? OP_ADJ : OP_FWD;
     engine = o->engine;
     nbv = c->vec_blocks;
-    nbn = (engine == ISG_ENGINE_TENSOR && tc_available(c)) ? tc_near_blocks(c) : near_blocks_per_rhs(c->P);
+    nbn = (engine == ISG_ENGINE_TENSOR && tc_available(c)) ? tc_near_blocks(c) : near_blocks_per_rhs(c->P, R);
     check = std::max(1, o->check_every);
     zero_guess = o->guess == ISG_GUESS_ZERO;
     gx = (kind == OP_FWD && engine == ISG_ENGINE_TENSOR && tc_available(c)) ? c->vgx : nullptr;

@@ -47,6 +47,11 @@ constexpr int kAHalf = 128 * kKC * 2;    // 16 KB: one FP16 split of an A chunk
 constexpr int kBHalf = kCols * kKC * 2;  // 16 KB
 constexpr int kSmem = 2 * kAHalf + 2 * kBHalf + 256 + 4 * kParents;  // + barriers, TMEM slot, scratch, per-parent maxima and flags
 constexpr int kErrBand = 121;
+// Largest level (samples of all clusters and RHS) that M2M leaves to the direct
+// kernel, where k_tc_m2m and where k_tc_band would take it: M2M of all levels
+// with and without, 256 x 256 x 1 at 11264 samples 29.7 / 30.7 us, at 26624
+// 31.9 / 29.7; 256 x 256 x 16 at 78848 34.1 / 38.4, x 64 at 142336 58.3 / 58.4.
+constexpr int64_t kPipeDirect = 16000, kBandDirect = 140000;
 
 struct BandArgs {
   const float2 *src;  // child-level multipoles (level base)
@@ -999,6 +1004,10 @@ static isg_status band_launch(isg_ctx *c, int lvl, const Transition &T, const fl
 bool band_m2m(isg_ctx *c, int lvl, float2 *mul, int nrhs, const int *active, cudaStream_t st, isg_status *e) {
   if (!c->band || lvl >= kMaxLevels) return false;
   const DevLevel &p = c->P.lv[lvl], &ch = c->P.lv[lvl + 1];
+  // Small launches take launch_m2m's one thread per output.  Every coarser level
+  // is smaller and has at most the same bound, so no kernel that needs this
+  // level's maximum follows.  At the bound both take 10 to 14 us.
+  if (level_outputs(c->P, lvl, nrhs) <= (c->band->pm2m[lvl].ok ? kPipeDirect : kBandDirect)) return false;
   if (c->band->pm2m[lvl].ok) {
     const M2mPlan &T = c->band->pm2m[lvl];
     M2mArgs A;
