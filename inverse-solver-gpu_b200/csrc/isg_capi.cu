@@ -496,9 +496,17 @@ isg_status isg_matvec(isg_ctx *c, const void *x, const void *g, int64_t g_stride
   const float2 *gb = nullptr;
   if ((e = contrast(c, g, g_stride, nrhs, order, st, &gb)) != ISG_OK) return e;
   const int64_t gs = (g_stride && order != ISG_ORDER_BLOCKED) ? c->P.U : g_stride;
-  const float2 *xb = to_blocked(c, x, c->wx, nrhs, order, st);
+  const float2 *xb, *gx = nullptr;
+  if (order != ISG_ORDER_BLOCKED && !hermitian && engine == ISG_ENGINE_TENSOR && tc_available(c)) {
+    // g x in the reordering's own pass
+    launch_permute_g(perm_for(c, order), (const float2 *)x, c->wx, gb, gs, c->vgx, c->P.U, nrhs, st);
+    xb = c->wx;
+    gx = c->vgx;
+  } else {
+    xb = to_blocked(c, x, c->wx, nrhs, order, st);
+  }
   float2 *yb = order == ISG_ORDER_BLOCKED ? (float2 *)y : c->wy;
-  e = run_matvec(c, xb, gb, gs, yb, nrhs, hermitian ? OP_ADJ : OP_FWD, engine, RED_NONE, nullptr, nullptr, st);
+  e = run_matvec(c, xb, gb, gs, yb, nrhs, hermitian ? OP_ADJ : OP_FWD, engine, RED_NONE, nullptr, nullptr, st, gx);
   if (e != ISG_OK) return e;
   from_blocked(c, yb, y, nrhs, order, st);
   return cuda_check(c, cudaGetLastError(), "matvec");
@@ -645,6 +653,8 @@ isg_status isg_receive(isg_ctx *c, const void *x, void *rx, int nrhs, int order,
   if (e != ISG_OK) return e;
   if (!x || !rx || bad_order(order) || (e = check_batch(c, nrhs)) != ISG_OK) return ISG_BAD_ARG;
   cudaStream_t st = pick(c, stream);
+  if (rxnear_active(c))  // reads the caller's order in place
+    return rxnear_apply(c, (const float2 *)x, (float2 *)rx, nrhs, 0, perm_for(c, order), st);
   return run_receive(c, to_blocked(c, x, c->wx, nrhs, order, st), (float2 *)rx, nrhs, st);
 }
 
@@ -653,10 +663,10 @@ isg_status isg_receiveh(isg_ctx *c, void *x, const void *rx, int nrhs, int order
   if (e != ISG_OK) return e;
   if (!x || !rx || bad_order(order) || (e = check_batch(c, nrhs)) != ISG_OK) return ISG_BAD_ARG;
   cudaStream_t st = pick(c, stream);
+  if (rxnear_active(c))  // writes the caller's order in place
+    return rxnear_apply(c, (const float2 *)rx, (float2 *)x, nrhs, 1, perm_for(c, order), st);
   float2 *y = order == ISG_ORDER_BLOCKED ? (float2 *)x : c->wy;
   if ((e = run_receiveh(c, y, (const float2 *)rx, nrhs, st)) != ISG_OK) return e;
-  if (rxnear_active(c))  // reads the caller's order in place
-    return rxnear_apply(c, (const float2 *)x, (float2 *)rx, nrhs, 0, perm_for(c, order), st);
   from_blocked(c, y, x, nrhs, order, st);
   return cuda_check(c, cudaGetLastError(), "receiveh");
 }
@@ -665,8 +675,6 @@ int64_t isg_kernel_launches(void) { return launch_count(); }
 
 isg_status isg_time_stages(isg_ctx *c, int nrhs, int engine, int reps, double *ms) {
   isg_status e = need_gpu(c);
-  if (rxnear_active(c))  // writes the caller's order in place
-    return rxnear_apply(c, (const float2 *)rx, (float2 *)x, nrhs, 1, perm_for(c, order), st);
   if (e != ISG_OK) return e;
   if (!ms || reps < 1 || (e = check_batch(c, nrhs)) != ISG_OK) return ISG_BAD_ARG;
   if (engine == ISG_ENGINE_TENSOR && !tc_available(c)) return ISG_UNSUPPORTED;

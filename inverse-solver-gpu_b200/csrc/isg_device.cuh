@@ -181,6 +181,12 @@ int64_t level_outputs(const DevPlan &P, int lvl, int nrhs);
 void launch_near(const DevPlan &P, const NearArgs &A, cudaStream_t st);
 void launch_rx_interp(const DevPlan &P, const float2 *mul, float2 *rx, int nrhs, cudaStream_t st);
 void launch_rx_anterp(const DevPlan &P, const float2 *rx, float2 *loc, int nrhs, float2 scale, cudaStream_t st);
+// launch_permute's gather with gx = g x of the reordered vectors in the same pass
+void launch_permute_g(const int *perm, const float2 *in, float2 *out, const float2 *g, int64_t gstride, float2 *gx,
+                      int U, int nrhs, cudaStream_t st);
+// gx = g x per RHS (16-byte aligned vectors, even gstride)
+void launch_gmul(const float2 *x, const float2 *g, int64_t gstride, float2 *gx, int U, int nrhs, const int *active,
+                 cudaStream_t st);
 void launch_permute(const int *perm, const float2 *in, float2 *out, int U, int nrhs, bool gather, cudaStream_t st);
 
 }  // namespace isg

@@ -819,7 +819,48 @@ __global__ void k_permute(const int *__restrict__ perm, const float2 *__restrict
   }
 }
 
+// k_permute's gather that also writes gx = g x (g already in the output order).
+__global__ void k_permute_g(const int *__restrict__ perm, const float2 *__restrict__ in, float2 *__restrict__ out,
+                            const float2 *__restrict__ g, int64_t gstride, float2 *__restrict__ gx, int U) {
+  const size_t r = blockIdx.y;
+  const float2 *gr = g + r * gstride;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < U; i += gridDim.x * blockDim.x) {
+    const float2 v = in[r * U + perm[i]];
+    out[r * U + i] = v;
+    gx[r * U + i] = cmul(gr[i], v);
+  }
+}
+
+// gx = g x, two elements a thread (16-byte aligned vectors, even U)
+__global__ void k_gmul(const float2 *__restrict__ x, const float2 *__restrict__ g, int64_t gstride,
+                       float2 *__restrict__ gx, int U, const int *__restrict__ active) {
+  const size_t r = blockIdx.y;
+  if (inactive(active, r)) return;
+  const float4 *xr = (const float4 *)(x + r * U), *gr = (const float4 *)(g + r * gstride);
+  float4 *o = (float4 *)(gx + r * U);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < U / 2; i += gridDim.x * blockDim.x) {
+    const float4 a = xr[i], b = __ldg(gr + i);
+    const float2 u = cmul(make_float2(b.x, b.y), make_float2(a.x, a.y)), v = cmul(make_float2(b.z, b.w), make_float2(a.z, a.w));
+    o[i] = make_float4(u.x, u.y, v.x, v.y);
+  }
+}
+
 }  // namespace
+
+// Leaves per block and per thread of k_p2m.
+enum P2mShape { P2M_2_1, P2M_8_2, P2M_32_4 };
+static P2mShape p2m_shape(const DevPlan &P, int nrhs) {
+  const int64_t leaves = (int64_t)P.nleaf * P.nleaf * nrhs;
+  return leaves <= kP2mSmall ? P2M_2_1 : leaves <= kP2mMid ? P2M_8_2 : P2M_32_4;
+}
+
+template <int LB, int LT>
+static void p2m_as(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
+  const int nleaves = P.nleaf * P.nleaf, units = LB / LT * P.ns_leaf;
+  const int threads = LB == 32 ? 128 : std::min(288, (units + 31) / 32 * 32);
+  k_p2m<LB, LT><<<dim3((nleaves + LB - 1) / LB, B.nrhs), threads, 0, st>>>(
+      B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U, mul + P.lv[P.L - 1].off, P.mp);
+}
 
 void launch_p2m(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
   count_launch();
@@ -866,8 +907,18 @@ static void p2m_as(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream
   return A;
 }
 
+int64_t level_outputs(const DevPlan &P, int lvl, int nrhs) {
+  return (int64_t)P.lv[lvl].n * P.lv[lvl].n * P.lv[lvl].ns * nrhs;
+}
+
 void launch_m2m(const DevPlan &P, int lvl, float2 *mul, int nrhs, const int *active, cudaStream_t st) {
   const DevLevel &p = P.lv[lvl], &c = P.lv[lvl + 1];
+  if (level_outputs(P, lvl, nrhs) <= kM2mDirect) {
+    const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
+    count_launch();
+    k_m2m_direct<<<dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    return;
+  }
   const int cap = (p.m2m_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? p.m2m_cols : 32;
   const TileArgs A = tile_args(mul, mul, P.mp, c.off, p.off, p.n, c.ns, p.ns, nrhs, p.mt, p.shmT, cap, active);
   const TileSmem L(p.mt.wmax, 4 * A.cols + 1, p.mt.out, 4 * A.cols, A.cols, (size_t)p.mt.out * (A.cols + 1));
@@ -926,6 +977,12 @@ int64_t level_outputs(const DevPlan &P, int lvl, int nrhs) {
 
 void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *active, cudaStream_t st) {
   const DevLevel &c = P.lv[lvl], &p = P.lv[lvl - 1];
+  if (level_outputs(P, lvl, nrhs) <= kL2lDirect) {
+    const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw, p.shl, active};
+    count_launch();
+    k_l2l_direct<<<dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    return;
+  }
   const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : 64;
   const TileArgs A = tile_args(loc, loc, P.mp, p.off, c.off, p.n, p.ns, c.ns, nrhs, c.at, p.shlT, cap, active);
   const TileSmem L(c.at.wmax, A.cols + 1, c.at.out, A.cols, 4 * A.cols, (size_t)4 * c.at.out * (A.cols + 1), true);
@@ -996,6 +1053,18 @@ void launch_permute(const int *perm, const float2 *in, float2 *out, int U, int n
   dim3 grid(std::min((U + 255) / 256, 1184), nrhs);
   count_launch();
   k_permute<<<grid, 256, 0, st>>>(perm, in, out, U, gather ? 1 : 0);
+}
+
+void launch_permute_g(const int *perm, const float2 *in, float2 *out, const float2 *g, int64_t gstride, float2 *gx,
+                      int U, int nrhs, cudaStream_t st) {
+  count_launch();
+  k_permute_g<<<dim3(std::min((U + 255) / 256, 1184), nrhs), 256, 0, st>>>(perm, in, out, g, gstride, gx, U);
+}
+
+void launch_gmul(const float2 *x, const float2 *g, int64_t gstride, float2 *gx, int U, int nrhs, const int *active,
+                 cudaStream_t st) {
+  count_launch();
+  k_gmul<<<dim3(std::min((U / 2 + 255) / 256, 1184), nrhs), 256, 0, st>>>(x, g, gstride, gx, U, active);
 }
 
 }  // namespace isg

@@ -352,9 +352,17 @@ isg_status run_matvec(isg_ctx *c, const float2 *x, const float2 *g, int64_t gs, 
   B.mode = (kind == OP_FWD) ? IN_G : (kind == OP_G ? IN_PLAIN : IN_CONJ);
   const bool tc = (engine == ISG_ENGINE_TENSOR) && tc_available(c);
   if (engine == ISG_ENGINE_TENSOR && !tc) return ISG_UNSUPPORTED;
-  // the tensor leaf kernels read g x directly when the caller already formed it
+  // The tensor leaf kernels read g x, formed once here unless the caller did: in
+  // the leaf kernels themselves it cost a load and a product per halo pixel and
+  // K-group (16 RHS at 1024 x 1024: 166 + 348 us of P2M and near field, against
+  // 66 + 278 us and this pass's 40).
   BatchArgs Bg = B;
-  const bool pre = tc && gx && kind == OP_FWD;
+  const bool pre = tc && kind == OP_FWD;
+  if (pre && !gx) {
+    if (((uintptr_t)x | (uintptr_t)g) & 15 || gs % 2) return ISG_UNSUPPORTED;
+    gx = c->vgx;
+    launch_gmul(x, g, gs, c->vgx, P.U, nrhs, active, st);
+  }
   if (pre) {
     Bg.x = gx;
     Bg.g = nullptr;

@@ -77,11 +77,6 @@ __device__ float loaders_max(float v, float *scratch) {
   return m;
 }
 
-__device__ __forceinline__ float2 transform(float2 v, float2 g, int mode) {
-  if (mode == IN_G) return cmul(g, v);
-  if (mode == IN_CONJ) return cconj(v);
-  return v;
-}
 
 __device__ __forceinline__ float cabs1(float2 v) { return fmaxf(fabsf(v.x), fabsf(v.y)); }
 
@@ -168,8 +163,8 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
 
   // ---- halo of the input: every thread stages x as FP32 with cp.async where its
   // FP16 halves will go (first two pixels of a 4-pixel chunk in the hi slot,
-  // last two in the lo slot); the loaders then form g x and its max in place,
-  // and convert to hi/lo once the pair's scale is known ----
+  // last two in the lo slot); the loaders then take its max (and conjugate) in
+  // place, and convert to hi/lo once the pair's scale is known ----
   // (halo row, 4-pixel chunk, halo column): consecutive items are consecutive
   // 16-byte slots, free of bank conflicts
   const int kItems = (A.pair * kTY + 2) * kHC * 16;
@@ -221,23 +216,13 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
     float mx = 0.f;
 #pragma unroll 8
     for (int it = li; it < kItems; it += kLoaders) {
-      const int hc = it % kHC, c = (it / kHC) & 15, hr = it / (kHC * 16);
-      const int off = hr * kSboA + c * kLboA + hc * 16;
+      const int hc = it % kHC, ck = (it / kHC) & 15, hr = it / (kHC * 16);
+      const int off = hr * kSboA + ck * kLboA + hc * 16;
       float4 *ph = (float4 *)(sm + NearSmem::hi + off), *pl = (float4 *)(sm + NearSmem::lo + off);
-      float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
-      if (A.mode == IN_G) {
-        const int ly = ty0 - 1 + hr, lx = tx0 - 1 + hc;
-        if (ly >= 0 && ly < A.nleaf && lx >= 0 && lx < A.nleaf) {
-          const size_t i = (size_t)(ly * A.nleaf + lx) * kBB + 4 * c;
-          g0 = *(const float4 *)(gr + i);
-          g1 = *(const float4 *)(gr + i + 2);
-        }
-      }
       const float4 a0 = *ph, a1 = *pl;
-      const float2 v0 = transform(make_float2(a0.x, a0.y), make_float2(g0.x, g0.y), A.mode);
-      const float2 v1 = transform(make_float2(a0.z, a0.w), make_float2(g0.z, g0.w), A.mode);
-      const float2 v2 = transform(make_float2(a1.x, a1.y), make_float2(g1.x, g1.y), A.mode);
-      const float2 v3 = transform(make_float2(a1.z, a1.w), make_float2(g1.z, g1.w), A.mode);
+      const float c = A.mode == IN_CONJ ? -1.f : 1.f;
+      const float2 v0 = make_float2(a0.x, c * a0.y), v1 = make_float2(a0.z, c * a0.w);
+      const float2 v2 = make_float2(a1.x, c * a1.y), v3 = make_float2(a1.z, c * a1.w);
       mx = fmaxf(mx, fmaxf(fmaxf(cabs1(v0), cabs1(v1)), fmaxf(cabs1(v2), cabs1(v3))));
       *ph = make_float4(v0.x, v0.y, v1.x, v1.y);
       *pl = make_float4(v2.x, v2.y, v3.x, v3.y);
@@ -483,12 +468,15 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
         s1v += dscr[w2 * 3 + 1];
         s2v += dscr[w2 * 3 + 2];
       }
-      const int tile = (pty * A.pair + u) * A.tiles_x + ptx;
-      double *p = A.part + ((size_t)rhs * A.tiles + tile) * 4;
-      p[0] = s0;
-      p[1] = s1v;
-      p[2] = s2v;
-      p[3] = 0;
+      // one record per 8 x 8 leaves: the tile's sum in its first, zero in its second
+      const int rows8 = (A.nleaf + 7) / 8, r0 = (ty0 + u * kTY) / 8;
+      for (int r = r0; r < min(rows8, r0 + kTY / 8); r++) {
+        double *p = A.part + (((size_t)rhs * rows8 + r) * A.tiles_x + ptx) * 4;
+        p[0] = r == r0 ? s0 : 0;
+        p[1] = r == r0 ? s1v : 0;
+        p[2] = r == r0 ? s2v : 0;
+        p[3] = 0;
+      }
     }
     __syncthreads();  // dscr is reused by the next tile
   }
@@ -498,13 +486,14 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
 }
 
 // ---- near field + L2P, persistent and pipelined ----
-// Items are pairs of vertically adjacent 16 x 8-leaf tiles of one RHS; a
-// persistent CTA walks them in steps of gridDim.x.  An item's K dimension (9
-// neighbour slots x 128 source reals of the halo, then 2 ns reals of the leaf
-// locals for L2P) is staged in shared memory one A-stage at a time: a halo
-// K-group (32 source reals of every leaf of the pair's 34 x 10-leaf halo)
-// feeds the nine weight stages of its K range; an L2P stage (32 reals of the
-// locals of the pair's 256 leaves) feeds one.  Stage order: H0 H1 H2 H3 L0 ..
+// Items are TR x 8 leaves of one RHS (TR = 32, or 16 or 8 where 32 would leave
+// SMs without an item, np_rows); a persistent CTA walks them in steps of
+// gridDim.x.  An item's K dimension (9 neighbour slots x 128 source reals of
+// the halo, then 2 ns reals of the leaf locals for L2P) is staged in shared
+// memory one A-stage at a time: a halo K-group (32 source reals of every leaf
+// of the item's (TR + 2) x 10-leaf halo) feeds the nine weight stages of its K
+// range; an L2P stage (32 reals of the locals of the item's 8 TR leaves) feeds
+// one.  Stage order: H0 H1 H2 H3 L0 ..
 // L4; the weights are packed in the same order.  An A-stage arrives as FP32 by
 // one tensor load whose rows are a leaf's 32 reals (128 contiguous bytes) into
 // a staging buffer, and the converters write it as FP16 hi/lo in the MMA's
@@ -515,11 +504,11 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
 //   warp 1      bulk copies of the weight stages
 //   warp 2      MMA issue (one thread)
 //   warps 3..6  A-stage conversion to FP16 hi/lo
-//   warps 7..14 epilogue, two per TMEM lane quarter (columns 0..63, 64..127)
-// Near field and L2P accumulate into one TMEM accumulator per tile: the input
+//   warps 7..14 epilogue, two per TMEM lane quarter (an item's upper and lower leaf rows)
+// Near field and L2P accumulate into one TMEM accumulator per item: the input
 // is scaled by the power of two that P2M's per-RHS maximum gives and the
 // locals by M2L's, each lowered until both products carry the same power of
-// two.  Two accumulator sets (two tiles x 128 columns each) alternate between
+// two.  Two accumulator sets (256 columns each) alternate between
 // items, so an item's epilogue runs under the next item's MMAs.
 constexpr int kNpKC = 4;                                       // 8-real K-chunks per A-stage
 constexpr int kNpHaloSplit = kHR * kNpKC * kHC * 16;           // 21760: one FP16 split of a halo K-group
@@ -600,7 +589,7 @@ struct TcNearPipeArgs {
   int epi, red;
   const float2 *dot_a;
   double *part;
-  int nleaf, U, tiles_x, tiles_y, tiles, ppr, nitems;
+  int nleaf, U, tiles_x, ppr, nitems;  // items of TR x kTX leaves: columns, per RHS, in all
   int *err;
 };
 
@@ -617,6 +606,7 @@ __device__ __forceinline__ void np_scales(const TcNearPipeArgs &A, int rhs, floa
   s2 = p / A.sb;
 }
 
+template <int TR>
 __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A, const __grid_constant__ CUtensorMap tmh,
                                                                 const __grid_constant__ CUtensorMap tml) {
   extern __shared__ __align__(1024) char sm[];
@@ -638,7 +628,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tslot;  // set s, tile u: columns [256 s + 128 u, +128)
+  const uint32_t tmem = *tslot;  // set s: columns [256 s, +8 TR)
   const int na = 4 + A.nl2p;     // A-stages per item
   const int nb = 36 + A.nl2p;    // weight stages per item
   auto next_item = [&](int w) {
@@ -648,13 +638,13 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
   };
   const int first = (A.active && blockIdx.x < A.nitems && !A.active[blockIdx.x / A.ppr]) ? next_item(blockIdx.x)
                                                                                            : blockIdx.x;
-  auto geom = [&](int w, int &rhs, int &ty0, int &tx0, int &ntile) {
+  auto geom = [&](int w, int &rhs, int &ty0, int &tx0) {
     rhs = w / A.ppr;
     const int pr = w % A.ppr, pty = pr / A.tiles_x, ptx = pr % A.tiles_x;
-    ty0 = pty * kPair * kTY;
+    ty0 = pty * TR;
     tx0 = ptx * kTX;
-    ntile = min(kPair, A.tiles_y - pty * kPair);
   };
+  const uint32_t halo_bytes = (uint32_t)(TR + 2) * kHC * 32 * 4, l2p_bytes = (uint32_t)TR * kTX * 32 * 4;
 
   if (warp == 0) {
     // ---- A-stage tensor loads into the staging buffers: rows of 32 reals ----
@@ -662,14 +652,14 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       int ka = 0;
       const bool pre_x = A.epi == EPI_FWD || A.epi == EPI_ADJ || A.red == RED_TS;
       for (int w = first; w < A.nitems && !*abort; w = next_item(w)) {
-        int rhs, ty0, tx0, ntile;
-        geom(w, rhs, ty0, tx0, ntile);
+        int rhs, ty0, tx0;
+        geom(w, rhs, ty0, tx0);
         // the rows the epilogue will read for this item (x, the dot vector, g), into L2
         // about one item ahead of it: its loads then wait on L2, not on HBM
         {
           const uint32_t run = (uint32_t)min(kTX, A.nleaf - tx0) * kBB * 8;
           const size_t rb = (size_t)rhs * A.U;
-          for (int r = 0; r < ntile * kTY && ty0 + r < A.nleaf; r++) {
+          for (int r = 0; r < TR && ty0 + r < A.nleaf; r++) {
             const size_t at = (size_t)((ty0 + r) * A.nleaf + tx0) * kBB;
             if (pre_x) bulk_prefetch_l2(A.xe + rb + at, run);
             if (A.red == RED_DOT) bulk_prefetch_l2(A.dot_a + rb + at, run);
@@ -682,10 +672,10 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
           char *dst = sm + NpSmem::s + i * kNpBuf;
           int idx;
           if (np_stage(a, A.nl2p, idx) == 0) {
-            mbar_expect_tx(sfull + i, kNpHaloBytes);
+            mbar_expect_tx(sfull + i, halo_bytes);
             tma_load_4d(dst, &tmh, 32 * idx, tx0 - 1, ty0 - 1, rhs, sfull + i);
           } else {
-            mbar_expect_tx(sfull + i, kNpL2pBytes);
+            mbar_expect_tx(sfull + i, l2p_bytes);
             tma_load_4d(dst, &tml, 32 * idx, tx0, ty0, rhs, sfull + i);
           }
         }
@@ -714,11 +704,11 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       }
     }
   } else if (warp == 2) {
-    // ---- MMA issue (one thread): D[128 target reals][256 leaves of the pair] +=
-    // weights (A, M = 128) x data (B, N = 256): both tiles in one instruction, so
-    // each weight stage is 2 K-steps x 3 split products ----
+    // ---- MMA issue (one thread): D[128 target reals][8 TR leaves of the item] +=
+    // weights (A, M = 128) x data (B, N = 8 TR): each weight stage is 2 K-steps x
+    // 3 split products ----
     if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(128, 2 * 128), sbase = smem_u32(sm);
+      const uint32_t idesc = idesc_f16_f32(128, kTX * TR), sbase = smem_u32(sm);
       int ka = 0, kb = 0, it = 0;
       bool ok = true;
       for (int w = first; w < A.nitems && ok; w = next_item(w), it++) {
@@ -742,7 +732,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
             if (!ok) break;
             const uint32_t bb = sbase + NpSmem::b + b * kStageBytes;
             const uint64_t wh0 = smem_desc(bb, 128, 512), wl0 = smem_desc(bb + kStageHalf, 128, 512);
-            // neighbour slot q: the pair's 32 leaf rows start at halo row 1 + dr, column 1 + dc
+            // neighbour slot q: the item's leaf rows start at halo row 1 + dr, column 1 + dc
             const uint32_t doff0 = kind == 0 ? (uint32_t)((q / 3) * (kNpKC * kHC * 16) + (q % 3) * 16) : 0u;
 #pragma unroll
             for (int ks = 0; ks < 2; ks++) {
@@ -769,11 +759,8 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     const int ct = threadIdx.x - 32 * kNpConvWarp0;
     int ka = 0;
     for (int w = first; w < A.nitems; w = next_item(w)) {
-      int rhs, ty0, tx0, ntile;
-      geom(w, rhs, ty0, tx0, ntile);
       float s1, s2, p;
-      np_scales(A, rhs, s1, s2, p);
-      const float2 *gr = A.g ? A.g + rhs * A.gstride : nullptr;
+      np_scales(A, w / A.ppr, s1, s2, p);
       for (int a = 0; a < na; a++, ka++) {
         const int i = ka % kNpNS, o = ka % kNpNO;
         const bool ok = mbar_wait_or(sfull + i, (ka / kNpNS) & 1, abort, A.err, kErrNp) &&
@@ -783,34 +770,22 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         int idx;
         if (np_stage(a, A.nl2p, idx) == 0) {
           char *lo = hi + kNpHaloSplit;
-          for (int e = ct; e < kHR * kHC * kNpKC && ok; e += kNpConv) {
+          for (int e = ct; e < (TR + 2) * kHC * kNpKC && ok; e += kNpConv) {
             const int c = e & 3, hc = (e >> 2) % kHC, hr = (e >> 2) / kHC;
             const float4 a0 = st[2 * e], a1 = st[2 * e + 1];  // staging offset ((hr * 10 + hc) * 32 + 8 c) reals
-            float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
-            if (A.mode == IN_G) {
-              const int ly = ty0 - 1 + hr, lx = tx0 - 1 + hc;
-              if (ly >= 0 && ly < A.nleaf && lx >= 0 && lx < A.nleaf) {
-                const size_t gi = (size_t)(ly * A.nleaf + lx) * kBB + 16 * idx + 4 * c;
-                g0 = *(const float4 *)(gr + gi);
-                g1 = *(const float4 *)(gr + gi + 2);
-              }
-            }
-            const float2 v0 = transform(make_float2(a0.x, a0.y), make_float2(g0.x, g0.y), A.mode);
-            const float2 v1 = transform(make_float2(a0.z, a0.w), make_float2(g0.z, g0.w), A.mode);
-            const float2 v2 = transform(make_float2(a1.x, a1.y), make_float2(g1.x, g1.y), A.mode);
-            const float2 v3 = transform(make_float2(a1.z, a1.w), make_float2(g1.z, g1.w), A.mode);
+            const float si = A.mode == IN_CONJ ? -s1 : s1;    // the imaginary parts' sign
             uint32_t h[4], l[4];
-            split2u(v0.x * s1, v0.y * s1, h[0], l[0]);
-            split2u(v1.x * s1, v1.y * s1, h[1], l[1]);
-            split2u(v2.x * s1, v2.y * s1, h[2], l[2]);
-            split2u(v3.x * s1, v3.y * s1, h[3], l[3]);
+            split2u(a0.x * s1, a0.y * si, h[0], l[0]);
+            split2u(a0.z * s1, a0.w * si, h[1], l[1]);
+            split2u(a1.x * s1, a1.y * si, h[2], l[2]);
+            split2u(a1.z * s1, a1.w * si, h[3], l[3]);
             const int off = ((hr * kNpKC + c) * kHC + hc) * 16;
             st_shared_v4(hi + off, h);
             st_shared_v4(lo + off, l);
           }
         } else {
           char *lo = hi + kNpL2pSplit;
-          for (int e = ct; e < kPair * kTY * kTX * kNpKC && ok; e += kNpConv) {
+          for (int e = ct; e < TR * kTX * kNpKC && ok; e += kNpConv) {
             const int c = e & 3, col = (e >> 2) & (kTX - 1), row = e >> 5;
             const float4 a0 = st[2 * e], a1 = st[2 * e + 1];  // staging offset ((row * 8 + col) * 32 + 8 c) reals
             uint32_t h[4], l[4];
@@ -833,9 +808,9 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     }
   } else {
     // ---- epilogue: TMEM lane = target real (pixel 16 qd + lane / 2, real part on
-    // even lanes), column = leaf of the pair; the warp's 32 lanes are 128 contiguous
+    // even lanes), column = leaf of the item; the warp's 32 lanes are 128 contiguous
     // bytes of one leaf's output, so every load and store is one coalesced row.
-    // Warps 7..10 take the pair's first tile (columns 0..127), 11..14 the second ----
+    // Warps 7..10 take the item's first TR / 2 leaf rows (columns 0 .. 4 TR - 1), 11..14 the rest ----
     const int ew = warp - kNpEpiWarp0, qd = warp & 3, hh = ew >> 2;
     const bool odd = lane & 1;
     const bool need_x = A.epi == EPI_FWD || A.epi == EPI_ADJ || A.red == RED_TS;
@@ -843,13 +818,14 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     float *yf = (float *)A.y;
     int it = 0;
     for (int w = first; w < A.nitems; w = next_item(w), it++) {
-      int rhs, ty0, tx0, ntile;
-      geom(w, rhs, ty0, tx0, ntile);
+      int rhs, ty0, tx0;
+      geom(w, rhs, ty0, tx0);
       const int set = it & 1;
       float s1, s2, p;
       np_scales(A, rhs, s1, s2, p);
       const float inv = 1.f / p;
       const bool ok = mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNp);
+      __syncwarp();  // the lanes leave the wait one by one; the TMEM loads are .aligned
       tc_fence_after();
       const size_t rbase = (size_t)rhs * A.U;
       const float *gf = A.g ? (const float *)(A.g + rhs * A.gstride) : nullptr;
@@ -857,10 +833,10 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       float *yr = yf + 2 * rbase;
       double r0 = 0, r1 = 0, r2 = 0;
       Acc32 q0, q1, q2;
-      if (hh < ntile) {  // warp-uniform
-        // chunks of 8 leaves (one leaf row of the tile); the loads of chunk ch + 1 are in
-        // flight while chunk ch is computed and stored
-        const int lyb = ty0 + hh * kTY;
+      const int nch = TR / 2, lyb = ty0 + hh * nch;  // the warp's leaf rows (an even number)
+      if (lyb < A.nleaf) {  // warp-uniform
+        // chunks of 8 leaves (one leaf row); the loads of chunk ch + 1 are in flight while
+        // chunk ch is computed and stored
         auto fidx = [&](int ch, int j) { return 2 * ((lyb + ch) * A.nleaf + tx0 + j) * kBB + 32 * qd + lane; };
         auto load = [&](int ch, float (&xv)[8], float (&av)[8], float (&gv)[8], unsigned &live) {
           live = 0;
@@ -876,7 +852,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         };
         auto process = [&](int ch, const float (&xv)[8], const float (&av)[8], const float (&gv)[8], unsigned live) {
           float d[8];
-          tmem_ld8(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(set * 256 + 128 * hh + 8 * ch), d);
+          tmem_ld8(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(set * 256 + kTX * (hh * nch + ch)), d);
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             if (!((live >> j) & 1)) continue;  // warp-uniform
@@ -912,10 +888,10 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         unsigned la, lb;
         load(0, xa, aa, ga, la);
 #pragma unroll 1
-        for (int ch = 0; ch < 16; ch += 2) {
+        for (int ch = 0; ch < nch; ch += 2) {
           load(ch + 1, xb, ab, gb, lb);
           process(ch, xa, aa, ga, la);
-          if (ch + 2 < 16) load(ch + 2, xa, aa, ga, la);
+          if (ch + 2 < nch) load(ch + 2, xa, aa, ga, la);
           process(ch + 1, xb, ab, gb, lb);
         }
       }
@@ -945,13 +921,14 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
             s1v += ds[1];
             s2v += ds[2];
           }
-          // the pair's sum goes to its first tile's slot, zero to the second's
-          const int pr = w % A.ppr, pty = pr / A.tiles_x, ptx = pr % A.tiles_x;
-          for (int u = 0; u < ntile; u++) {
-            double *pp = A.part + ((size_t)rhs * A.tiles + (pty * kPair + u) * A.tiles_x + ptx) * 4;
-            pp[0] = u ? 0.0 : s0;
-            pp[1] = u ? 0.0 : s1v;
-            pp[2] = u ? 0.0 : s2v;
+          // the item's sum goes to the record of its first 8 x 8 leaves, zero to the others'
+          const int rows8 = (A.nleaf + 7) / 8;
+          for (int r = ty0 / 8; r < min(rows8, (ty0 + TR) / 8); r++) {
+            const bool first8 = r == ty0 / 8;
+            double *pp = A.part + (((size_t)rhs * rows8 + r) * A.tiles_x + tx0 / kTX) * 4;
+            pp[0] = first8 ? s0 : 0.0;
+            pp[1] = first8 ? s1v : 0.0;
+            pp[2] = first8 ? s2v : 0.0;
             pp[3] = 0.0;
           }
         }
@@ -964,23 +941,11 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
 }
 
 // ---- P2M: persistent CTAs over (RHS, 128-leaf tile) items, N = 2 ns padded to 16 ----
-// The coefficient matrix is loaded once per CTA; each item's input is loaded
-// into registers while the previous item's outputs are written, converted to
-// FP16 hi/lo, multiplied, and its multipoles go back through shared memory so
-// that the 128 consecutive leaf rings are written as one contiguous block.
 constexpr int kP2mA = 16 * 2048;  // one FP16 split of the [128 x 128] operand
-struct P2mSmem {
-  static constexpr int hi = 0, lo = kP2mA, b = 2 * kP2mA;
-  // then: B (4 stages), output tile [128][ns + 1] float2, barriers
-  __host__ __device__ static size_t out(int stage_bytes) { return (size_t)b + 4 * (size_t)stage_bytes; }
-  __host__ __device__ static size_t bars(int stage_bytes, int ns) { return (out(stage_bytes) + (size_t)128 * (ns + 1) * 8 + 15) & ~(size_t)15; }
-  __host__ __device__ static size_t total(int stage_bytes, int ns) { return bars(stage_bytes, ns) + 64; }
-};
 
 struct TcP2mArgs {
-  const float2 *x, *g;
-  int64_t gstride;
-  int mode;
+  const float2 *x;
+  int conj;  // the input is conjugated
   const int *active;
   const uint8_t *B;  // 4 stages of [npad x 32] hi then lo
   int npad, stage_bytes;
@@ -993,173 +958,11 @@ struct TcP2mArgs {
   int lvl;
 };
 
-__global__ void __launch_bounds__(256, 1) k_tc_p2m(TcP2mArgs A) {
-  extern __shared__ __align__(1024) char sm[];
-  float2 *osm = (float2 *)(sm + P2mSmem::out(A.stage_bytes));
-  uint64_t *bar = (uint64_t *)(sm + P2mSmem::bars(A.stage_bytes, A.ns));
-  uint64_t *done = bar + 1;
-  uint32_t *tslot = (uint32_t *)(bar + 2);
-  float *fscr = (float *)(bar + 3);  // [8]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_init(done, 1);
-    fence_mbar_init();
-  }
-  if (warp == 0) tmem_alloc(tslot, 256);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tslot;
-  const int bbytes = 4 * A.stage_bytes;
-  if (threadIdx.x == 0) {
-    mbar_expect_tx(bar, bbytes);
-    for (int c = 0; c < 4; c++)
-      bulk_g2s(sm + P2mSmem::b + c * A.stage_bytes, A.B + (size_t)c * A.stage_bytes, A.stage_bytes, bar);
-  }
-  auto active_item = [&](int w) {
-    while (w < A.nitems && A.active && !A.active[w / A.tiles]) w += gridDim.x;
-    return w;
-  };
-  // one item's input: 128 leaves x 16 chunks of 4 pixels, 8 chunks per thread;
-  // chunk r of thread t is (row group, chunk, row in group) = it >> 7, (it >> 3) & 15, it & 7
-  constexpr int kPer = 128 * 16 / 256;
-  float2 v[kPer][4];
-  auto load = [&](int w, float &mx) {
-    const int rhs = w / A.tiles, leaf0 = (w % A.tiles) * 128;
-    const size_t rbase = (size_t)rhs * A.U;
-    const float2 *gr = A.g ? A.g + rhs * A.gstride : nullptr;
-    mx = 0.f;
-#pragma unroll
-    for (int r = 0; r < kPer; r++) {
-      const int it = threadIdx.x + r * 256;
-      const int m = ((it >> 7) << 3) | (it & 7), c = (it >> 3) & 15, leaf = leaf0 + m;
-#pragma unroll
-      for (int p = 0; p < 4; p++) v[r][p] = make_float2(0.f, 0.f);
-      if (leaf < A.nleaves) {
-        const size_t i = (size_t)leaf * kBB + 4 * c;
-        const float4 a0 = *(const float4 *)(A.x + rbase + i), a1 = *(const float4 *)(A.x + rbase + i + 2);
-        float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
-        if (A.mode == IN_G) {
-          g0 = *(const float4 *)(gr + i);
-          g1 = *(const float4 *)(gr + i + 2);
-        }
-        v[r][0] = transform(make_float2(a0.x, a0.y), make_float2(g0.x, g0.y), A.mode);
-        v[r][1] = transform(make_float2(a0.z, a0.w), make_float2(g0.z, g0.w), A.mode);
-        v[r][2] = transform(make_float2(a1.x, a1.y), make_float2(g1.x, g1.y), A.mode);
-        v[r][3] = transform(make_float2(a1.z, a1.w), make_float2(g1.z, g1.w), A.mode);
-#pragma unroll
-        for (int p = 0; p < 4; p++) mx = fmaxf(mx, cabs1(v[r][p]));
-      }
-    }
-  };
-  const uint32_t sbase = smem_u32(sm);
-  const uint32_t idesc = idesc_f16_f32(128, A.npad);
-  const int nchunks = A.npad / 16;
-  const int q = warp & 3, hh = warp >> 2;
-  const int c0 = hh ? (nchunks + 1) / 2 : 0, c1 = hh ? nchunks : (nchunks + 1) / 2;
-  bool ok = mbar_wait(bar, 0, A.err, kErrP2m);  // the coefficients
-  int parity = 0;
-  int w = active_item(blockIdx.x);
-  float mx = 0.f;
-  if (w < A.nitems) load(w, mx);
-  while (w < A.nitems) {
-    // scale, convert and store this item's operand; the previous item's MMAs are done
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) fscr[warp] = mx;
-    __syncthreads();
-    float m2 = 0.f;
-    for (int k = 0; k < 8; k++) m2 = fmaxf(m2, fscr[k]);
-    const float s = pow2_scale(m2);
-    // the input's maximum per RHS: the near-field kernel's scale for the same input
-    if (threadIdx.x == 0 && m2 > 0.f && A.lvl < kInMaxSlot)
-      atomicMax(&A.levmax[(w / A.tiles) * kMaxLevels + kInMaxSlot], __float_as_uint(m2));
-#pragma unroll
-    for (int r = 0; r < kPer; r++) {
-      const int it = threadIdx.x + r * 256;
-      __align__(16) __half h[8], l[8];
-#pragma unroll
-      for (int p = 0; p < 4; p++) {
-        split_f16(v[r][p].x * s, h[2 * p], l[2 * p]);
-        split_f16(v[r][p].y * s, h[2 * p + 1], l[2 * p + 1]);
-      }
-      const int off = it * 16;  // (it >> 7) * 2048 + ((it >> 3) & 15) * 128 + (it & 7) * 16
-      *(uint4 *)(sm + P2mSmem::hi + off) = *(uint4 *)h;
-      *(uint4 *)(sm + P2mSmem::lo + off) = *(uint4 *)l;
-    }
-    fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      if (ok) {
-        const uint64_t ah0 = smem_desc(sbase + P2mSmem::hi, 128, 2048);
-        const uint64_t al0 = smem_desc(sbase + P2mSmem::lo, 128, 2048);
-        const uint64_t bh0 = smem_desc(sbase + P2mSmem::b, 128, 512);
-        const uint64_t bl0 = smem_desc(sbase + P2mSmem::b + A.stage_bytes / 2, 128, 512);
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-          for (int ks = 0; ks < 2; ks++) {
-            const uint32_t aoff = (uint32_t)(c * 4 + ks * 2) * 128, boff = c * A.stage_bytes + ks * 256;
-            mma_f16(tmem, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, (c | ks) ? 1 : 0);
-            mma_f16(tmem, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, 1);
-            mma_f16(tmem, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
-          }
-      }
-      mma_commit(done);
-    }
-    // the next item's input, in flight while this one is multiplied and written
-    const int rhs = w / A.tiles, leaf0 = (w % A.tiles) * 128;
-    const int nxt = active_item(w + gridDim.x);
-    float mxn = 0.f;
-    if (nxt < A.nitems) load(nxt, mxn);
-    ok = mbar_wait(done, parity, A.err, kErrP2m) && ok;
-    parity ^= 1;
-    tc_fence_after();
-    const float inv = A.inv_c / s;
-    const int m = 32 * q + lane;
-    float omx = 0.f;
-    for (int ch = c0; ch < c1; ch++) {
-      float d[16];
-      tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + 16 * ch, d);
-#pragma unroll
-      for (int p = 0; p < 8; p++) {
-        const int k = 8 * ch + p;
-        if (k < A.ns) {
-          const float2 o = make_float2(d[2 * p] * inv, d[2 * p + 1] * inv);
-          osm[m * (A.ns + 1) + k] = o;
-          if (leaf0 + m < A.nleaves) omx = fmaxf(omx, fmaxf(fabsf(o.x), fabsf(o.y)));
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) omx = fmaxf(omx, __shfl_xor_sync(0xffffffffu, omx, o));
-    if (lane == 0 && ok) atomicMax(&A.levmax[rhs * kMaxLevels + A.lvl], __float_as_uint(omx));
-    tc_fence_before();
-    __syncthreads();
-    if (ok) {
-      const int nl = min(128, A.nleaves - leaf0);
-      float2 *out = A.mul_leaf + (size_t)rhs * A.mp + (size_t)leaf0 * A.ns;
-      for (int e = threadIdx.x; e < nl * A.ns; e += blockDim.x) {
-        const int mm = e / A.ns, k = e - mm * A.ns;
-        out[e] = osm[mm * (A.ns + 1) + k];
-      }
-    }
-    __syncthreads();  // the output tile and fscr are reused by the next item
-    w = nxt;
-    mx = mxn;
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
-}
-
-// ---- P2M, pipelined: converter, MMA and epilogue roles over double-buffered
-// A operands (128 leaves x 64 pixels x re, im, FP16 hi/lo) and TMEM
-// accumulators; the coefficients (B, 4 stages) stay resident.  The converters
-// load an item's pixels straight from global memory (every leaf is 512
-// contiguous bytes), apply the input transform, take the item's maximum among
-// themselves, and split.  The epilogue reads each leaf's ring from its TMEM
+// Converter, MMA and epilogue roles over double-buffered A operands (128 leaves
+// x 64 pixels x re, im, FP16 hi/lo) and TMEM accumulators; the coefficients (B,
+// 4 stages) stay resident.  An item's pixels (one contiguous run) are bulk-copied
+// as FP32 into the operand buffer they will fill; the converters take them into
+// registers, take the item's maximum among themselves, and split them in place.  The epilogue reads each leaf's ring from its TMEM
 // lane and turns lanes into contiguous runs through a small per-warp tile;
 // it keeps the level maximum for the M2M above. ----
 struct P2mPipeSmem {
@@ -1242,11 +1045,10 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
           const int odd = m & 1;
           const float4 x0 = zst[m * 32 + 2 * c + odd], x1 = zst[m * 32 + 2 * c + 1 - odd];
           const float4 a0 = odd ? x1 : x0, a1 = odd ? x0 : x1;
-          const float2 g0 = make_float2(0.f, 0.f);
-          v[r][0] = transform(make_float2(a0.x, a0.y), g0, A.mode);
-          v[r][1] = transform(make_float2(a0.z, a0.w), g0, A.mode);
-          v[r][2] = transform(make_float2(a1.x, a1.y), g0, A.mode);
-          v[r][3] = transform(make_float2(a1.z, a1.w), g0, A.mode);
+          v[r][0] = make_float2(a0.x, A.conj ? -a0.y : a0.y);
+          v[r][1] = make_float2(a0.z, A.conj ? -a0.w : a0.w);
+          v[r][2] = make_float2(a1.x, A.conj ? -a1.y : a1.y);
+          v[r][3] = make_float2(a1.z, A.conj ? -a1.w : a1.w);
 #pragma unroll
           for (int p = 0; p < 4; p++) mx = fmaxf(mx, cabs1(v[r][p]));
         }
@@ -1493,9 +1295,8 @@ isg_status tc_setup(isg_ctx *c) {
   cudaMemcpy(P.p2mB, pb.data(), pb.size(), cudaMemcpyHostToDevice);
   cudaMemset(P.err, 0, sizeof(int));
   cudaFuncSetAttribute(k_tc_near, cudaFuncAttributeMaxDynamicSharedMemorySize, NearSmem::total);
-  cudaFuncSetAttribute(k_tc_near_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, NpSmem::total);
-  cudaFuncSetAttribute(k_tc_p2m, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)P2mSmem::total(P.p2m_stage, ns));
+  for (auto k : {k_tc_near_pipe<8>, k_tc_near_pipe<16>, k_tc_near_pipe<32>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, NpSmem::total);
   cudaFuncSetAttribute(k_tc_p2m_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)P2mPipeSmem::total(P.p2m_stage));
   if ((e = cuda_check(c, cudaGetLastError(), "tc setup")) != ISG_OK) return e;
@@ -1514,8 +1315,19 @@ void tc_destroy(isg_ctx *c) {
 }
 
 int tc_near_blocks(const isg_ctx *c) {
-  const int tx = (c->P.nleaf + kTX - 1) / kTX, ty = (c->P.nleaf + kTY - 1) / kTY;
-  return tx * ty;
+  const int n8 = (c->P.nleaf + 7) / 8;
+  return n8 * n8;
+}
+
+// Leaf rows per item of the pipelined near field: 32 (the most MMA columns, so
+// each weight stage serves 256 leaves), unless 16 or 8 rows still give every
+// item an SM of its own or the grid is no higher than that: the launch is then
+// as long as one item, whose time falls with its rows.
+static int np_rows(const DevPlan &P, int nrhs, int sms) {
+  const int cols = (P.nleaf + kTX - 1) / kTX;
+  for (int tr : {8, 16})
+    if (tr >= P.nleaf || (int64_t)cols * ((P.nleaf + tr - 1) / tr) * nrhs <= sms) return tr;
+  return 32;
 }
 
 int tc_error(isg_ctx *c) {
@@ -1546,14 +1358,15 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // The pipelined near-field kernel; returns false (launching nothing) when the
-// call does not meet its conditions: P2M's input maximum known (N.inmax), leaf
+// call does not meet its conditions: the input plain or conjugated (not still
+// without its contrast), P2M's input maximum known (N.inmax), leaf
 // rings of a multiple of 4 samples (<= 80), 16-byte aligned vectors and both
 // tensor maps encoded.
 static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_status *e) {
   const DevPlan &P = c->P;
   const TcPlan &T = *c->tc;
   const float2 *loc_leaf = N.loc + P.lv[P.L - 1].off;
-  if (!N.inmax || !N.locmax || !T.nearNp || P.ns_leaf % 4 || P.ns_leaf > 4 * kLocChunksMax || P.mp % 2 ||
+  if (N.in.mode == IN_G || !N.inmax || !N.locmax || !T.nearNp || P.ns_leaf % 4 || P.ns_leaf > 4 * kLocChunksMax || P.mp % 2 ||
       !aligned16(loc_leaf) || P.L - 1 >= kInMaxSlot)
     return false;
   const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
@@ -1579,26 +1392,27 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
   A.part = N.part;
   A.nleaf = P.nleaf;
   A.U = P.U;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
+  const int tr = np_rows(P, N.in.nrhs, sms);
   A.tiles_x = (P.nleaf + kTX - 1) / kTX;
-  A.tiles_y = (P.nleaf + kTY - 1) / kTY;
-  A.tiles = A.tiles_x * A.tiles_y;
-  A.ppr = A.tiles_x * ((A.tiles_y + kPair - 1) / kPair);
+  A.ppr = A.tiles_x * ((P.nleaf + tr - 1) / tr);
   A.nitems = A.ppr * N.in.nrhs;
   A.err = T.err;
   // tmh: the input as [RHS][leaf row][leaf column][128 reals], a box is one halo
-  // K-group (32 reals) of the pair's 34 x 10 halo; tml: the leaf locals as
-  // [RHS][leaf row][leaf column][2 ns reals], a box is one L2P stage of the pair
+  // K-group (32 reals) of the item's (tr + 2) x 10 halo; tml: the leaf locals as
+  // [RHS][leaf row][leaf column][2 ns reals], a box is one L2P stage of the item
   CUtensorMap tmh, tml;
   memset(&tmh, 0, sizeof(tmh));
   memset(&tml, 0, sizeof(tml));
   const cuuint32_t one[4] = {1, 1, 1, 1};
   const cuuint64_t hd[4] = {2 * kBB, (cuuint64_t)P.nleaf, (cuuint64_t)P.nleaf, (cuuint64_t)N.in.nrhs};
   const cuuint64_t hs[3] = {(cuuint64_t)kBB * 8, (cuuint64_t)P.nleaf * kBB * 8, (cuuint64_t)P.U * 8};
-  const cuuint32_t hb[4] = {32, (cuuint32_t)kHC, (cuuint32_t)kHR, 1};
+  const cuuint32_t hb[4] = {32, (cuuint32_t)kHC, (cuuint32_t)(tr + 2), 1};
   const cuuint64_t ld[4] = {(cuuint64_t)(2 * P.ns_leaf), (cuuint64_t)P.nleaf, (cuuint64_t)P.nleaf,
                             (cuuint64_t)N.in.nrhs};
   const cuuint64_t ls[3] = {(cuuint64_t)P.ns_leaf * 8, (cuuint64_t)P.nleaf * P.ns_leaf * 8, (cuuint64_t)P.mp * 8};
-  const cuuint32_t lb[4] = {32, (cuuint32_t)kTX, (cuuint32_t)(kPair * kTY), 1};
+  const cuuint32_t lb[4] = {32, (cuuint32_t)kTX, (cuuint32_t)tr, 1};
   if (encode(&tmh, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)A.x, hd, hs, hb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
@@ -1606,10 +1420,9 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
   count_launch();
-  k_tc_near_pipe<<<std::min(A.nitems, sms), kNpThreads, NpSmem::total, st>>>(A, tmh, tml);
+  (tr == 32 ? k_tc_near_pipe<32> : tr == 16 ? k_tc_near_pipe<16> : k_tc_near_pipe<8>)
+      <<<std::min(A.nitems, sms), kNpThreads, NpSmem::total, st>>>(A, tmh, tml);
   *e = cuda_check(c, cudaGetLastError(), "tc near launch");
   return true;
 }
@@ -1692,12 +1505,10 @@ isg_status tc_near(isg_ctx *c, const NearArgs &N, cudaStream_t st) {
 isg_status tc_p2m(isg_ctx *c, const BatchArgs &B, float2 *mul, cudaStream_t st) {
   const DevPlan &P = c->P;
   const TcPlan &T = *c->tc;
-  if (!aligned16(B.x) || (B.g && !aligned16(B.g)) || (B.gstride % 2)) return ISG_UNSUPPORTED;
+  if (!aligned16(B.x) || B.mode == IN_G) return ISG_UNSUPPORTED;  // callers form g x first (run_matvec)
   TcP2mArgs A;
   A.x = B.x;
-  A.g = B.g;
-  A.gstride = B.gstride;
-  A.mode = B.mode;
+  A.conj = B.mode == IN_CONJ;
   A.active = B.active;
   A.B = T.p2mB;
   A.npad = T.npad;
@@ -1716,10 +1527,7 @@ isg_status tc_p2m(isg_ctx *c, const BatchArgs &B, float2 *mul, cudaStream_t st) 
   count_launch();
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
-  if (B.mode == IN_G)  // the pipelined kernel stages x alone
-    k_tc_p2m<<<std::min(A.nitems, sms), 256, P2mSmem::total(T.p2m_stage, A.ns), st>>>(A);
-  else
-    k_tc_p2m_pipe<<<std::min(A.nitems, sms), kP2mThreads, P2mPipeSmem::total(T.p2m_stage), st>>>(A);
+  k_tc_p2m_pipe<<<std::min(A.nitems, sms), kP2mThreads, P2mPipeSmem::total(T.p2m_stage), st>>>(A);
   return cuda_check(c, cudaGetLastError(), "tc p2m launch");
 }
 
