@@ -889,21 +889,6 @@ static TileArgs tile_args(const float2 *src, float2 *dst, size_t mp, size_t off_
   A.tb = tb;
   A.shT = shT;
   A.active = active;
-// Leaves per block and per thread of k_p2m.
-enum P2mShape { P2M_2_1, P2M_8_2, P2M_32_4 };
-static P2mShape p2m_shape(const DevPlan &P, int nrhs) {
-  const int64_t leaves = (int64_t)P.nleaf * P.nleaf * nrhs;
-  return leaves <= kP2mSmall ? P2M_2_1 : leaves <= kP2mMid ? P2M_8_2 : P2M_32_4;
-}
-
-template <int LB, int LT>
-static void p2m_as(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
-  const int nleaves = P.nleaf * P.nleaf, units = LB / LT * P.ns_leaf;
-  const int threads = LB == 32 ? 128 : std::min(288, (units + 31) / 32 * 32);
-  k_p2m<LB, LT><<<dim3((nleaves + LB - 1) / LB, B.nrhs), threads, 0, st>>>(
-      B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U, mul + P.lv[P.L - 1].off, P.mp);
-}
-
   return A;
 }
 
@@ -943,18 +928,8 @@ void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int n
   A.zeros = P.zeros;
   A.locmax = locmax;
   A.lvl = lvl;
-int64_t level_outputs(const DevPlan &P, int lvl, int nrhs) {
-  return (int64_t)P.lv[lvl].n * P.lv[lvl].n * P.lv[lvl].ns * nrhs;
-}
-
   // two sibling-group columns per thread where the level has at least four
   const int half = c.n / 2, nc = half >= 4 ? 2 : 1, bx = (half / nc * c.ns + 127) / 128;
-  if (level_outputs(P, lvl, nrhs) <= kM2mDirect) {
-    const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
-    count_launch();
-    k_m2m_direct<<<dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
-    return;
-  }
   // eight groups per thread when the grid stays large, fewer for small batches
   int ty = std::min(8, half);
   while (ty > 1 && (size_t)bx * ((half + ty - 1) / ty) * nrhs < 4 * 148) ty /= 2;
@@ -1033,12 +1008,6 @@ void launch_near(const DevPlan &P, const NearArgs &A, cudaStream_t st) {
 
 void launch_rx_interp(const DevPlan &P, const float2 *mul, float2 *rx, int nrhs, cudaStream_t st) {
   dim3 grid((P.numrx + 127) / 128, nrhs);
-  if (level_outputs(P, lvl, nrhs) <= kL2lDirect) {
-    const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw, p.shl, active};
-    count_launch();
-    k_l2l_direct<<<dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
-    return;
-  }
   count_launch();
   k_rx_interp<<<grid, 128, 0, st>>>(mul + P.lv[0].off, P.mp, rx, P.numrx, P.lv[0].ns, P.hfirst, P.hw, P.ninter);
 }
