@@ -17,8 +17,9 @@
 //     adjoint  re = D_re[j] + D_im[R + j],  im = D_re[R + j] - D_im[j]
 // (the adjoint table stores Re and Im of go, not of its conjugate).  The
 // kernel is bound by reading its table once; persistent CTAs keep four 32 KB
-// table blocks in flight while converter warps turn the right-hand sides' next
-// K-block from FP32 into the FP16 hi/lo B operand (its loads a block ahead) and
+// table blocks in flight while converter warps turn the right-hand sides' K-blocks
+// from FP32 into the FP16 hi/lo B operand (their loads 4 blocks ahead, 2 above 64
+// right-hand sides: one block ahead, a block took as long as a trip to memory) and
 // epilogue warps write the item before.  The caller's order is applied where
 // pixels are read or written: 8 consecutive pixels of the blocked order are one
 // leaf row, contiguous in every order.  The forward GEMM has K = numunk and is
@@ -63,8 +64,9 @@ struct RxSmem {
   static constexpr int a = 0;                      // kRxNA A blocks
   static constexpr int b = kRxNA * kRxBlock;       // 2 B operands
   static constexpr int bars = b + 2 * kRxBBuf;     // afull, aempty [kRxNA]; bfull, bempty, tfull, tfree [2]; fin
-  static constexpr int misc = bars + (2 * kRxNA + 9) * 8;
-  static constexpr int total = misc + 16;          // TMEM base, abort flag
+  static constexpr int misc = bars + (2 * kRxNA + 9) * 8;  // TMEM base, abort flag
+  static constexpr int inv = misc + 16;                    // [kRxMaxN / 2] 1 / (table scale x RHS scale)
+  static constexpr int total = inv + kRxMaxN / 2 * 4;
 };
 
 // Offset of element (row, k) of a 128 x 32 (or N x 32) K-major FP16 block in
@@ -139,7 +141,7 @@ __global__ void k_rx_rowmax(const float2 *x, int64_t ld, int kvalid, int vec, un
   const float2 *r = x + (size_t)j * ld;
   float m = 0.f;
   if (vec) {
-#pragma unroll 4
+#pragma unroll 8
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kvalid / 2; k += gridDim.x * blockDim.x) {
       const float4 v = __ldg((const float4 *)r + k);
       m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
@@ -173,6 +175,8 @@ struct RxGemmArgs {
   int *err;
 };
 
+// UN: units of 8 K of one RHS per converter thread and K-block (1 up to 64 RHS).
+template <int UN>
 __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
   extern __shared__ __align__(1024) char sm[];
   uint64_t *afull = (uint64_t *)(sm + RxSmem::bars), *aempty = afull + kRxNA;
@@ -185,6 +189,8 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
     *abort = 0;
     fence_mbar_init();
   }
+  float *inv = (float *)(sm + RxSmem::inv);
+  for (int j = threadIdx.x; j < R; j += kRxThreads) inv[j] = A.ainv / pow2_scale(__uint_as_float(A.rowmax[j]));
   if (warp == 0) tmem_alloc(tslot, 512);
   tc_fence_before();
   __syncthreads();
@@ -217,76 +223,83 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
       for (int j = 1; j <= kRxNA && j <= ka; j++) mbar_wait(afull + (ka - j) % kRxNA, ((ka - j) / kRxNA) & 1, A.err, kErrRx);
     }
   } else if (warp == 1) {
-    // ---- MMA issue: D_re += Re(A) B, D_im += Im(A) B, three split products each ----
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(128, A.npad), sbase = smem_u32(sm);
-      int ka = 0, it = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < A.nitems && ok; w += gridDim.x, it++) {
-        int kb0, kb1;
-        blocks(w, kb0, kb1);
-        const int set = it % nset;
-        ok = mbar_wait_or(tfree + set, ((it / nset) & 1) ^ 1, abort, A.err, kErrRx);
-        for (int kb = kb0; kb < kb1 && ok; kb++, ka++) {
-          const int i = ka % kRxNA, b = ka & 1;
-          ok = mbar_wait_or(afull + i, (ka / kRxNA) & 1, abort, A.err, kErrRx) &&
-               mbar_wait_or(bfull + b, (ka >> 1) & 1, abort, A.err, kErrRx);
-          tc_fence_after();
-          if (!ok) break;
-          const uint32_t ab = sbase + RxSmem::a + i * kRxBlock, bb = sbase + RxSmem::b + b * kRxBBuf;
-          const uint64_t brh = smem_desc(bb, 128, 512), brl = smem_desc(bb + A.npad * kRxKB * 2, 128, 512);
+    // ---- MMA issue (the warp waits, one elected lane issues): D_re += Re(A) B, D_im += Im(A) B, three
+    // split products each ----
+    const uint32_t idesc = idesc_f16_f32(128, A.npad), sbase = smem_u32(sm);
+    int ka = 0, it = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < A.nitems && ok; w += gridDim.x, it++) {
+      int kb0, kb1;
+      blocks(w, kb0, kb1);
+      const int set = it % nset;
+      ok = mbar_wait_or(tfree + set, ((it / nset) & 1) ^ 1, abort, A.err, kErrRx);
+      for (int kb = kb0; kb < kb1; kb++, ka++) {
+        const int i = ka % kRxNA, b = ka & 1;
+        ok = __all_sync(0xffffffffu, ok && mbar_wait_or(afull + i, (ka / kRxNA) & 1, abort, A.err, kErrRx) &&
+                                         mbar_wait_or(bfull + b, (ka >> 1) & 1, abort, A.err, kErrRx));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ab = sbase + RxSmem::a + i * kRxBlock, bb = sbase + RxSmem::b + b * kRxBBuf;
+        const uint64_t brh = smem_desc(bb, 128, 512), brl = smem_desc(bb + A.npad * kRxKB * 2, 128, 512);
+        const uint64_t a0 = smem_desc(ab, 128, 512);
+        const uint32_t d0 = tmem + (uint32_t)(set * 256);
+        const int acc = kb > kb0 ? 1 : 0;
+        if (elect_one()) {
 #pragma unroll
           for (int part = 0; part < 2; part++) {  // re, im of the table
-            const uint64_t ah = smem_desc(ab + part * 2 * kRxSplit, 128, 512);
-            const uint64_t al = smem_desc(ab + part * 2 * kRxSplit + kRxSplit, 128, 512);
-            const uint32_t d = tmem + (uint32_t)(set * 256 + part * dim);
+            const uint64_t ah = desc_add(a0, part * 2 * kRxSplit), al = desc_add(a0, part * 2 * kRxSplit + kRxSplit);
+            const uint32_t d = d0 + (uint32_t)(part * dim);
 #pragma unroll
             for (int ks = 0; ks < kRxKB / 16; ks++) {
-              mma_f16(d, desc_add(ah, ks * 256), desc_add(brh, ks * 256), idesc, (kb > kb0 || ks > 0) ? 1 : 0);
+              mma_f16(d, desc_add(ah, ks * 256), desc_add(brh, ks * 256), idesc, ks ? 1 : acc);
               mma_f16(d, desc_add(ah, ks * 256), desc_add(brl, ks * 256), idesc, 1);
               mma_f16(d, desc_add(al, ks * 256), desc_add(brh, ks * 256), idesc, 1);
             }
           }
           mma_commit(aempty + i);
           mma_commit(bempty + b);
+          if (kb == kb1 - 1) mma_commit(tfull + set);
         }
-        if (ok) mma_commit(tfull + set);
+        __syncwarp();
       }
-      // every MMA issued is complete before TMEM is freed (bounded wait)
-      mma_commit(fin);
-      mbar_wait(fin, 0, A.err, kErrRx);
     }
+    // every MMA issued is complete before TMEM is freed (bounded wait)
+    if (elect_one()) mma_commit(fin);
+    __syncwarp();
+    mbar_wait(fin, 0, A.err, kErrRx);
   } else if (warp < kRxEpiWarp0) {
     // ---- converters: B row j = Re x_j, row R + j = Im x_j over the K-block's 32 elements, scaled per
-    // RHS.  A unit is 8 consecutive K of one RHS; a thread has at most two, loaded a block ahead ----
+    // RHS.  A unit is 8 consecutive K of one RHS; a thread has UN of them, loaded kAhead blocks ahead
+    // of their conversion, across items ----
+    constexpr int kAhead = UN == 1 ? 4 : 2;
     const int ct = threadIdx.x - 32 * kRxConvWarp0, nu = 4 * R;
-    float sc[2];
+    float sc[UN];
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < UN; q++) {
       const int u = ct + q * kRxConv;
       sc[q] = u < nu ? pow2_scale(__uint_as_float(A.rowmax[u >> 2])) : 1.f;
     }
-    float2 v[2][8];
-    auto load = [&](int kb) {
+    float2 v[kAhead][UN][8];
+    auto load = [&](int kb, float2(&d)[UN][8]) {
 #pragma unroll
-      for (int q = 0; q < 2; q++) {
+      for (int q = 0; q < UN; q++) {
         const int u = ct + q * kRxConv, K = kb * kRxKB + (u & 3) * 8;
         const float2 *row = A.x + (size_t)(u >> 2) * A.ldx;
 #pragma unroll
-        for (int e = 0; e < 8; e++) v[q][e] = make_float2(0.f, 0.f);
+        for (int e = 0; e < 8; e++) d[q][e] = make_float2(0.f, 0.f);
         if (u >= nu || K >= A.kvalid) continue;
         const float2 *src = row + (A.perm ? A.perm[K] : K);
         if (A.vec && K + 8 <= A.kvalid) {
 #pragma unroll
           for (int e = 0; e < 4; e++) {
             const float4 t = __ldg((const float4 *)src + e);
-            v[q][2 * e] = make_float2(t.x, t.y);
-            v[q][2 * e + 1] = make_float2(t.z, t.w);
+            d[q][2 * e] = make_float2(t.x, t.y);
+            d[q][2 * e + 1] = make_float2(t.z, t.w);
           }
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e++)
-            if (K + e < A.kvalid) v[q][e] = src[e];
+            if (K + e < A.kvalid) d[q][e] = src[e];
         }
       }
     };
@@ -297,26 +310,38 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
       *(uint4 *)(bh + rx_core_off(r, c * 8)) = make_uint4(0, 0, 0, 0);
       *(uint4 *)(bl + rx_core_off(r, c * 8)) = make_uint4(0, 0, 0, 0);
     }
-    int ka = 0;
-    for (int w = blockIdx.x; w < A.nitems; w += gridDim.x) {
-      int kb0, kb1;
-      blocks(w, kb0, kb1);
-      if (kb0 < kb1) load(kb0);
-      for (int kb = kb0; kb < kb1; kb++, ka++) {
-        const int b = ka & 1;
-        uint32_t rh[2][4], rl[2][4], ih[2][4], il[2][4];
+    // the CTA's K-blocks in order, items one after another: the next to load (w, kb of [.., kb1))
+    int w = blockIdx.x, kb = 0, kb1 = 0;
+    if (w < A.nitems) blocks(w, kb, kb1);
+    auto load_next = [&](float2(&d)[UN][8]) {  // false once every block is loaded
+      if (w >= A.nitems) return false;
+      load(kb, d);
+      if (++kb == kb1 && (w += gridDim.x) < A.nitems) blocks(w, kb, kb1);
+      return true;
+    };
+    bool have[kAhead];
 #pragma unroll
-        for (int q = 0; q < 2; q++)
+    for (int p = 0; p < kAhead; p++) have[p] = load_next(v[p]);
+    for (int ka = 0;; ka += kAhead) {
+      bool more = false;
+#pragma unroll
+      for (int p = 0; p < kAhead; p++) {
+        if (!have[p]) break;  // the same in every thread
+        const int b = (ka + p) & 1;
+        uint32_t rh[UN][4], rl[UN][4], ih[UN][4], il[UN][4];
+#pragma unroll
+        for (int q = 0; q < UN; q++)
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            split2u(v[q][2 * e].x * sc[q], v[q][2 * e + 1].x * sc[q], rh[q][e], rl[q][e]);
-            split2u(v[q][2 * e].y * sc[q], v[q][2 * e + 1].y * sc[q], ih[q][e], il[q][e]);
+            split2u(v[p][q][2 * e].x * sc[q], v[p][q][2 * e + 1].x * sc[q], rh[q][e], rl[q][e]);
+            split2u(v[p][q][2 * e].y * sc[q], v[p][q][2 * e + 1].y * sc[q], ih[q][e], il[q][e]);
           }
-        if (kb + 1 < kb1) load(kb + 1);
-        const bool ok = mbar_wait_or(bempty + b, ((ka >> 1) & 1) ^ 1, abort, A.err, kErrRx);
+        have[p] = load_next(v[p]);
+        more = more || have[p];
+        const bool ok = mbar_wait_or(bempty + b, (((ka + p) >> 1) & 1) ^ 1, abort, A.err, kErrRx);
         char *bh = sm + RxSmem::b + b * kRxBBuf, *bl = bh + A.npad * kRxKB * 2;
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
+        for (int q = 0; q < UN; q++) {
           const int u = ct + q * kRxConv, j = u >> 2, c = u & 3;
           if (u >= nu || !ok) continue;
           st_shared_v4(bh + rx_core_off(j, c * 8), rh[q]);
@@ -328,6 +353,7 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
         named_sync(1, kRxConv);
         if (ct == 0) mbar_arrive(bfull + b);
       }
+      if (!more) break;
     }
   } else {
     // ---- epilogue: lane = table row, columns = right-hand sides ----
@@ -354,10 +380,9 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
         for (int q = 0; q < 16; q++) {
           const int j = j0 + q;
           if (j >= R) break;
-          const float inv = A.ainv / pow2_scale(__uint_as_float(A.rowmax[j]));
           const float re = A.adjoint ? dre[q] + dim2[q] : dre[q] - dim2[q];
           const float im = A.adjoint ? dre2[q] - dim1[q] : dre2[q] + dim1[q];
-          out[(size_t)j * A.ldo] = make_float2(re * inv, im * inv);
+          out[(size_t)j * A.ldo] = make_float2(re * inv[j], im * inv[j]);
         }
       }
       tc_fence_before();
@@ -451,7 +476,8 @@ isg_status rxnear_setup(isg_ctx *c, double radius) {
   int ex = 0;
   std::frexp((double)fm, &ex);
   P->ainv = (float)std::ldexp(1.0, ex - 14);  // 1 / pow2_scale(fm)
-  cudaFuncSetAttribute(k_rx_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, RxSmem::total);
+  for (auto k : {k_rx_gemm<1>, k_rx_gemm<2>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RxSmem::total);
   if ((e = cuda_check(c, cudaDeviceSynchronize(), "receiver tables")) != ISG_OK) {
     rxnear_destroy(c);
     return e;
@@ -502,9 +528,9 @@ isg_status rxnear_apply(isg_ctx *c, const float2 *in, float2 *out, int nrhs, int
     }
     cudaMemsetAsync(P.rowmax, 0, (size_t)R * sizeof(unsigned), st);
     count_launch(2);
-    k_rx_rowmax<<<dim3(std::max(1, std::min(64, (int)((ldin + 2047) / 2048))), R), 256, 0, st>>>(A.x, ldin, A.kvalid,
+    k_rx_rowmax<<<dim3(std::max(1, std::min(32, (int)((ldin + 2047) / 2048))), R), 256, 0, st>>>(A.x, ldin, A.kvalid,
                                                                                                 A.vec, P.rowmax);
-    k_rx_gemm<<<std::min(A.nitems, sms), kRxThreads, RxSmem::total, st>>>(A);
+    (R <= 64 ? k_rx_gemm<1> : k_rx_gemm<2>)<<<std::min(A.nitems, sms), kRxThreads, RxSmem::total, st>>>(A);
     if (!adjoint) {
       count_launch();
       k_rx_sum<<<(R * P.nrx + 127) / 128, 128, 0, st>>>(P.part, nsplit, A.split_stride, R, P.nrx,

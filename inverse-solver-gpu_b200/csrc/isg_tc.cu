@@ -704,54 +704,57 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       }
     }
   } else if (warp == 2) {
-    // ---- MMA issue (one thread): D[128 target reals][8 TR leaves of the item] +=
-    // weights (A, M = 128) x data (B, N = 8 TR): each weight stage is 2 K-steps x
-    // 3 split products ----
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(128, kTX * TR), sbase = smem_u32(sm);
-      int ka = 0, kb = 0, it = 0;
-      bool ok = true;
-      for (int w = first; w < A.nitems && ok; w = next_item(w), it++) {
-        const int set = it & 1;
-        const uint32_t d = tmem + (uint32_t)(set * 256);
-        ok = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNp);
-        for (int a = 0; a < na && ok; a++, ka++) {
-          const int i = ka % kNpNO;
-          ok = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNp);
-          int idx;
-          const int kind = np_stage(a, A.nl2p, idx);
-          const uint32_t obase = sbase + NpSmem::o + i * kNpBuf;
-          const uint32_t lbo = kind == 0 ? kHC * 16 : kTX * 16;  // K-adjacent core matrices
-          const uint64_t dh0 = smem_desc(obase, lbo, kNpKC * lbo);
-          const uint64_t dl0 = smem_desc(obase + (kind == 0 ? kNpHaloSplit : kNpL2pSplit), lbo, kNpKC * lbo);
-          const int nq = kind == 0 ? 9 : 1;
-          for (int q = 0; q < nq && ok; q++, kb++) {
-            const int b = kb % kNpNB;
-            ok = mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNp);
-            tc_fence_after();
-            if (!ok) break;
-            const uint32_t bb = sbase + NpSmem::b + b * kStageBytes;
-            const uint64_t wh0 = smem_desc(bb, 128, 512), wl0 = smem_desc(bb + kStageHalf, 128, 512);
-            // neighbour slot q: the item's leaf rows start at halo row 1 + dr, column 1 + dc
-            const uint32_t doff0 = kind == 0 ? (uint32_t)((q / 3) * (kNpKC * kHC * 16) + (q % 3) * 16) : 0u;
+    // ---- MMA issue (the warp waits, one elected lane issues): D[128 target
+    // reals][8 TR leaves of the item] += weights (A, M = 128) x data (B, N = 8 TR):
+    // each weight stage is 2 K-steps x 3 split products ----
+    const uint32_t idesc = idesc_f16_f32(128, kTX * TR), sbase = smem_u32(sm);
+    int ka = 0, kb = 0, it = 0;
+    bool ok = true;
+    for (int w = first; w < A.nitems && ok; w = next_item(w), it++) {
+      const int set = it & 1;
+      const uint32_t d = tmem + (uint32_t)(set * 256);
+      ok = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNp);
+      for (int a = 0; a < na && ok; a++, ka++) {
+        const int i = ka % kNpNO;
+        ok = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNp);
+        int idx;
+        const int kind = np_stage(a, A.nl2p, idx);
+        const uint32_t obase = sbase + NpSmem::o + i * kNpBuf;
+        const uint32_t lbo = kind == 0 ? kHC * 16 : kTX * 16;  // K-adjacent core matrices
+        const uint64_t dh0 = smem_desc(obase, lbo, kNpKC * lbo);
+        const uint64_t dl0 = smem_desc(obase + (kind == 0 ? kNpHaloSplit : kNpL2pSplit), lbo, kNpKC * lbo);
+        const int nq = kind == 0 ? 9 : 1;
+        for (int q = 0; q < nq; q++, kb++) {
+          const int b = kb % kNpNB;
+          ok = __all_sync(0xffffffffu, ok && mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNp));
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t bb = sbase + NpSmem::b + b * kStageBytes;
+          const uint64_t wh0 = smem_desc(bb, 128, 512), wl0 = smem_desc(bb + kStageHalf, 128, 512);
+          // neighbour slot q: the item's leaf rows start at halo row 1 + dr, column 1 + dc
+          const uint32_t doff0 = kind == 0 ? (uint32_t)((q / 3) * (kNpKC * kHC * 16) + (q % 3) * 16) : 0u;
+          const uint64_t dh = desc_add(dh0, doff0), dl = desc_add(dl0, doff0);
+          const int acc = (a | q) ? 1 : 0;
+          if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 2; ks++) {
-              const uint32_t doff = doff0 + (uint32_t)ks * 2 * lbo;
-              const int acc = (a | q | ks) ? 1 : 0;
-              mma_f16(d, desc_add(wh0, ks * 256), desc_add(dh0, doff), idesc, acc);
-              mma_f16(d, desc_add(wh0, ks * 256), desc_add(dl0, doff), idesc, 1);
-              mma_f16(d, desc_add(wl0, ks * 256), desc_add(dh0, doff), idesc, 1);
+              const uint32_t doff = (uint32_t)ks * 2 * lbo;
+              mma_f16(d, desc_add(wh0, ks * 256), desc_add(dh, doff), idesc, ks ? 1 : acc);
+              mma_f16(d, desc_add(wh0, ks * 256), desc_add(dl, doff), idesc, 1);
+              mma_f16(d, desc_add(wl0, ks * 256), desc_add(dh, doff), idesc, 1);
             }
             mma_commit(bempty + b);
+            if (q == nq - 1) mma_commit(ofree + i);
+            if (q == nq - 1 && a == na - 1) mma_commit(tfull + set);
           }
-          if (ok) mma_commit(ofree + i);
+          __syncwarp();
         }
-        if (ok) mma_commit(tfull + set);
       }
-      // every MMA issued is complete before the CTA frees TMEM (bounded wait)
-      mma_commit(mdone);
-      mbar_wait(mdone, 0, A.err, kErrNp);
     }
+    // every MMA issued is complete before the CTA frees TMEM (bounded wait)
+    if (elect_one()) mma_commit(mdone);
+    __syncwarp();
+    mbar_wait(mdone, 0, A.err, kErrNp);
   } else if (warp < kNpEpiWarp0) {
     // ---- converters: a staged FP32 A-stage becomes the FP16 hi/lo operand.  One
     // unit is a 4-complex chunk (32 bytes) of one leaf: staging [row][col][32 reals]
@@ -1045,10 +1048,10 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
           const int odd = m & 1;
           const float4 x0 = zst[m * 32 + 2 * c + odd], x1 = zst[m * 32 + 2 * c + 1 - odd];
           const float4 a0 = odd ? x1 : x0, a1 = odd ? x0 : x1;
-          v[r][0] = make_float2(a0.x, A.conj ? -a0.y : a0.y);
-          v[r][1] = make_float2(a0.z, A.conj ? -a0.w : a0.w);
-          v[r][2] = make_float2(a1.x, A.conj ? -a1.y : a1.y);
-          v[r][3] = make_float2(a1.z, A.conj ? -a1.w : a1.w);
+          v[r][0] = make_float2(a0.x, a0.y);
+          v[r][1] = make_float2(a0.z, a0.w);
+          v[r][2] = make_float2(a1.x, a1.y);
+          v[r][3] = make_float2(a1.z, a1.w);
 #pragma unroll
           for (int p = 0; p < 4; p++) mx = fmaxf(mx, cabs1(v[r][p]));
         }
@@ -1059,7 +1062,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
       named_sync(1, kP2mConv);  // every staged value is in registers: the buffer is rewritten in place
       float m2 = 0.f;
       for (int k = 0; k < kP2mConvWarps; k++) m2 = fmaxf(m2, fscr[k]);
-      const float s = pow2_scale(m2);
+      const float s = pow2_scale(m2), si = A.conj ? -s : s;
       // the input's maximum per RHS: the near-field kernel's scale for the same input
       if (threadIdx.x == 0 && fok && m2 > 0.f && A.lvl < kInMaxSlot)
         atomicMax(&A.levmax[(w / A.tiles) * kMaxLevels + kInMaxSlot], __float_as_uint(m2));
@@ -1071,7 +1074,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
           if (u >= kP2mUnits) continue;
           uint32_t h[4], l[4];
 #pragma unroll
-          for (int p = 0; p < 4; p++) split2u(v[r][p].x * s, v[r][p].y * s, h[p], l[p]);
+          for (int p = 0; p < 4; p++) split2u(v[r][p].x * s, v[r][p].y * si, h[p], l[p]);
           st_shared_v4(ahi + u * 16, h);  // u * 16 = (m >> 3) * 2048 + c * 128 + (m & 7) * 16
           st_shared_v4(alo + u * 16, l);
         }
@@ -1092,23 +1095,26 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
     for (int it = 0; w < A.nitems; it++) {
       const int b = it & 1, ph = (it >> 1) & 1;
       const bool ok = mbar_wait_or(Bq.bfull + b, ph, Bq.abort, A.err, kErrP2m) && aok;
-      if (lane == 0) {
-        tc_fence_after();
-        if (ok) {
-          const uint64_t ah0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b), 128, 2048);
-          const uint64_t al0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b) + kP2mA, 128, 2048);
-          const uint32_t d = tmem + (uint32_t)(b * 256);
-          for (int c = 0; c < 4; c++)
+      tc_fence_after();
+      if (__all_sync(0xffffffffu, ok)) {
+        const uint64_t ah0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b), 128, 2048);
+        const uint64_t al0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b) + kP2mA, 128, 2048);
+        const uint32_t d = tmem + (uint32_t)(b * 256);
+        for (int c = 0; c < 4; c++) {
+          const uint32_t aoff0 = (uint32_t)c * 512, boff0 = c * A.stage_bytes;
+          if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 2; ks++) {
-              const uint32_t aoff = (uint32_t)(c * 4 + ks * 2) * 128, boff = c * A.stage_bytes + ks * 256;
+              const uint32_t aoff = aoff0 + ks * 256, boff = boff0 + ks * 256;
               mma_f16(d, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, (c | ks) ? 1 : 0);
               mma_f16(d, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, 1);
               mma_f16(d, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
             }
+          }
+          __syncwarp();
         }
-        mma_commit(Bq.tfull + b);
       }
+      if (elect_one()) mma_commit(Bq.tfull + b);
       __syncwarp();
       w = next_item(w);
     }

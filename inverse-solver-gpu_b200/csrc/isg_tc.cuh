@@ -144,6 +144,17 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
          | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
 
+// One lane of a converged warp.  MMA warps run their loops and waits as a whole warp
+// and only issue under this: descriptors then stay in uniform registers.  Issued
+// from a branch on the lane index an MMA took 46 cycles or more whatever its size;
+// so elected, M = 128 x K = 16 takes 40 / 48 / 64 / 128 at N = 32 / 64 / 128 / 256
+// (bound by the operands' reads from shared memory below 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r != 0;
+}
+
 __device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"

@@ -194,22 +194,27 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
     }
     fence_proxy_async();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
+      const bool aok = mbar_wait(abar, ch & 1, A.err, kErrBand);
       tc_fence_after();
-      if (mbar_wait(abar, ch & 1, A.err, kErrBand)) {
+      if (__all_sync(0xffffffffu, aok)) {
         const uint64_t ah = smem_desc(sbase, 128, (kKC / 8) * 128);
         const uint64_t al = smem_desc(sbase + kAHalf, 128, (kKC / 8) * 128);
         const uint64_t bh = smem_desc(sbase + 2 * kAHalf, 128, (kKC / 8) * 128);
         const uint64_t bl = smem_desc(sbase + 2 * kAHalf + kBHalf, 128, (kKC / 8) * 128);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kKC / 16; ks++) {
-          const uint32_t k = ks * 256;
-          mma_f16(tmem, desc_add(ah, k), desc_add(bh, k), idesc, (ch | ks) ? 1 : 0);
-          mma_f16(tmem, desc_add(ah, k), desc_add(bl, k), idesc, 1);
-          mma_f16(tmem, desc_add(al, k), desc_add(bh, k), idesc, 1);
+          for (int ks = 0; ks < kKC / 16; ks++) {
+            const uint32_t k = ks * 256;
+            mma_f16(tmem, desc_add(ah, k), desc_add(bh, k), idesc, (ch | ks) ? 1 : 0);
+            mma_f16(tmem, desc_add(ah, k), desc_add(bl, k), idesc, 1);
+            mma_f16(tmem, desc_add(al, k), desc_add(bh, k), idesc, 1);
+          }
         }
       }
-      mma_commit(mbar);
+      __syncwarp();
+      if (elect_one()) mma_commit(mbar);
+      __syncwarp();
     }
     ok = mbar_wait(mbar, ch & 1, A.err, kErrBand) && ok;
     __syncthreads();
@@ -404,19 +409,22 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
       const int b = it & 1, ph = (it >> 1) & 1;
       const bool ok = mbar_wait_or(Bq.bfull + b, ph, Bq.abort, A.err, kErrL2l) &&
                       mbar_wait_or(Bq.tfree + b, ph ^ 1, Bq.abort, A.err, kErrL2l) && aok;
-      if (lane == 0) {
-        tc_fence_after();
-        if (ok) {
-          const uint64_t bh = smem_desc(smem_u32(bbuf(b)), 128, sbo);
-          const uint64_t bl = smem_desc(smem_u32(bbuf(b)) + N * Kp * 2, 128, sbo);
-          const uint32_t d = tmem + (uint32_t)(b * N);
-          for (int ks = 0; ks < Kp / 16; ks++) {
-            const uint32_t k = ks * 256;
+      tc_fence_after();
+      if (__all_sync(0xffffffffu, ok)) {
+        const uint64_t bh = smem_desc(smem_u32(bbuf(b)), 128, sbo);
+        const uint64_t bl = smem_desc(smem_u32(bbuf(b)) + N * Kp * 2, 128, sbo);
+        const uint32_t d = tmem + (uint32_t)(b * N);
+        for (int ks = 0; ks < Kp / 16; ks++) {
+          const uint32_t k = ks * 256;
+          if (elect_one()) {
             mma_f16(d, desc_add(ah, k), desc_add(bh, k), idesc, ks ? 1 : 0);
             mma_f16(d, desc_add(ah, k), desc_add(bl, k), idesc, 1);
             mma_f16(d, desc_add(al, k), desc_add(bh, k), idesc, 1);
           }
+          __syncwarp();
         }
+      }
+      if (elect_one()) {
         mma_commit(Bq.bfree + b);
         mma_commit(Bq.tfull + b);
       }
@@ -614,21 +622,24 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
       const int b = it & 1, ph = (it >> 1) & 1;
       const bool ok = mbar_wait_or(bfull + b, ph, abort, A.err, kErrM2m) &&
                       mbar_wait_or(tfree + b, ph ^ 1, abort, A.err, kErrM2m) && aok;
-      if (lane == 0) {
-        tc_fence_after();
-        if (ok) {
-          const uint64_t bh = smem_desc(smem_u32(bbuf(b)), 128, sbo);
-          const uint64_t bl = smem_desc(smem_u32(bbuf(b)) + N * Kp * 2, 128, sbo);
-          for (int t = 0; t < A.mt; t++) {
-            const uint32_t d = tmem + (uint32_t)((b * A.mt + t) * N), ta = t * tile_bytes;
-            for (int ks = 0; ks < Kp / 16; ks++) {
-              const uint32_t k = ks * 256;
+      tc_fence_after();
+      if (__all_sync(0xffffffffu, ok)) {
+        const uint64_t bh = smem_desc(smem_u32(bbuf(b)), 128, sbo);
+        const uint64_t bl = smem_desc(smem_u32(bbuf(b)) + N * Kp * 2, 128, sbo);
+        for (int t = 0; t < A.mt; t++) {
+          const uint32_t d = tmem + (uint32_t)((b * A.mt + t) * N), ta = t * tile_bytes;
+          for (int ks = 0; ks < Kp / 16; ks++) {
+            const uint32_t k = ks * 256;
+            if (elect_one()) {
               mma_f16(d, desc_add(ah, ta + k), desc_add(bh, k), idesc, ks ? 1 : 0);
               mma_f16(d, desc_add(ah, ta + k), desc_add(bl, k), idesc, 1);
               mma_f16(d, desc_add(al, ta + k), desc_add(bh, k), idesc, 1);
             }
+            __syncwarp();
           }
         }
+      }
+      if (elect_one()) {
         mma_commit(bfree + b);
         mma_commit(tfull + b);
       }
