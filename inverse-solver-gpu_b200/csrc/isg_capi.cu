@@ -375,11 +375,11 @@ isg_status isg_setup_gpu(isg_ctx *c) {
   if ((e = dalloc(c, &c->mul, R * P.mp)) || (e = dalloc(c, &c->loc, R * P.mp)) || (e = dalloc(c, &c->wx, R * U)) ||
       (e = dalloc(c, &c->wy, R * U)) || (e = dalloc(c, &c->wg, R * U)) || (e = dalloc(c, &c->vr, R * U)) ||
       (e = dalloc(c, &c->vrt, R * U)) || (e = dalloc(c, &c->vp, R * U)) || (e = dalloc(c, &c->vv, R * U)) ||
-      (e = dalloc(c, &c->vs, R * U)) || (e = dalloc(c, &c->vt, R * U)) || (e = dalloc(c, &c->vgx, R * U)) || (e = dalloc(c, &c->levmax, 2 * R * kMaxLevels)) ||
+      (e = dalloc(c, &c->vs, R * U)) || (e = dalloc(c, &c->vt, R * U)) || (e = dalloc(c, &c->vgx, R * U)) || (e = dalloc(c, &c->levmax, R * kLevStride)) ||
       (e = dalloc(c, &c->part, parts * 4 + 64)) || (e = dalloc(c, &c->state, R)) ||
       (e = dalloc(c, &c->active, R)) || (e = dalloc(c, &c->count, 1)))
     return e;
-  c->locmax = c->levmax + R * kMaxLevels;
+  c->locmax = c->levmax + kMaxLevels;
   if ((e = cuda_check(c, cudaMallocHost(&c->h_count, sizeof(int)), "cudaMallocHost"))) return e;
   if ((e = cuda_check(c, cudaMemset(c->mul, 0, R * P.mp * sizeof(float2)), "memset"))) return e;
   if ((e = cuda_check(c, cudaMemset(c->loc, 0, R * P.mp * sizeof(float2)), "memset"))) return e;
@@ -715,8 +715,7 @@ isg_status isg_time_stages(isg_ctx *c, int nrhs, int engine, int reps, double *m
   for (int r = -1; r < reps; r++) {
     cudaEventRecord(ev[0], st);
     if (tc) {
-      cudaMemsetAsync(c->levmax, 0, (size_t)nrhs * kMaxLevels * sizeof(unsigned), st);
-      cudaMemsetAsync(c->locmax, 0, (size_t)nrhs * kMaxLevels * sizeof(unsigned), st);
+      cudaMemsetAsync(c->levmax, 0, (size_t)nrhs * kLevStride * sizeof(unsigned), st);
       tc_p2m(c, B, c->mul, st);
     } else {
       launch_p2m(P, B, c->mul, st);

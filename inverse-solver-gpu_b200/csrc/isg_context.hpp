@@ -45,8 +45,8 @@ struct isg_ctx {
   float2 *wg = nullptr;                   // [R][U] contrast in blocked order
   float2 *vr = nullptr, *vrt = nullptr, *vp = nullptr, *vv = nullptr, *vs = nullptr, *vt = nullptr;
   float2 *vgx = nullptr;  // [R][U] g times the next matvec's input, written by the update kernels
-  unsigned *levmax = nullptr;  // [R][kMaxLevels] per-level max |re|, |im| of the multipoles (FP32 bits)
-  unsigned *locmax = nullptr;  // [R][kMaxLevels] the same for the locals (written by M2L)
+  unsigned *levmax = nullptr;  // [R][kLevStride] per-level max |re|, |im| of the multipoles (FP32 bits)
+  unsigned *locmax = nullptr;  // levmax + kMaxLevels: the same for the locals (written by M2L)
   double *part = nullptr;  // FP64 partial records [RHS][block][4]
   isg::RhsState *state = nullptr;  // [R]
   int *active = nullptr;           // [R]
@@ -78,9 +78,10 @@ struct isg_ctx {
 namespace isg {
 // Internal operator entry points shared by the C ABI and the solver.
 enum OpKind { OP_G = 0, OP_GCONJ = 1, OP_FWD = 2, OP_ADJ = 3 };
+// gx: g x when the caller formed it; zeroed: the level maxima of the batch are already 0.
 isg_status run_matvec(isg_ctx *c, const float2 *x, const float2 *g, int64_t gs, float2 *y, int nrhs, int kind,
                       int engine, int red, const float2 *dot_a, const int *active, cudaStream_t st,
-                      const float2 *gx = nullptr);
+                      const float2 *gx = nullptr, bool zeroed = false);
 isg_status run_bicgs(isg_ctx *c, float2 *x, const float2 *g, int64_t gs, const float2 *b, int nrhs, int hermitian,
                      const isg_solve_opts *o, isg_solve_info *info, cudaStream_t st);
 isg_status run_bicgs_group(int n, isg_ctx *const *cs, float2 *const *xs, const float2 *const *gs, const int64_t *gss,

@@ -9,6 +9,8 @@
 namespace isg {
 
 constexpr int kMaxLevels = 12;
+// Per RHS: the maxima of the multipoles' levels, then of the locals' (FP32 bits).
+constexpr int kLevStride = 2 * kMaxLevels;
 constexpr int kBox = 8;
 constexpr int kBB = 64;  // pixels per leaf
 // Kernels put one RHS per grid row (gridDim.y or .z), so no batch may exceed this.
@@ -71,6 +73,36 @@ struct DevPlan {
   int *perm_tree = nullptr;   // blocked index -> tree index
   int *perm_raster = nullptr; // blocked index -> raster index
 };
+
+// Programmatic dependent launch.  The kernels of a matvec and of a BiCGSTAB
+// iteration are launched so that the next one's blocks come up as this one's leave:
+// launch, barrier set-up, TMEM allocation and static tables then overlap (a 256 x
+// 256 x 9 adjoint 147 -> 115 us, a 128 x 128 x 32 iteration 249 -> 229).  Every such
+// kernel calls grid_wait() before it touches anything an earlier kernel wrote or
+// reads: it returns once the kernel before, which waited in its turn, has finished.
+// The result is 0 and goes into the block index, so that no load that depends on it
+// can move ahead.  No kernel lets the next one in earlier (griddepcontrol.launch_
+// dependents): blocks that wait beside a large M2L slow it down (M2L + L2L at 1024 x
+// 1024 x 64 1368 -> 1575 us).
+__device__ __forceinline__ int grid_wait() {
+  int z;
+  asm volatile("griddepcontrol.wait;\n mov.u32 %0, 0;\n" : "=r"(z)::"memory");
+  return z;
+}
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // How the operator input is formed from the caller's vector.
 enum InMode { IN_PLAIN = 0, IN_G = 1, IN_CONJ = 2 };
@@ -169,7 +201,7 @@ struct NearArgs {
   double *part = nullptr;         // [R][nblocks][4]
   const float2 *x_epi = nullptr;  // x of the `x - ...` epilogue when in.x already holds g x (else in.x)
   const unsigned *locmax = nullptr;  // tensor engine: per-RHS level maxima of the locals, written by M2L
-  const unsigned *inmax = nullptr;   // tensor engine: [R][kMaxLevels] whose last slot holds the input's
+  const unsigned *inmax = nullptr;   // tensor engine: [R][kLevStride] whose slot kMaxLevels - 1 holds the input's
                                      // maximum per RHS, written by the tensor-core P2M of the same matvec
 };
 // FP64 partial records per RHS that launch_near writes for a batch of nrhs, and

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(288) k_p2m(const float2 *__restrict__ x, const
                                              int64_t gstride, int mode, const int *__restrict__ active,
                                              const float2 *__restrict__ coeffT, int ns, int nleaves, int U,
                                              float2 *__restrict__ mul_leaf, size_t mp) {
-  const int rhs = blockIdx.y;
+  const int rhs = blockIdx.y + grid_wait();
   if (inactive(active, rhs)) return;
   __shared__ float2 xs[LB][kBB];
   const int leaf0 = blockIdx.x * LB;
@@ -121,7 +121,7 @@ struct M2lArgs {
   const float2 *T;
   const int *active;
   const float2 *zeros;  // at least ns zeros
-  unsigned *locmax;     // optional [R][kMaxLevels]: max |re|, |im| of the level's locals (FP32 bits)
+  unsigned *locmax;     // optional [R][kLevStride]: max |re|, |im| of the level's locals (FP32 bits)
   int lvl;
 };
 
@@ -155,7 +155,7 @@ template <bool ACC, int NC>
 __global__ void __launch_bounds__(kM2lThreads, NC == 1 ? 3 : 2) k_m2l(M2lArgs A) {
   constexpr int NW = m2l_cols(NC);
   extern __shared__ __align__(16) float2 m2l_ring[];  // [kM2lRing][NW][kM2lThreads]
-  const int rhs = blockIdx.z;
+  const int rhs = blockIdx.z + grid_wait();
   if (A.active && !A.active[rhs]) return;
   const int half = A.n >> 1, ns = A.ns, ncp = half / NC;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kM2lThreads, NC == 1 ? 3 : 2) k_m2l(M2lArgs A)
   cp_async_wait_group<0>();
   if (A.locmax) {  // the level's maximum, for the power-of-two scale of the tensor-core L2L below it
     const unsigned mm = __activemask(), bits = __reduce_max_sync(mm, __float_as_uint(mx));
-    if ((threadIdx.x & 31) == __ffs(mm) - 1 && bits) atomicMax(&A.locmax[rhs * kMaxLevels + A.lvl], bits);
+    if ((threadIdx.x & 31) == __ffs(mm) - 1 && bits) atomicMax(&A.locmax[rhs * kLevStride + A.lvl], bits);
   }
 }
 
@@ -343,7 +343,7 @@ __device__ __forceinline__ bool any_active_column(const TileArgs &A, int c0) {
 // written over the children's locals.
 __global__ void __launch_bounds__(128) k_l2l_tile(TileArgs A) {
   extern __shared__ float2 sm[];
-  const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = blockIdx.x * cols;
+  const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = (blockIdx.x + grid_wait()) * cols;
   if (!any_active_column(A, c0)) return;
   const int a0 = A.tb.a0[tile], wl = A.tb.wl[tile], ld = cols + 1;
   const TileSmem L(A.tb.wmax, ld, TO, cols, 4 * cols, (size_t)4 * TO * ld, true);
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(128) k_l2l_tile(TileArgs A) {
 // tile's band weights, then shifted by shm[q][k] and summed.
 __global__ void __launch_bounds__(128) k_m2m_tile(TileArgs A) {
   extern __shared__ float2 sm[];
-  const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = blockIdx.x * cols;
+  const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = (blockIdx.x + grid_wait()) * cols;
   if (!any_active_column(A, c0)) return;
   const int a0 = A.tb.a0[tile], wl = A.tb.wl[tile], ld = 4 * cols + 1;
   const TileSmem L(A.tb.wmax, ld, TO, 4 * cols, cols, (size_t)TO * (cols + 1));
@@ -516,7 +516,7 @@ struct DirectArgs {
 };
 
 __global__ void __launch_bounds__(128) k_m2m_direct(DirectArgs A) {
-  const int rhs = blockIdx.y;
+  const int rhs = blockIdx.y + grid_wait();
   if (inactive(A.active, rhs)) return;
   const int o = blockIdx.x * blockDim.x + threadIdx.x, P = o / A.ns_out, k = o - P * A.ns_out;
   if (P >= A.n_p * A.n_p) return;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(128) k_m2m_direct(DirectArgs A) {
 }
 
 __global__ void __launch_bounds__(128) k_l2l_direct(DirectArgs A) {
-  const int rhs = blockIdx.y;
+  const int rhs = blockIdx.y + grid_wait();
   if (inactive(A.active, rhs)) return;
   const int o = blockIdx.x * blockDim.x + threadIdx.x, c = o / A.ns_out, k = o - c * A.ns_out, n_c = 2 * A.n_p;
   if (c >= n_c * n_c) return;
@@ -620,8 +620,8 @@ __global__ void __launch_bounds__(64 * TY, TX == 8 ? 0 : 2) k_near(
     const float2 *__restrict__ dot_a, double *__restrict__ part, int nleaf, int U, int tiles_x, int tiles_total) {
   constexpr int kHalo = (TY + 2) * (TX + 2), kThreads = 64 * TY;
   constexpr int kStages = near_stages(TX), kRows = near_rows(TX);
+  if (inactive(active, blockIdx.y + grid_wait())) return;
   const int rhs = blockIdx.y;
-  if (inactive(active, rhs)) return;
   extern __shared__ __align__(16) float2 sm[];
   float2 *ring = sm;                              // [kStages][kRows][64]
   float2 *hx = ring + kStages * kRows * kBB;      // [kHalo leaves][64]
@@ -810,7 +810,7 @@ __global__ void k_rx_anterp(const float2 *__restrict__ rx, float2 *__restrict__ 
 
 __global__ void k_permute(const int *__restrict__ perm, const float2 *__restrict__ in, float2 *__restrict__ out, int U,
                           int gather) {
-  const size_t r = blockIdx.y;
+  const size_t r = blockIdx.y + grid_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < U; i += gridDim.x * blockDim.x) {
     if (gather)
       out[r * U + i] = in[r * U + perm[i]];
@@ -822,7 +822,7 @@ __global__ void k_permute(const int *__restrict__ perm, const float2 *__restrict
 // k_permute's gather that also writes gx = g x (g already in the output order).
 __global__ void k_permute_g(const int *__restrict__ perm, const float2 *__restrict__ in, float2 *__restrict__ out,
                             const float2 *__restrict__ g, int64_t gstride, float2 *__restrict__ gx, int U) {
-  const size_t r = blockIdx.y;
+  const size_t r = blockIdx.y + grid_wait();
   const float2 *gr = g + r * gstride;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < U; i += gridDim.x * blockDim.x) {
     const float2 v = in[r * U + perm[i]];
@@ -834,7 +834,7 @@ __global__ void k_permute_g(const int *__restrict__ perm, const float2 *__restri
 // gx = g x, two elements a thread (16-byte aligned vectors, even U)
 __global__ void k_gmul(const float2 *__restrict__ x, const float2 *__restrict__ g, int64_t gstride,
                        float2 *__restrict__ gx, int U, const int *__restrict__ active) {
-  const size_t r = blockIdx.y;
+  const size_t r = blockIdx.y + grid_wait();
   if (inactive(active, r)) return;
   const float4 *xr = (const float4 *)(x + r * U), *gr = (const float4 *)(g + r * gstride);
   float4 *o = (float4 *)(gx + r * U);
@@ -858,8 +858,7 @@ template <int LB, int LT>
 static void p2m_as(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
   const int nleaves = P.nleaf * P.nleaf, units = LB / LT * P.ns_leaf;
   const int threads = LB == 32 ? 128 : std::min(288, (units + 31) / 32 * 32);
-  k_p2m<LB, LT><<<dim3((nleaves + LB - 1) / LB, B.nrhs), threads, 0, st>>>(
-      B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U, mul + P.lv[P.L - 1].off, P.mp);
+  launch(k_p2m<LB, LT>, dim3((nleaves + LB - 1) / LB, B.nrhs), threads, 0, st, B.x, B.g, B.gstride, B.mode, B.active, P.coeffT, P.ns_leaf, nleaves, P.U, mul + P.lv[P.L - 1].off, P.mp);
 }
 
 void launch_p2m(const DevPlan &P, const BatchArgs &B, float2 *mul, cudaStream_t st) {
@@ -901,7 +900,7 @@ void launch_m2m(const DevPlan &P, int lvl, float2 *mul, int nrhs, const int *act
   if (level_outputs(P, lvl, nrhs) <= kM2mDirect) {
     const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
     count_launch();
-    k_m2m_direct<<<dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    launch(k_m2m_direct, dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st, D);
     return;
   }
   const int cap = (p.m2m_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? p.m2m_cols : 32;
@@ -909,7 +908,7 @@ void launch_m2m(const DevPlan &P, int lvl, float2 *mul, int nrhs, const int *act
   const TileSmem L(p.mt.wmax, 4 * A.cols + 1, p.mt.out, 4 * A.cols, A.cols, (size_t)p.mt.out * (A.cols + 1));
   const size_t smem = L.total * sizeof(float2);
   count_launch();
-  k_m2m_tile<<<dim3((A.ncols + A.cols - 1) / A.cols, p.mt.tiles), A.cols * (p.mt.out / kTileOut), smem, st>>>(A);
+  launch(k_m2m_tile, dim3((A.ncols + A.cols - 1) / A.cols, p.mt.tiles), A.cols * (p.mt.out / kTileOut), smem, st, A);
 }
 
 void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int nrhs, const int *active, bool accumulate,
@@ -939,14 +938,14 @@ void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int n
   const dim3 grid(bx, (half + ty - 1) / ty, nrhs);
   if (nc == 2) {
     if (accumulate)
-      k_m2l<true, 2><<<grid, kM2lThreads, m2l_smem(2), st>>>(A);
+      launch(k_m2l<true, 2>, grid, kM2lThreads, m2l_smem(2), st, A);
     else
-      k_m2l<false, 2><<<grid, kM2lThreads, m2l_smem(2), st>>>(A);
+      launch(k_m2l<false, 2>, grid, kM2lThreads, m2l_smem(2), st, A);
   } else {
     if (accumulate)
-      k_m2l<true, 1><<<grid, kM2lThreads, m2l_smem(1), st>>>(A);
+      launch(k_m2l<true, 1>, grid, kM2lThreads, m2l_smem(1), st, A);
     else
-      k_m2l<false, 1><<<grid, kM2lThreads, m2l_smem(1), st>>>(A);
+      launch(k_m2l<false, 1>, grid, kM2lThreads, m2l_smem(1), st, A);
   }
 }
 
@@ -955,7 +954,7 @@ void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *act
   if (level_outputs(P, lvl, nrhs) <= kL2lDirect) {
     const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw, p.shl, active};
     count_launch();
-    k_l2l_direct<<<dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st>>>(D);
+    launch(k_l2l_direct, dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st, D);
     return;
   }
   const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : 64;
@@ -963,7 +962,7 @@ void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *act
   const TileSmem L(c.at.wmax, A.cols + 1, c.at.out, A.cols, 4 * A.cols, (size_t)4 * c.at.out * (A.cols + 1), true);
   const size_t smem = L.total * sizeof(float2);
   count_launch();
-  k_l2l_tile<<<dim3((A.ncols + A.cols - 1) / A.cols, c.at.tiles), A.cols * (c.at.out / kTileOut), smem, st>>>(A);
+  launch(k_l2l_tile, dim3((A.ncols + A.cols - 1) / A.cols, c.at.tiles), A.cols * (c.at.out / kTileOut), smem, st, A);
 }
 
 // Leaf rows and columns of a near-field tile (k_near).
@@ -993,8 +992,7 @@ static void near_as(const DevPlan &P, const NearArgs &A, cudaStream_t st) {
   const int tiles_x = (P.nleaf + TX - 1) / TX, tiles = near_blocks_per_rhs(P, A.in.nrhs);
   const size_t smem =
       (size_t)((near_stages(TX) * near_rows(TX) + (TY + 2) * (TX + 2)) * kBB + TY * TX * P.ns_leaf) * sizeof(float2);
-  k_near<TY, TX><<<dim3(tiles, A.in.nrhs), 64 * TY, smem, st>>>(
-      A.in.x, A.in.g, A.in.gstride, A.in.mode, A.in.active, A.loc + P.lv[P.L - 1].off, P.mp, P.ns_leaf, P.nearW,
+  launch(k_near<TY, TX>, dim3(tiles, A.in.nrhs), 64 * TY, smem, st, A.in.x, A.in.g, A.in.gstride, A.in.mode, A.in.active, A.loc + P.lv[P.L - 1].off, P.mp, P.ns_leaf, P.nearW,
       P.basisT, A.y, A.epi, A.red, A.dot_a, A.part, P.nleaf, P.U, tiles_x, tiles);
 }
 
@@ -1021,19 +1019,19 @@ void launch_rx_anterp(const DevPlan &P, const float2 *rx, float2 *loc, int nrhs,
 void launch_permute(const int *perm, const float2 *in, float2 *out, int U, int nrhs, bool gather, cudaStream_t st) {
   dim3 grid(std::min((U + 255) / 256, 1184), nrhs);
   count_launch();
-  k_permute<<<grid, 256, 0, st>>>(perm, in, out, U, gather ? 1 : 0);
+  launch(k_permute, grid, 256, 0, st, perm, in, out, U, gather ? 1 : 0);
 }
 
 void launch_permute_g(const int *perm, const float2 *in, float2 *out, const float2 *g, int64_t gstride, float2 *gx,
                       int U, int nrhs, cudaStream_t st) {
   count_launch();
-  k_permute_g<<<dim3(std::min((U + 255) / 256, 1184), nrhs), 256, 0, st>>>(perm, in, out, g, gstride, gx, U);
+  launch(k_permute_g, dim3(std::min((U + 255) / 256, 1184), nrhs), 256, 0, st, perm, in, out, g, gstride, gx, U);
 }
 
 void launch_gmul(const float2 *x, const float2 *g, int64_t gstride, float2 *gx, int U, int nrhs, const int *active,
                  cudaStream_t st) {
   count_launch();
-  k_gmul<<<dim3(std::min((U / 2 + 255) / 256, 1184), nrhs), 256, 0, st>>>(x, g, gstride, gx, U, active);
+  launch(k_gmul, dim3(std::min((U / 2 + 255) / 256, 1184), nrhs), 256, 0, st, x, g, gstride, gx, U, active);
 }
 
 }  // namespace isg

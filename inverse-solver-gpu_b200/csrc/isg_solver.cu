@@ -149,15 +149,21 @@ __global__ void __launch_bounds__(256) k_fin_init(RhsState *st, int *active, int
   if (s.active) atomicAdd(count, 1);
 }
 
+// The level maxima of an active RHS, cleared for the matvec that follows (lev may be null).
+__device__ __forceinline__ void zero_levels(unsigned *lev, int rhs) {
+  if (lev && blockIdx.x == 0 && threadIdx.x < kLevStride) lev[rhs * kLevStride + threadIdx.x] = 0u;
+}
+
 // p = r (first iteration) or p = r + beta (p - omega v), beta = (rho/rho1)(alpha/omega)
 // (bicgs.cpp:132-139).
 // With gp: also gp = g p, the input of the forward matvec that follows.
 __global__ void __launch_bounds__(256) k_update_p(const RhsState *st, const int *active, const float2 *__restrict__ r,
                                                   float2 *__restrict__ p, const float2 *__restrict__ v, int U,
                                                   const float2 *__restrict__ g, int64_t gstride,
-                                                  float2 *__restrict__ gp) {
-  const int rhs = blockIdx.y;
+                                                  float2 *__restrict__ gp, unsigned *lev) {
+  const int rhs = blockIdx.y + grid_wait();
   if (inactive(active, rhs)) return;
+  zero_levels(lev, rhs);
   const RhsState &s = st[rhs];
   const size_t base = (size_t)rhs * U;
   const float2 *gr = g + rhs * gstride;
@@ -174,7 +180,7 @@ __global__ void __launch_bounds__(256) k_update_p(const RhsState *st, const int 
 
 // alpha = rho / <r~, v> (bicgs.cpp:145).
 __global__ void __launch_bounds__(256) k_fin_alpha(RhsState *st, int *active, const double *part, int nb) {
-  const int rhs = blockIdx.x;
+  const int rhs = blockIdx.x + grid_wait();
   if (!active[rhs]) return;
   double tot[3];
   sum_partials(part, rhs, nb, tot);
@@ -196,9 +202,10 @@ __global__ void __launch_bounds__(256) k_fin_alpha(RhsState *st, int *active, co
 __global__ void __launch_bounds__(256) k_update_s(const RhsState *st, const int *active, const float2 *__restrict__ r,
                                                   const float2 *__restrict__ v, float2 *__restrict__ s, int U,
                                                   const float2 *__restrict__ g, int64_t gstride,
-                                                  float2 *__restrict__ gsv) {
-  const int rhs = blockIdx.y;
+                                                  float2 *__restrict__ gsv, unsigned *lev) {
+  const int rhs = blockIdx.y + grid_wait();
   if (inactive(active, rhs)) return;
+  zero_levels(lev, rhs);
   const float2 a = f2(ld2(st[rhs].alpha));
   const size_t base = (size_t)rhs * U;
   const float2 *gr = g + rhs * gstride;
@@ -212,7 +219,7 @@ __global__ void __launch_bounds__(256) k_update_s(const RhsState *st, const int 
 // omega = <t, s> / ||t||^2 (bicgs.cpp:153); zero when t vanishes, which only
 // happens when s itself is zero (bicgs_gpu.cu:197 guards the same case).
 __global__ void __launch_bounds__(256) k_fin_omega(RhsState *st, const int *active, const double *part, int nb) {
-  const int rhs = blockIdx.x;
+  const int rhs = blockIdx.x + grid_wait();
   if (!active[rhs]) return;
   double tot[3];
   sum_partials(part, rhs, nb, tot);
@@ -232,8 +239,9 @@ __global__ void __launch_bounds__(256) k_fin_omega(RhsState *st, const int *acti
 __global__ void __launch_bounds__(256) k_update_xr(const RhsState *st, const int *active, float2 *__restrict__ x,
                                                    float2 *__restrict__ r, const float2 *__restrict__ rt,
                                                    const float2 *__restrict__ p, const float2 *__restrict__ s,
-                                                   const float2 *__restrict__ t, int U, double *part) {
-  const int rhs = blockIdx.y;
+                                                   const float2 *__restrict__ t, int U, double *part, int *count) {
+  const int rhs = blockIdx.y + grid_wait();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *count = 0;  // k_fin_iter counts the active RHS
   if (inactive(active, rhs)) return;
   const float2 a = f2(ld2(st[rhs].alpha)), o = f2(ld2(st[rhs].omega));
   const size_t base = (size_t)rhs * U;
@@ -254,7 +262,7 @@ __global__ void __launch_bounds__(256) k_update_xr(const RhsState *st, const int
 // Convergence and breakdown tests of one iteration (bicgs.cpp:160-169, 127-131).
 __global__ void __launch_bounds__(256) k_fin_iter(RhsState *st, int *active, int *count, const double *part, int nb,
                                                   double tol, int maxit) {
-  const int rhs = blockIdx.x;
+  const int rhs = blockIdx.x + grid_wait();
   if (!active[rhs]) return;
   double tot[3];
   sum_partials(part, rhs, nb, tot);
@@ -341,7 +349,7 @@ __global__ void __launch_bounds__(256) k_fin_true(RhsState *st, int *active, int
 
 isg_status run_matvec(isg_ctx *c, const float2 *x, const float2 *g, int64_t gs, float2 *y, int nrhs, int kind,
                       int engine, int red, const float2 *dot_a, const int *active, cudaStream_t st,
-                      const float2 *gx) {
+                      const float2 *gx, bool zeroed) {
   const DevPlan &P = c->P;
   BatchArgs B;
   B.x = x;
@@ -370,8 +378,7 @@ isg_status run_matvec(isg_ctx *c, const float2 *x, const float2 *g, int64_t gs, 
     Bg.mode = IN_PLAIN;
   }
   if (tc) {
-    cudaMemsetAsync(c->levmax, 0, (size_t)nrhs * kMaxLevels * sizeof(unsigned), st);
-    cudaMemsetAsync(c->locmax, 0, (size_t)nrhs * kMaxLevels * sizeof(unsigned), st);
+    if (!zeroed) cudaMemsetAsync(c->levmax, 0, (size_t)nrhs * kLevStride * sizeof(unsigned), st);
     isg_status e = tc_p2m(c, Bg, c->mul, st);
     if (e != ISG_OK) return e;
   } else {
@@ -448,24 +455,26 @@ struct BicgsRun {
   // `check` iterations of every active RHS (bicgs.cpp:120-177); inactive ones return at once
   isg_status block(cudaStream_t st) {
     const int U = c->P.U;
+    // the updates clear the tensor engine's level maxima, so that an iteration is kernels only
+    unsigned *lev = engine == ISG_ENGINE_TENSOR ? c->levmax : nullptr;
     for (int k = 0; k < check; k++) {
       count_launch();
-      k_update_p<<<vgrid(), 256, 0, st>>>(c->state, c->active, c->vr, c->vp, c->vv, U, g, gs, gx);
-      isg_status be = run_matvec(c, c->vp, g, gs, c->vv, R, kind, engine, RED_DOT, c->vrt, c->active, st, gx);
+      launch(k_update_p, vgrid(), 256, 0, st, c->state, c->active, c->vr, c->vp, c->vv, U, g, gs, gx, lev);
+      isg_status be = run_matvec(c, c->vp, g, gs, c->vv, R, kind, engine, RED_DOT, c->vrt, c->active, st, gx, lev);
       if (be != ISG_OK) return be;
       count_launch();
-      k_fin_alpha<<<R, 256, 0, st>>>(c->state, c->active, c->part, nbn);
+      launch(k_fin_alpha, R, 256, 0, st, c->state, c->active, c->part, nbn);
       count_launch();
-      k_update_s<<<vgrid(), 256, 0, st>>>(c->state, c->active, c->vr, c->vv, c->vs, U, g, gs, gx);
-      be = run_matvec(c, c->vs, g, gs, c->vt, R, kind, engine, RED_TS, nullptr, c->active, st, gx);
+      launch(k_update_s, vgrid(), 256, 0, st, c->state, c->active, c->vr, c->vv, c->vs, U, g, gs, gx, lev);
+      be = run_matvec(c, c->vs, g, gs, c->vt, R, kind, engine, RED_TS, nullptr, c->active, st, gx, lev);
       if (be != ISG_OK) return be;
       count_launch();
-      k_fin_omega<<<R, 256, 0, st>>>(c->state, c->active, c->part, nbn);
+      launch(k_fin_omega, R, 256, 0, st, c->state, c->active, c->part, nbn);
       count_launch();
-      k_update_xr<<<vgrid(), 256, 0, st>>>(c->state, c->active, x, c->vr, c->vrt, c->vp, c->vs, c->vt, U, c->part);
-      cudaMemsetAsync(c->count, 0, sizeof(int), st);
+      launch(k_update_xr, vgrid(), 256, 0, st, c->state, c->active, x, c->vr, c->vrt, c->vp, c->vs, c->vt, U, c->part,
+             c->count);
       count_launch();
-      k_fin_iter<<<R, 256, 0, st>>>(c->state, c->active, c->count, c->part, nbv, o->tol, o->maxit);
+      launch(k_fin_iter, R, 256, 0, st, c->state, c->active, c->count, c->part, nbv, o->tol, o->maxit);
     }
     return cuda_check(c, cudaGetLastError(), "bicgs iteration");
   }

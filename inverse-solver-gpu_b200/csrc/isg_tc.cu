@@ -111,7 +111,7 @@ struct TcNearArgs {
   int nleaf, U, tiles_x, tiles;
   int loc_vec;  // leaf locals can be copied in 16-byte chunks (ns % 4 == 0, aligned)
   int pair;     // tiles per CTA: kPair, or 1 when the launch is too small to fill the GPU
-  const unsigned *locmax;  // when set: [R][kMaxLevels] maxima of the locals (written by M2L), the L2P scale
+  const unsigned *locmax;  // when set: [R][kLevStride] maxima of the locals (written by M2L), the L2P scale
   int lvl_leaf;
   int tma_x;    // the halo comes by two tensor loads (map tmx)
   int tma_loc;  // the leaf locals come by tensor loads (map tml)
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
       cp_async_wait_all();
       loaders_bar();
       if (A.locmax) {  // the leaf level's maximum per RHS, from M2L
-        s2 = pow2_scale(__uint_as_float(A.locmax[rhs * kMaxLevels + A.lvl_leaf]));
+        s2 = pow2_scale(__uint_as_float(A.locmax[rhs * kLevStride + A.lvl_leaf]));
       } else {
         float mx2 = 0.f;
         for (int it = li; it < kL; it += kLoaders) {
@@ -583,7 +583,7 @@ struct TcNearPipeArgs {
   const uint8_t *B;  // weight stages in A-stage order
   int nl2p;
   float sw, sb;      // power-of-two scales of the near-field weights and the L2P basis
-  const unsigned *levmax, *locmax;  // [R][kMaxLevels]: P2M's input maximum (slot kInMaxSlot), M2L's locals
+  const unsigned *levmax, *locmax;  // [R][kLevStride]: P2M's input maximum (slot kInMaxSlot), M2L's locals
   int lvl_leaf;
   float2 *y;
   int epi, red;
@@ -596,8 +596,8 @@ struct TcNearPipeArgs {
 // The item's operand scales: input s1 and locals s2 lowered to a common product scale p = s1 sw = s2 sb.
 // A zero maximum (an all-zero input or locals) leaves the other operand's scale alone.
 __device__ __forceinline__ void np_scales(const TcNearPipeArgs &A, int rhs, float &s1, float &s2, float &p) {
-  const float mx = __uint_as_float(A.levmax[rhs * kMaxLevels + kInMaxSlot]);
-  const float ml = __uint_as_float(A.locmax[rhs * kMaxLevels + A.lvl_leaf]);
+  const float mx = __uint_as_float(A.levmax[rhs * kLevStride + kInMaxSlot]);
+  const float ml = __uint_as_float(A.locmax[rhs * kLevStride + A.lvl_leaf]);
   const float a = mx > 0.f ? pow2_scale(mx) * A.sw : INFINITY;
   const float b = ml > 0.f ? pow2_scale(ml) * A.sb : INFINITY;
   p = fminf(a, b);
@@ -636,8 +636,8 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     while (w < A.nitems && A.active && !A.active[w / A.ppr]);
     return w;
   };
-  const int first = (A.active && blockIdx.x < A.nitems && !A.active[blockIdx.x / A.ppr]) ? next_item(blockIdx.x)
-                                                                                           : blockIdx.x;
+  const int blk = blockIdx.x + grid_wait();
+  const int first = (A.active && blk < A.nitems && !A.active[blk / A.ppr]) ? next_item(blk) : blk;
   auto geom = [&](int w, int &rhs, int &ty0, int &tx0) {
     rhs = w / A.ppr;
     const int pr = w % A.ppr, pty = pr / A.tiles_x, ptx = pr % A.tiles_x;
@@ -957,7 +957,7 @@ struct TcP2mArgs {
   size_t mp;
   int ns, nleaves, U, tiles, nitems;
   int *err;
-  unsigned *levmax;  // [R][kMaxLevels]: this level's max |re|, |im| per RHS (FP32 bits)
+  unsigned *levmax;  // [R][kLevStride]: this level's max |re|, |im| per RHS (FP32 bits)
   int lvl;
 };
 
@@ -1004,7 +1004,13 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
     while (w < A.nitems && A.active && !A.active[w / A.tiles]);
     return w;
   };
-  const int first = (A.active && !A.active[blockIdx.x / A.tiles]) ? next_item(blockIdx.x) : blockIdx.x;
+  if (threadIdx.x == 0) {  // the coefficients, which no earlier kernel writes
+    mbar_expect_tx(Bq.abar, 4 * A.stage_bytes);
+    for (int c = 0; c < 4; c++)
+      bulk_g2s(sm + P2mPipeSmem::bst() + c * A.stage_bytes, A.B + (size_t)c * A.stage_bytes, A.stage_bytes, Bq.abar);
+  }
+  const int blk = blockIdx.x + grid_wait();
+  const int first = (A.active && !A.active[blk / A.tiles]) ? next_item(blk) : blk;
   // an item's pixels (its leaves are one contiguous run) into operand buffer b, as FP32
   auto stage = [&](int w, int b) {
     const int rhs = w / A.tiles, leaf0 = (w % A.tiles) * 128;
@@ -1016,10 +1022,6 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
   if (warp < kP2mConvWarps) {
     // ---- converters ----
     if (threadIdx.x == 0) {
-      mbar_expect_tx(Bq.abar, 4 * A.stage_bytes);
-      for (int c = 0; c < 4; c++)
-        bulk_g2s(sm + P2mPipeSmem::bst() + c * A.stage_bytes, A.B + (size_t)c * A.stage_bytes, A.stage_bytes,
-                 Bq.abar);
       if (first < A.nitems) {
         stage(first, 0);
         const int second = next_item(first);
@@ -1065,7 +1067,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
       const float s = pow2_scale(m2), si = A.conj ? -s : s;
       // the input's maximum per RHS: the near-field kernel's scale for the same input
       if (threadIdx.x == 0 && fok && m2 > 0.f && A.lvl < kInMaxSlot)
-        atomicMax(&A.levmax[(w / A.tiles) * kMaxLevels + kInMaxSlot], __float_as_uint(m2));
+        atomicMax(&A.levmax[(w / A.tiles) * kLevStride + kInMaxSlot], __float_as_uint(m2));
       char *ahi = sm + P2mPipeSmem::a(b), *alo = ahi + kP2mA;
       if (fok) {
 #pragma unroll
@@ -1164,7 +1166,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
       named_sync(2, kP2mEpi);  // the accumulator is read out
       if (ew == 0 && lane == 0) mbar_arrive(Bq.tfree + b);
       const unsigned mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(omx));  // omx >= 0
-      if (lane == 0 && ok && mbits) atomicMax(&A.levmax[rhs * kMaxLevels + A.lvl], mbits);
+      if (lane == 0 && ok && mbits) atomicMax(&A.levmax[rhs * kLevStride + A.lvl], mbits);
       w = next_item(w);
     }
   }
@@ -1427,8 +1429,8 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   count_launch();
-  (tr == 32 ? k_tc_near_pipe<32> : tr == 16 ? k_tc_near_pipe<16> : k_tc_near_pipe<8>)
-      <<<std::min(A.nitems, sms), kNpThreads, NpSmem::total, st>>>(A, tmh, tml);
+  launch(tr == 32 ? k_tc_near_pipe<32> : tr == 16 ? k_tc_near_pipe<16> : k_tc_near_pipe<8>, std::min(A.nitems, sms),
+         kNpThreads, NpSmem::total, st, A, tmh, tml);
   *e = cuda_check(c, cudaGetLastError(), "tc near launch");
   return true;
 }
@@ -1533,7 +1535,7 @@ isg_status tc_p2m(isg_ctx *c, const BatchArgs &B, float2 *mul, cudaStream_t st) 
   count_launch();
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
-  k_tc_p2m_pipe<<<std::min(A.nitems, sms), kP2mThreads, P2mPipeSmem::total(T.p2m_stage), st>>>(A);
+  launch(k_tc_p2m_pipe, std::min(A.nitems, sms), kP2mThreads, P2mPipeSmem::total(T.p2m_stage), st, A);
   return cuda_check(c, cudaGetLastError(), "tc p2m launch");
 }
 

@@ -65,7 +65,7 @@ struct BandArgs {
   int nparents, ncols;  // ncols = parents x RHS
   const int *active;
   int *err;
-  unsigned *levmax;        // [R][kMaxLevels] max |re|, |im| per RHS and level (FP32 bits)
+  unsigned *levmax;        // [R][kLevStride] max |re|, |im| per RHS and level (FP32 bits)
   int lvl_in, lvl_out;
 };
 
@@ -74,8 +74,8 @@ struct RingRef {
   const float2 *p;
 };
 
-__device__ __forceinline__ RingRef ring_ref(const BandArgs &A, int ring) {
-  const int pl = ring >> 2, q = ring & 3, gp = blockIdx.x * kParents + pl;
+__device__ __forceinline__ RingRef ring_ref(const BandArgs &A, int bx, int ring) {
+  const int pl = ring >> 2, q = ring & 3, gp = bx * kParents + pl;
   RingRef r{nullptr};
   if (gp >= A.ncols) return r;
   const int rhs = gp / A.nparents, P = gp % A.nparents;
@@ -127,10 +127,11 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   uint32_t *tslot = (uint32_t *)(abar + 2);
   float *fscr = (float *)(abar + 3);  // [8]
   unsigned *pmax = (unsigned *)(abar + 16);  // [kParents] output maxima (FP32 bits)
+  const int bx = blockIdx.x + grid_wait();
   if (threadIdx.x < kParents) pmax[threadIdx.x] = 0u;
   int *pvalid = (int *)(pmax + kParents);  // [kParents] the parent exists and its RHS is active
   if (threadIdx.x < kParents) {
-    const int gp = blockIdx.x * kParents + threadIdx.x;
+    const int gp = bx * kParents + threadIdx.x;
     pvalid[threadIdx.x] = gp < A.ncols && !(A.active && !A.active[gp / A.nparents]);
   }
   // no parent of this CTA exists with an active RHS (converged RHS at the end
@@ -145,9 +146,9 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   // (written by the kernel that produced that level)
   float mx = 0.f;
   if (threadIdx.x == 0) {
-    const int g0 = blockIdx.x * kParents, g1 = min(A.ncols, g0 + kParents) - 1;
+    const int g0 = bx * kParents, g1 = min(A.ncols, g0 + kParents) - 1;
     for (int r = g0 / A.nparents; r <= g1 / A.nparents; r++)
-      mx = fmaxf(mx, __uint_as_float(A.levmax[r * kMaxLevels + A.lvl_in]));
+      mx = fmaxf(mx, __uint_as_float(A.levmax[r * kLevStride + A.lvl_in]));
   }
   if (lane == 0) fscr[warp] = mx;
   if (threadIdx.x == 0) {
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
       const int r = it >> 3, g8 = it & 7;
       __align__(16) __half hr[8], lr[8], hi8[8], li8[8];
       float2 v[8];
-      ring_load8(A, ring_ref(A, r), ch * kKC + g8 * 8, kw0, v);
+      ring_load8(A, ring_ref(A, bx, r), ch * kKC + g8 * 8, kw0, v);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         split_f16(v[k].x * s, hr[k], lr[k]);
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       // the parent is the same for every lane of the warp
-      const int pl = (kParents / 2) * h + 2 * pp + u, gp = blockIdx.x * kParents + pl;
+      const int pl = (kParents / 2) * h + 2 * pp + u, gp = bx * kParents + pl;
       if (!pvalid[pl]) continue;
       const int rhs = gp / A.nparents, P = gp % A.nparents;
       unsigned mbits = 0u;
@@ -256,9 +257,9 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   __syncthreads();
   // the parent level's maximum per RHS, read by the next coarser M2M
   if (threadIdx.x < kParents) {
-    const int gp = blockIdx.x * kParents + threadIdx.x;
+    const int gp = bx * kParents + threadIdx.x;
     if (gp < A.ncols && pmax[threadIdx.x])
-      atomicMax(&A.levmax[(gp / A.nparents) * kMaxLevels + A.lvl_out], pmax[threadIdx.x]);
+      atomicMax(&A.levmax[(gp / A.nparents) * kLevStride + A.lvl_out], pmax[threadIdx.x]);
   }
   if (warp == 0) tmem_dealloc(tmem, kCols);
 }
@@ -277,7 +278,7 @@ struct L2lArgs {
   int nparents, items_per_rhs, nitems;
   const int *active;
   int *err;
-  const unsigned *locmax;  // [R][kMaxLevels] max |re|, |im| of the locals per level (written by M2L)
+  const unsigned *locmax;  // [R][kLevStride] max |re|, |im| of the locals per level (written by M2L)
   int lvl_in;
 };
 
@@ -332,9 +333,14 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
     while (w < A.nitems && A.active && !A.active[w / A.items_per_rhs]);
     return w;
   };
-  const int first = (A.active && !A.active[blockIdx.x / A.items_per_rhs]) ? next_item(blockIdx.x) : blockIdx.x;
+  if (threadIdx.x == 0) {  // the anterpolation matrix, which no earlier kernel writes
+    mbar_expect_tx(Bq.abar, 512 * Kp);
+    bulk_g2s(sm + L.a, A.A, 512 * Kp, Bq.abar);
+  }
+  const int blk = blockIdx.x + grid_wait();
+  const int first = (A.active && !A.active[blk / A.items_per_rhs]) ? next_item(blk) : blk;
   auto scale_of = [&](int w) {
-    return pow2_scale(1.5f * A.shl_max * __uint_as_float(A.locmax[(w / A.items_per_rhs) * kMaxLevels + A.lvl_in]));
+    return pow2_scale(1.5f * A.shl_max * __uint_as_float(A.locmax[(w / A.items_per_rhs) * kLevStride + A.lvl_in]));
   };
   // an item's ppi consecutive parent rings: one bulk copy
   const uint32_t run = (uint32_t)A.ppi * A.ns_in * 8;
@@ -349,10 +355,6 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
   if (warp < R::conv_warps) {
     // ---- converters: B[b] rows 8 parent + 2 q + (re, im) = shl[q][j] z[j] s ----
     if (warp == 0) {
-      if (lane == 0) {
-        mbar_expect_tx(Bq.abar, 512 * Kp);
-        bulk_g2s(sm + L.a, A.A, 512 * Kp, Bq.abar);
-      }
       if (first < A.nitems) stage(first, 0);
       const int second = first < A.nitems ? next_item(first) : A.nitems;
       if (second < A.nitems) stage(second, 1);
@@ -542,9 +544,14 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
     while (w < A.nitems && A.active && !A.active[w / A.items_per_rhs]);
     return w;
   };
-  const int first = (A.active && !A.active[blockIdx.x / A.items_per_rhs]) ? next_item(blockIdx.x) : blockIdx.x;
+  if (threadIdx.x == 0) {  // the interpolation matrix, which no earlier kernel writes
+    mbar_expect_tx(abar, 512 * Kp * A.mt);
+    bulk_g2s(sm + L.a, A.A, 512 * Kp * A.mt, abar);
+  }
+  const int blk = blockIdx.x + grid_wait();
+  const int first = (A.active && !A.active[blk / A.items_per_rhs]) ? next_item(blk) : blk;
   auto scale_of = [&](int w) {
-    return pow2_scale(__uint_as_float(A.levmax[(w / A.items_per_rhs) * kMaxLevels + A.lvl_in]));
+    return pow2_scale(__uint_as_float(A.levmax[(w / A.items_per_rhs) * kLevStride + A.lvl_in]));
   };
   const int nc = 2 << A.lg_np, npm = (1 << A.lg_np) - 1;
   const uint32_t ring_bytes = (uint32_t)A.ns_in * 8;
@@ -564,11 +571,6 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
   if (warp < R::conv_warps) {
     // ---- converters: B[b] rows 8 parent + 2 q + (re, im) = child q's samples times s ----
     if (warp == 0) {
-      if (lane == 0) {
-        mbar_expect_tx(abar, 512 * Kp * A.mt);
-        bulk_g2s(sm + L.a, A.A, 512 * Kp * A.mt, abar);
-      }
-      __syncwarp();
       if (first < A.nitems) stage(first, 0);
       const int second = first < A.nitems ? next_item(first) : A.nitems;
       if (second < A.nitems) stage(second, 1);
@@ -692,7 +694,7 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
       if (ew == 0 && lane == 0) mbar_arrive(tfree + b);
       // the parent level's maximum for the next transition (omx >= 0: bits order as values)
       const unsigned mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(omx));
-      if (lane == 0 && ok && mbits) atomicMax(&A.levmax[rhs * kMaxLevels + A.lvl_out], mbits);
+      if (lane == 0 && ok && mbits) atomicMax(&A.levmax[rhs * kLevStride + A.lvl_out], mbits);
       w = next_item(w);
     }
   }
@@ -1008,7 +1010,7 @@ static isg_status band_launch(isg_ctx *c, int lvl, const Transition &T, const fl
   A.lvl_in = lvl + 1;
   A.lvl_out = lvl;
   count_launch();
-  k_tc_band<<<dim3((A.ncols + kParents - 1) / kParents, T.mtiles), 256, kSmem, st>>>(A);
+  launch(k_tc_band, dim3((A.ncols + kParents - 1) / kParents, T.mtiles), 256, kSmem, st, A);
   return cuda_check(c, cudaGetLastError(), "band launch");
 }
 
@@ -1046,7 +1048,8 @@ bool band_m2m(isg_ctx *c, int lvl, float2 *mul, int nrhs, const int *active, cud
     A.lvl_in = lvl + 1;
     A.lvl_out = lvl;
     count_launch();
-    k_tc_m2m<M2mRoles><<<std::min(A.nitems, c->band->sms), M2mRoles::threads, M2mSmem(T.Kp, T.ppi, ch.ns, T.mt).total, st>>>(A);
+    launch(k_tc_m2m<M2mRoles>, std::min(A.nitems, c->band->sms), M2mRoles::threads,
+           M2mSmem(T.Kp, T.ppi, ch.ns, T.mt).total, st, A);
     *e = cuda_check(c, cudaGetLastError(), "m2m launch");
     return true;
   }
@@ -1085,7 +1088,8 @@ bool band_l2l(isg_ctx *c, int lvl, float2 *loc, int nrhs, const int *active, cud
   A.active = active;
   A.err = c->tc_err_flag();
   count_launch();
-  k_tc_l2l<L2lRoles><<<std::min(A.nitems, c->band->sms), L2lRoles::threads, L2lSmem(T.Kp, T.ppi, p.ns).total, st>>>(A);
+  launch(k_tc_l2l<L2lRoles>, std::min(A.nitems, c->band->sms), L2lRoles::threads, L2lSmem(T.Kp, T.ppi, p.ns).total, st,
+         A);
   *e = cuda_check(c, cudaGetLastError(), "l2l launch");
   return true;
 }
