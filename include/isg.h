@@ -296,7 +296,7 @@ isg_status isg_make_line_sources(const isg_ctx *ctx, int ntx, int first, int cou
 
 /* ---- launch-shape autotuner (no counterpart in the reference) ----
  * Times the candidate launch shapes of the level-dependent kernels (M2L rows
- * per thread, L2L and M2M columns per block, near-field tiles per tensor-core
+ * per thread, L2L and SIMT M2M columns per block, near-field tiles per tensor-core
  * CTA) on the context's buffers with nrhs right-hand sides and keeps the
  * fastest per level; later calls with at least nrhs / 4 RHS use them.  The
  * outputs do not depend on the shapes.  Overwrites the context's multipole and

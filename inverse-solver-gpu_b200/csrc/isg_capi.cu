@@ -324,11 +324,7 @@ isg_status isg_setup_gpu(isg_ctx *c) {
         sl[q] = to_f2(T.shiftloc[i][q]);
       }
       if ((e = upload(c, &d.ifirst, f)) || (e = upload(c, &d.iw, w)) || (e = upload(c, &d.shm, sm)) ||
-          (e = upload(c, &d.shl, sl)))
-        return e;
-      if ((e = upload_tile_band(c, &d.mt, T.intind[i], T.interp[i], ni, ni, d.ns, T.nsamp[i + 1], 2 * kTileOut)) ||
-          (e = upload(c, &d.shmT, transpose4(T.shiftmul[i], d.ns))) ||
-          (e = upload(c, &d.shlT, transpose4(T.shiftloc[i], d.ns))))
+          (e = upload(c, &d.shl, sl)) || (e = upload(c, &d.shlT, transpose4(T.shiftloc[i], d.ns))))
         return e;
     }
     if (i >= 1) {

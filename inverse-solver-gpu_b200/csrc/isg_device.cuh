@@ -44,14 +44,12 @@ struct DevLevel {
   float *aw = nullptr;     // [awidth][ns]
   int awidth = 0;
   float2 *T = nullptr;     // [49][ns] translation operators (level >= 2)
-  TileBand mt;             // interpolation into this level (M2M), tiled
   TileBand at;             // anterpolation into this level (L2L), tiled
-  float2 *shmT = nullptr;  // [ns][4] shm transposed
   float2 *shlT = nullptr;  // [ns][4] shl transposed
   // launch shapes picked by isg_autotune (0: the built-in choice)
   int m2l_ty = 0;    // sibling-group rows per M2L thread
   int l2l_cols = 0;  // columns per L2L tile block
-  int m2m_cols = 0;  // columns per M2M tile block
+  int m2m_cols = 0;  // M2M columns (four threads, two samples each) per block
 };
 
 struct DevPlan {

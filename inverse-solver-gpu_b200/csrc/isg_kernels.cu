@@ -30,12 +30,15 @@ namespace {
 // block, 4096: 20.2 / 15.3 / 27.0, 16384: 40.3 / 30.0 / 32.1.  Near field by
 // leaves: 256: 22.5 / 43.9 / 72.7 with 2 x 2, 4 x 4 and 4 x 8 leaves, 1024: 30.8 /
 // 45.0 / 75.8, 2048: 62.4 / 45.1 / 75.8, 4096: 90.6 / 62.0 / 76.3, 8192: 149 / 115
-// / 88.  All M2M levels of 1024 x 1024 x 1 (up to 425984 outputs) 70.8 direct,
-// 102.6 tiled; L2L (with M2L) of 256 x 256 x 2 (139264 leaf outputs) 61.5 / 73.5,
-// of 512 x 512 x 2 (212992 and 557056 outputs) 111 / 103.
+// / 88.  M2M with one and two samples a thread, all levels: one sample up to 142336
+// outputs 151.9 / 153.6, up to 180224 55.4 / 53.3, 212992 44.2 / 38.8.  L2L (with M2L)
+// with one child and four a thread: up to 45056 outputs 58.5 / 60.4, 69632 46.0 /
+// 47.4, 106496 68.9 / 70.7 and 56.3 / 56.3, 139264 38.8 / 34.8; four a thread and
+// tiled: 139264 34.8 / 38.9, 212992 49.1 / 53.3, 557056 46.0 / 49.1, 720896 223.7 /
+// 224.5, 1114112 114.6 / 107.9, 1703936 234.3 / 223.7.
 constexpr int64_t kP2mSmall = 2048, kP2mMid = 16384;
 constexpr int64_t kNearSmall = 1024, kNearMid = 4096;
-constexpr int64_t kM2mDirect = 500000, kL2lDirect = 200000;
+constexpr int64_t kM2mSingle = 150000, kL2lSingle = 110000, kL2lDirect = 600000;
 
 __device__ __forceinline__ bool inactive(const int *active, int rhs) { return active && !active[rhs]; }
 
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(kM2lThreads, NC == 1 ? 3 : 2) k_m2l(M2lArgs A)
   }
 }
 
-// Tiled M2M / L2L.  A column is one (RHS, parent) pair.  A block takes `cols`
+// Tiled L2L.  A column is one (RHS, parent) pair.  A block takes `cols`
 // columns and one tile of tb.out output samples; tb.out / kTileOut threads per
 // column each accumulate kTileOut of them.  The block stages the tile's input
 // window of every ring it reads in shared memory ([window sample][ring],
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(kM2lThreads, NC == 1 ? 3 : 2) k_m2l(M2lArgs A)
 // worked out the ring's address.  Each thread then walks the window once with
 // its kTileOut x 4 accumulators live: the band weights (and the L2L shift
 // phases) are the same for every thread of the block, so each staged value
-// feeds 32 (M2M) or 36 (L2L) FMAs from registers.  Outputs go back through
+// feeds 36 FMAs from registers.  Outputs go back through
 // shared memory so that every ring is written in runs of tb.out samples.
 struct TileArgs {
   const float2 *src;
@@ -295,7 +298,7 @@ struct TileArgs {
   size_t mp, off_in, off_out;
   int n_p, ns_in, ns_out, nparent, ncols, cols;
   TileBand tb;
-  const float2 *shT;  // [ns][4]: L2L shiftloc of the parent level, M2M shiftmul of the parent level
+  const float2 *shT;  // [ns][4]: shiftloc of the parent level
   const int *active;
 };
 
@@ -423,87 +426,16 @@ __global__ void __launch_bounds__(128) k_l2l_tile(TileArgs A) {
   }
 }
 
-// M2M into each column's parent: the four children's rings interpolated by the
-// tile's band weights, then shifted by shm[q][k] and summed.
-__global__ void __launch_bounds__(128) k_m2m_tile(TileArgs A) {
-  extern __shared__ float2 sm[];
-  const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = (blockIdx.x + grid_wait()) * cols;
-  if (!any_active_column(A, c0)) return;
-  const int a0 = A.tb.a0[tile], wl = A.tb.wl[tile], ld = 4 * cols + 1;
-  const TileSmem L(A.tb.wmax, ld, TO, 4 * cols, cols, (size_t)TO * (cols + 1));
-  const float2 **sp = (const float2 **)(sm + L.src);
-  float2 **dp = (float2 **)(sm + L.dst);
-  float4 *sw = (float4 *)(sm + L.w);
-  const int n_c = 2 * A.n_p;
-  for (int t = threadIdx.x; t < 4 * cols; t += blockDim.x) {
-    sp[t] = ring_ptr(A, A.src, A.off_in, c0 + (t >> 2), t & 3, n_c, A.ns_in);
-    if (t < cols) dp[t] = (float2 *)ring_ptr(A, A.dst, A.off_out, c0 + t, -1, A.n_p, A.ns_out);
-  }
-  {
-    const float4 *wt = (const float4 *)(A.tb.w + (size_t)tile * A.tb.wmax * TO);
-    for (int e = threadIdx.x; e < wl * TO / 4; e += blockDim.x) cp_async16(sw + e, wt + e);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int r = warp; r < 4 * cols; r += nw) {
-    const float2 *ring = sp[r];
-    float2 *dst = sm + (r & 3) * cols + (r >> 2);
-    for (int jj = lane; jj < wl; jj += 32) {
-      int j = a0 + jj;
-      if (j >= A.ns_in) j -= A.ns_in;
-      cp_async8(dst + jj * ld, ring ? ring + j : A.src, ring != nullptr);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  const int col = threadIdx.x % cols, sub = threadIdx.x / cols;
-  float2 acc[kTileOut][4] = {};
-  const int wstep = TO / 4;
-  const int2 span = A.tb.span[tile * (TO / kTileOut) + sub];
-#pragma unroll 2
-  for (int jj = span.x; jj < span.y; jj++) {
-    float2 v[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) v[q] = sm[jj * ld + q * cols + col];
-    const float4 w0 = sw[jj * wstep + 2 * sub], w1 = sw[jj * wstep + 2 * sub + 1];
-    const float wv[kTileOut] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-    for (int i = 0; i < kTileOut; i++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) rfma(acc[i][q], wv[i], v[q]);
-  }
-  const float4 *sh = (const float4 *)A.shT;
-  float2 res[kTileOut];
-#pragma unroll
-  for (int i = 0; i < kTileOut; i++) {
-    const int k = min(tile * TO + sub * kTileOut + i, A.ns_out - 1);
-    const float4 s01 = __ldg(sh + 2 * k), s23 = __ldg(sh + 2 * k + 1);
-    res[i] = make_float2(0.f, 0.f);
-    cfma(res[i], make_float2(s01.x, s01.y), acc[i][0]);
-    cfma(res[i], make_float2(s01.z, s01.w), acc[i][1]);
-    cfma(res[i], make_float2(s23.x, s23.y), acc[i][2]);
-    cfma(res[i], make_float2(s23.z, s23.w), acc[i][3]);
-  }
-  __syncthreads();
-  const int ldo = cols + 1;
-#pragma unroll
-  for (int i = 0; i < kTileOut; i++) sm[(sub * kTileOut + i) * ldo + col] = res[i];
-  __syncthreads();
-  for (int e = threadIdx.x; e < cols * TO; e += blockDim.x) {
-    const int i = e % TO, cl = e / TO, kp = tile * TO + i;
-    float2 *d = dp[cl];
-    if (d && kp < A.ns_out) d[kp] = sm[i * ldo + cl];
-  }
-}
-
-
-// M2M and L2L of a small launch: one thread per output sample, the taps read
-// straight from L1 / L2 (consecutive threads take consecutive samples, so the
-// loads of a warp fall on the same few lines).  The tiled kernels above stage
-// 32 or more columns per block and read each value once; a launch with fewer
-// outputs than kM2mDirect or kL2lDirect leaves most SMs without a block there
-// and is as long as one block's chain of staging, walk and write-back.  Both add
-// an output's taps in ring order, with the same roundings.
+// M2M and L2L with the taps read straight from L1 / L2, consecutive threads on
+// consecutive samples (the loads of a warp fall on the same few lines): no staging,
+// no block barrier.  On large launches L1 bounds them.  So an M2M thread takes S = 2
+// consecutive samples of a parent and reads a child's value once for both; a parent's
+// ring has at least its children's samples (both multiples of four), so the windows
+// start at most one tap apart.  An L2L thread takes one sample of all C = 4 children
+// and reads a parent's value once for four; the shifts of opposite children are
+// conjugates of each other.  On small launches the time is one thread's chain of
+// loads, which S = 1 and C = 1 keep shortest.  M2M of 1024 x 1024 x 16, all levels:
+// 450 us, tiled through shared memory 642; x 1: 62 / 94.
 struct DirectArgs {
   const float2 *src;  // input level, one RHS' block every mp elements
   float2 *dst;
@@ -511,34 +443,61 @@ struct DirectArgs {
   int n_p, ns_in, ns_out, width;
   const int *first;    // [ns_out] first tap
   const float *w;      // [width][ns_out]
-  const float2 *shift; // M2M shiftmul [4][ns_out], L2L shiftloc [4][ns_in]
+  const float2 *shift; // M2M shiftmul [4][ns_out], L2L shiftloc [4][ns_in] (C = 1) or [ns_in][4]
   const int *active;
 };
 
-__global__ void __launch_bounds__(128) k_m2m_direct(DirectArgs A) {
+template <int S>
+__global__ void __launch_bounds__(256) k_m2m_direct(DirectArgs A) {
   const int rhs = blockIdx.y + grid_wait();
   if (inactive(A.active, rhs)) return;
-  const int o = blockIdx.x * blockDim.x + threadIdx.x, P = o / A.ns_out, k = o - P * A.ns_out;
+  const int per = A.ns_out / S, o = blockIdx.x * blockDim.x + threadIdx.x, P = o / per, k = S * (o - P * per);
   if (P >= A.n_p * A.n_p) return;
   const int py = P / A.n_p, px = P - py * A.n_p, n_c = 2 * A.n_p;
   const float2 *c0 = A.src + (size_t)rhs * A.mp + (size_t)(2 * py * n_c + 2 * px) * A.ns_in;
   const float2 *c[4] = {c0, c0 + A.ns_in, c0 + (size_t)n_c * A.ns_in, c0 + (size_t)(n_c + 1) * A.ns_in};
-  float2 acc[4] = {};
+  float2 acc[S][4] = {};
   int j = A.first[k];
-#pragma unroll 10
-  for (int t = 0; t < A.width; t++) {
-    const float w = __ldg(&A.w[(size_t)t * A.ns_out + k]);
+  const bool late = S == 2 && A.first[k + S - 1] != j;  // the second sample's window starts a tap later
+  float before = 0.f;
+  auto tap = [&](const float (&w)[S]) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) rfma(acc[q], w, c[q][j]);
+    for (int q = 0; q < 4; q++) {
+      const float2 v = c[q][j];
+#pragma unroll
+      for (int i = 0; i < S; i++) rfma(acc[i][q], w[i], v);
+    }
     if (++j == A.ns_in) j = 0;
+  };
+#pragma unroll(S == 1 ? 10 : 6)
+  for (int t = 0; t < A.width; t++) {
+    const float *w = &A.w[(size_t)t * A.ns_out + k];
+    if constexpr (S == 1) {
+      tap({__ldg(w)});
+    } else {
+      const float2 w2 = __ldg((const float2 *)w);
+      tap({w2.x, late ? before : w2.y});
+      before = w2.y;
+    }
   }
-  float2 r = make_float2(0.f, 0.f);
+  if constexpr (S == 2) {
+    if (late) tap({0.f, before});
+  }
+  float2 res[S] = {};
 #pragma unroll
-  for (int q = 0; q < 4; q++) cfma(r, __ldg(&A.shift[q * A.ns_out + k]), acc[q]);
-  A.dst[(size_t)rhs * A.mp + o] = r;
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int i = 0; i < S; i++) cfma(res[i], __ldg(&A.shift[q * A.ns_out + k + i]), acc[i][q]);
+  float2 *dst = A.dst + (size_t)rhs * A.mp + (size_t)P * A.ns_out + k;
+#pragma unroll
+  for (int i = 0; i < S; i++) dst[i] = res[i];
 }
 
-__global__ void __launch_bounds__(128) k_l2l_direct(DirectArgs A) {
+template <int C>
+__global__ void __launch_bounds__(128) k_l2l_direct(DirectArgs A);
+
+template <>
+__global__ void __launch_bounds__(128) k_l2l_direct<1>(DirectArgs A) {
   const int rhs = blockIdx.y + grid_wait();
   if (inactive(A.active, rhs)) return;
   const int o = blockIdx.x * blockDim.x + threadIdx.x, c = o / A.ns_out, k = o - c * A.ns_out, n_c = 2 * A.n_p;
@@ -556,6 +515,36 @@ __global__ void __launch_bounds__(128) k_l2l_direct(DirectArgs A) {
     if (++j == A.ns_in) j = 0;
   }
   A.dst[(size_t)rhs * A.mp + o] = acc;
+}
+
+template <>
+__global__ void __launch_bounds__(128) k_l2l_direct<4>(DirectArgs A) {
+  const int rhs = blockIdx.y + grid_wait();
+  if (inactive(A.active, rhs)) return;
+  const int o = blockIdx.x * blockDim.x + threadIdx.x, P = o / A.ns_out, k = o - P * A.ns_out;
+  if (P >= A.n_p * A.n_p) return;
+  const float2 *z = A.src + (size_t)rhs * A.mp + (size_t)P * A.ns_in;
+  float2 acc[4] = {};
+  int j = A.first[k];
+#pragma unroll 6
+  for (int t = 0; t < A.width; t++) {
+    const float w = __ldg(&A.w[(size_t)t * A.ns_out + k]);
+    const float4 s = __ldg((const float4 *)&A.shift[4 * j]);  // children 0 and 1; 3 and 2 are their conjugates
+    const float2 v = z[j];
+    // the products of k_l2l_tile, with its roundings
+    const float ax = __fmul_rn(s.x, v.x), ay = __fmul_rn(s.x, v.y), bx = __fmul_rn(s.z, v.x), by = __fmul_rn(s.z, v.y);
+    rfma(acc[0], w, make_float2(fmaf(-s.y, v.y, ax), fmaf(s.y, v.x, ay)));
+    rfma(acc[3], w, make_float2(fmaf(s.y, v.y, ax), fmaf(-s.y, v.x, ay)));
+    rfma(acc[1], w, make_float2(fmaf(-s.w, v.y, bx), fmaf(s.w, v.x, by)));
+    rfma(acc[2], w, make_float2(fmaf(s.w, v.y, bx), fmaf(-s.w, v.x, by)));
+    if (++j == A.ns_in) j = 0;
+  }
+  const int py = P / A.n_p, px = P - py * A.n_p, n_c = 2 * A.n_p;
+  float2 *d = A.dst + (size_t)rhs * A.mp + (size_t)(2 * py * n_c + 2 * px) * A.ns_out + k;
+  d[0] = acc[0];
+  d[A.ns_out] = acc[1];
+  d[(size_t)n_c * A.ns_out] = acc[2];
+  d[(size_t)(n_c + 1) * A.ns_out] = acc[3];
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -897,18 +886,12 @@ int64_t level_outputs(const DevPlan &P, int lvl, int nrhs) {
 
 void launch_m2m(const DevPlan &P, int lvl, float2 *mul, int nrhs, const int *active, cudaStream_t st) {
   const DevLevel &p = P.lv[lvl], &c = P.lv[lvl + 1];
-  if (level_outputs(P, lvl, nrhs) <= kM2mDirect) {
-    const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
-    count_launch();
-    launch(k_m2m_direct, dim3((p.n * p.n * p.ns + 127) / 128, nrhs), 128, 0, st, D);
-    return;
-  }
-  const int cap = (p.m2m_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? p.m2m_cols : 32;
-  const TileArgs A = tile_args(mul, mul, P.mp, c.off, p.off, p.n, c.ns, p.ns, nrhs, p.mt, p.shmT, cap, active);
-  const TileSmem L(p.mt.wmax, 4 * A.cols + 1, p.mt.out, 4 * A.cols, A.cols, (size_t)p.mt.out * (A.cols + 1));
-  const size_t smem = L.total * sizeof(float2);
+  const DirectArgs D{mul + c.off, mul + p.off, P.mp, p.n, c.ns, p.ns, P.ninter, p.ifirst, p.iw, p.shm, active};
+  const int threads = 4 * ((p.m2m_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? p.m2m_cols : 32);
+  const int64_t out = level_outputs(P, lvl, nrhs);
+  const int S = out <= kM2mSingle ? 1 : 2, samples = p.n * p.n * p.ns / S;
   count_launch();
-  launch(k_m2m_tile, dim3((A.ncols + A.cols - 1) / A.cols, p.mt.tiles), A.cols * (p.mt.out / kTileOut), smem, st, A);
+  launch(S == 1 ? k_m2m_direct<1> : k_m2m_direct<2>, dim3((samples + threads - 1) / threads, nrhs), threads, 0, st, D);
 }
 
 void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int nrhs, const int *active, bool accumulate,
@@ -951,10 +934,13 @@ void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int n
 
 void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *active, cudaStream_t st) {
   const DevLevel &c = P.lv[lvl], &p = P.lv[lvl - 1];
-  if (level_outputs(P, lvl, nrhs) <= kL2lDirect) {
-    const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw, p.shl, active};
+  const int64_t out = level_outputs(P, lvl, nrhs);
+  if (out <= kL2lDirect) {
+    const int C = out <= kL2lSingle ? 1 : 4, samples = 4 * p.n * p.n * c.ns / C;
+    const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw,
+                       C == 1 ? p.shl : p.shlT, active};
     count_launch();
-    launch(k_l2l_direct, dim3((c.n * c.n * c.ns + 127) / 128, nrhs), 128, 0, st, D);
+    launch(C == 1 ? k_l2l_direct<1> : k_l2l_direct<4>, dim3((samples + 127) / 128, nrhs), 128, 0, st, D);
     return;
   }
   const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : 64;
@@ -1051,7 +1037,6 @@ cudaError_t kernels_setup() {
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e == cudaSuccess) e = allow_max_smem(k_m2m_tile, optin);
   if (e == cudaSuccess) e = allow_max_smem(k_l2l_tile, optin);
   if (e == cudaSuccess) e = allow_max_smem(k_near<4, 8>, optin);
   if (e == cudaSuccess) e = allow_max_smem(k_near<4, 4>, optin);
@@ -1069,8 +1054,8 @@ cudaError_t aggregate_kernels_load() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<2, 1>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<8, 2>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_p2m<32, 4>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_direct);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_tile);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_direct<1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_m2m_direct<2>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_rx_interp);
   return e;
 }

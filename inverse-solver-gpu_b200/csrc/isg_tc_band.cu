@@ -47,11 +47,11 @@ constexpr int kAHalf = 128 * kKC * 2;    // 16 KB: one FP16 split of an A chunk
 constexpr int kBHalf = kCols * kKC * 2;  // 16 KB
 constexpr int kSmem = 2 * kAHalf + 2 * kBHalf + 256 + 4 * kParents;  // + barriers, TMEM slot, scratch, per-parent maxima and flags
 constexpr int kErrBand = 121;
-// Largest level (samples of all clusters and RHS) that M2M leaves to the direct
-// kernel, where k_tc_m2m and where k_tc_band would take it: M2M of all levels
-// with and without, 256 x 256 x 1 at 11264 samples 29.7 / 30.7 us, at 26624
-// 31.9 / 29.7; 256 x 256 x 16 at 78848 34.1 / 38.4, x 64 at 142336 58.3 / 58.4.
-constexpr int64_t kPipeDirect = 16000, kBandDirect = 140000;
+// Largest level (samples of all clusters and RHS) that k_tc_band leaves to the
+// SIMT M2M, by the times of all levels with and without: 78848 samples 31.2 / 34.0
+// us, 142336 51.9 / 52.2, 180224 41.3 / 40.9, 293568 95.3 / 93.4, 360448 39.5 / 32.7.
+// k_tc_m2m beats the SIMT kernel at every size from 6656 samples on.
+constexpr int64_t kBandDirect = 140000;
 
 struct BandArgs {
   const float2 *src;  // child-level multipoles (level base)
@@ -1020,7 +1020,7 @@ bool band_m2m(isg_ctx *c, int lvl, float2 *mul, int nrhs, const int *active, cud
   // Small launches take launch_m2m's one thread per output.  Every coarser level
   // is smaller and has at most the same bound, so no kernel that needs this
   // level's maximum follows.  At the bound both take 10 to 14 us.
-  if (level_outputs(c->P, lvl, nrhs) <= (c->band->pm2m[lvl].ok ? kPipeDirect : kBandDirect)) return false;
+  if (!c->band->pm2m[lvl].ok && level_outputs(c->P, lvl, nrhs) <= kBandDirect) return false;
   if (c->band->pm2m[lvl].ok) {
     const M2mPlan &T = c->band->pm2m[lvl];
     M2mArgs A;

@@ -1,9 +1,8 @@
 """Launch shapes: small and large launches of the same kernels agree.
 
-The plain engine's shapes (leaves per P2M and near-field block, one thread per
-output or tiles for M2M / L2L) add every output's terms in the same order, so a
-right-hand side alone and inside a batch that takes the larger shapes must agree
-bit for bit.  The tensor engine's near-field items (8, 16 or 32 leaf rows) are
+The plain engine's shapes (leaves per P2M and near-field block, direct or tiled L2L)
+add every output's terms in the same order, so a right-hand side alone and inside a
+batch that takes the larger shapes must agree bit for bit.  The tensor engine's near-field items (8, 16 or 32 leaf rows) are
 compared with the plain engine at the tolerance of its split products."""
 import math
 
@@ -22,7 +21,7 @@ def _rand(n, U, seed):
 
 
 # 64 leaves per RHS: 2 x 2-leaf blocks alone, 4 x 4 at 20, 4 x 8 from 65, the largest P2M
-# blocks from 257 and the tiled M2M from 301 (1664 outputs each), the tiled L2L from 46 (4352)
+# blocks from 257, the tiled L2L from 138 (4352 outputs each)
 @pytest.mark.parametrize("nrhs", [17, 20, 47, 65, 257, 305])
 def test_plain_shapes_agree_bit_for_bit(nrhs):
     import torch
