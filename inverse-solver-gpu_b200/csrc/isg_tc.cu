@@ -1102,19 +1102,23 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
         const uint64_t ah0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b), 128, 2048);
         const uint64_t al0 = smem_desc(sbase + (uint32_t)P2mPipeSmem::a(b) + kP2mA, 128, 2048);
         const uint32_t d = tmem + (uint32_t)(b * 256);
-        for (int c = 0; c < 4; c++) {
-          const uint32_t aoff0 = (uint32_t)c * 512, boff0 = c * A.stage_bytes;
-          if (elect_one()) {
+        for (int pass = 0; pass < 2; pass++)  // the small products first, as in k_tc_l2l
+          for (int c = 0; c < 4; c++) {
+            const uint32_t aoff0 = (uint32_t)c * 512, boff0 = c * A.stage_bytes;
+            if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-              const uint32_t aoff = aoff0 + ks * 256, boff = boff0 + ks * 256;
-              mma_f16(d, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, (c | ks) ? 1 : 0);
-              mma_f16(d, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, 1);
-              mma_f16(d, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
+              for (int ks = 0; ks < 2; ks++) {
+                const uint32_t aoff = aoff0 + ks * 256, boff = boff0 + ks * 256;
+                if (pass == 0) {
+                  mma_f16(d, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, (c | ks) ? 1 : 0);
+                  mma_f16(d, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
+                } else {
+                  mma_f16(d, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, 1);
+                }
+              }
             }
+            __syncwarp();
           }
-          __syncwarp();
-        }
       }
       if (elect_one()) mma_commit(Bq.tfull + b);
       __syncwarp();

@@ -50,7 +50,7 @@ constexpr int kErrBand = 121;
 // Largest level (samples of all clusters and RHS) that k_tc_band leaves to the
 // SIMT M2M, by the times of all levels with and without: 78848 samples 31.2 / 34.0
 // us, 142336 51.9 / 52.2, 180224 41.3 / 40.9, 293568 95.3 / 93.4, 360448 39.5 / 32.7.
-// k_tc_m2m beats the SIMT kernel at every size from 6656 samples on.
+// k_tc_m2m and k_tc_l2l beat the SIMT kernels at every size from 6656 samples on.
 constexpr int64_t kBandDirect = 140000;
 
 struct BandArgs {
@@ -265,6 +265,12 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
 }
 
 // ---- L2L ----
+// The tensor cores cut off what an accumulator cannot hold at every MMA.  So the two
+// cross products of the split (hi lo, lo hi) go in first for the whole of K, while the
+// accumulator is 2^-11 of the result, and hi hi last: Kp / 16 roundings of the full sum
+// in place of 3 Kp / 16.  With k_tc_m2m and the P2M in this order the error of the
+// operator against 64 bits went from 2.28e-6 to 1.97e-6 at 256 x 256 and from 2.14e-6
+// to 1.59e-6 at 512 x 512 (random inputs), at the same time or less.
 constexpr int kErrL2l = 122;
 
 struct L2lArgs {
@@ -419,10 +425,14 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
         for (int ks = 0; ks < Kp / 16; ks++) {
           const uint32_t k = ks * 256;
           if (elect_one()) {
-            mma_f16(d, desc_add(ah, k), desc_add(bh, k), idesc, ks ? 1 : 0);
-            mma_f16(d, desc_add(ah, k), desc_add(bl, k), idesc, 1);
+            mma_f16(d, desc_add(ah, k), desc_add(bl, k), idesc, ks ? 1 : 0);
             mma_f16(d, desc_add(al, k), desc_add(bh, k), idesc, 1);
           }
+          __syncwarp();
+        }
+        for (int ks = 0; ks < Kp / 16; ks++) {
+          const uint32_t k = ks * 256;
+          if (elect_one()) mma_f16(d, desc_add(ah, k), desc_add(bh, k), idesc, 1);
           __syncwarp();
         }
       }
@@ -446,17 +456,18 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
       tc_fence_after();
       const int rhs = w / A.items_per_rhs, p0 = (w % A.items_per_rhs) * A.ppi;
       const float inv = A.inv_a / scale_of(w);
-      // the item's parents share a row: parent p0 + pl's first child is 2 pl clusters on
-      float2 *ob = A.loc + (size_t)rhs * A.mp + A.off_out + km +
-                   (size_t)(2 * (p0 >> A.lg_np) * nc + 2 * (p0 & npm)) * so;
+      float2 *ob = A.loc + (size_t)rhs * A.mp + A.off_out + km;
       for (int cg = 0; cg < N / (32 * R::epi_groups); cg++) {  // 32 columns = 4 parents
         const int col0 = ch0 * (N / R::epi_groups) + 32 * cg;
         float d[32];
         tmem_ld32(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(b * N + col0), d);
         if (!ok || km >= A.ns_out) continue;
+        // the four parents share a row: each one's first child is two clusters on
+        const int pf = p0 + col0 / 8;
+        float2 *of = ob + (size_t)(2 * (pf >> A.lg_np) * nc + 2 * (pf & npm)) * so;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          float2 *o = ob + (size_t)2 * (col0 / 8 + u) * so;
+          float2 *o = of + (size_t)2 * u * so;
 #pragma unroll
           for (int q = 0; q < 4; q++) o[qoff[q]] = make_float2(d[8 * u + 2 * q] * inv, d[8 * u + 2 * q + 1] * inv);
         }
@@ -630,13 +641,17 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
         const uint64_t bl = smem_desc(smem_u32(bbuf(b)) + N * Kp * 2, 128, sbo);
         for (int t = 0; t < A.mt; t++) {
           const uint32_t d = tmem + (uint32_t)((b * A.mt + t) * N), ta = t * tile_bytes;
-          for (int ks = 0; ks < Kp / 16; ks++) {
+          for (int ks = 0; ks < Kp / 16; ks++) {  // the small products first, as in k_tc_l2l
             const uint32_t k = ks * 256;
             if (elect_one()) {
-              mma_f16(d, desc_add(ah, ta + k), desc_add(bh, k), idesc, ks ? 1 : 0);
-              mma_f16(d, desc_add(ah, ta + k), desc_add(bl, k), idesc, 1);
+              mma_f16(d, desc_add(ah, ta + k), desc_add(bl, k), idesc, ks ? 1 : 0);
               mma_f16(d, desc_add(al, ta + k), desc_add(bh, k), idesc, 1);
             }
+            __syncwarp();
+          }
+          for (int ks = 0; ks < Kp / 16; ks++) {
+            const uint32_t k = ks * 256;
+            if (elect_one()) mma_f16(d, desc_add(ah, ta + k), desc_add(bh, k), idesc, 1);
             __syncwarp();
           }
         }
@@ -829,14 +844,14 @@ static isg_status build_l2l(isg_ctx *c, int i, size_t smem_cap) {
   L2lPlan &T = c->band->l2l[i];
   if (ns_out > 128) return ISG_OK;
   const int Kp = (ns_in + 15) / 16 * 16;
+  const int nparents = 1 << (2 * (i - 1));
   int ppi = 0;
   for (int cand : {32, 16, 8})
-    if (L2lSmem(Kp, cand, ns_in).total <= smem_cap) {
+    if (nparents % cand == 0 && L2lSmem(Kp, cand, ns_in).total <= smem_cap) {
       ppi = cand;
       break;
     }
-  const int nparents = 1 << (2 * (i - 1));
-  if (!ppi || nparents % ppi || (1 << (i - 1)) < ppi) return ISG_OK;  // an item's parents share a row
+  if (!ppi || i < 3) return ISG_OK;  // four parents next to each other share a row
   std::vector<double> dense((size_t)128 * Kp, 0.0);
   for (int k = 0; k < ns_out; k++)
     for (int t = 0; t < taps; t++) {
@@ -1075,20 +1090,23 @@ bool band_l2l(isg_ctx *c, int lvl, float2 *loc, int nrhs, const int *active, cud
   A.ns_out = ch.ns;
   A.Kp = T.Kp;
   A.kc_magic = T.kc_magic;
+  A.nparents = p.n * p.n;
+  // fewer parents per item while the GPU has fewer items than SMs (L2L and M2L of
+  // 128 x 128 x 32: 36.4 us, L2L with the SIMT kernels 46.4)
   A.ppi = T.ppi;
+  while (A.ppi > 8 && A.nparents / A.ppi * nrhs < c->band->sms) A.ppi /= 2;
   A.A = T.A;
   A.shl = p.shlT;
   A.inv_a = T.inv_a;
   A.shl_max = T.shl_max;
   A.locmax = c->locmax;
   A.lvl_in = lvl - 1;
-  A.nparents = p.n * p.n;
-  A.items_per_rhs = A.nparents / T.ppi;
+  A.items_per_rhs = A.nparents / A.ppi;
   A.nitems = A.items_per_rhs * nrhs;
   A.active = active;
   A.err = c->tc_err_flag();
   count_launch();
-  launch(k_tc_l2l<L2lRoles>, std::min(A.nitems, c->band->sms), L2lRoles::threads, L2lSmem(T.Kp, T.ppi, p.ns).total, st,
+  launch(k_tc_l2l<L2lRoles>, std::min(A.nitems, c->band->sms), L2lRoles::threads, L2lSmem(T.Kp, A.ppi, p.ns).total, st,
          A);
   *e = cuda_check(c, cudaGetLastError(), "l2l launch");
   return true;

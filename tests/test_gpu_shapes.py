@@ -2,8 +2,9 @@
 
 The plain engine's shapes (leaves per P2M and near-field block, direct or tiled L2L)
 add every output's terms in the same order, so a right-hand side alone and inside a
-batch that takes the larger shapes must agree bit for bit.  The tensor engine's near-field items (8, 16 or 32 leaf rows) are
-compared with the plain engine at the tolerance of its split products."""
+batch that takes the larger shapes must agree bit for bit.  The tensor engine's
+near-field items (8, 16 or 32 leaf rows) and translations are compared with the plain
+engine at the tolerance of its split products."""
 import math
 
 import pytest
@@ -57,6 +58,20 @@ def test_tensor_near_field_items_match_the_plain_engine(level, nrhs):
     gs, u = ((2 * math.pi) ** 2 * chi).to(torch.complex64), torch.zeros_like(x)
     info = s.bicgs(u, gs, x, engine=isg.ENGINE_TENSOR, tol=1e-5)
     assert all(i["status"] == 0 and i["true_residual"] <= 1e-5 for i in info), info
+
+
+# L2L items of 8, 16 and 32 parents on parent grids of 4, 8 and 16 rows (64 leaves: at most 16
+# parents), M2M of the same grids, the SIMT M2M for the coarse levels up to 140000 outputs
+@pytest.mark.parametrize("level,nrhs", [(4, 1), (4, 73), (4, 149), (5, 2), (5, 19), (5, 37), (5, 75), (6, 5), (6, 33)])
+def test_tensor_translations_match_the_plain_engine(level, nrhs):
+    import torch
+    s = isg.Solver(level, max_rhs=nrhs, device=0)
+    x = _rand(nrhs, s.numunk, 8)
+    for conj in (False, True):
+        a, b = s.mlfma(x, conj=conj, engine=isg.ENGINE_TENSOR), s.mlfma(x, conj=conj)
+        # the field of a unit input is a sum of ~650 split products of 2^-22 each
+        for j in range(nrhs):
+            assert torch.linalg.norm(a[j] - b[j]) <= 1e-5 * torch.linalg.norm(b[j])
 
 
 # row pairs aligned to 16 bytes or not (odd receiver counts), one and two accumulator sets,
