@@ -42,16 +42,37 @@ using namespace tc;
 
 constexpr int kCols = 128;        // MMA N: 16 parents x 4 children x (re, im)
 constexpr int kParents = 16;
-constexpr int kKC = 64;           // K chunk
-constexpr int kAHalf = 128 * kKC * 2;    // 16 KB: one FP16 split of an A chunk
-constexpr int kBHalf = kCols * kKC * 2;  // 16 KB
-constexpr int kSmem = 2 * kAHalf + 2 * kBHalf + 256 + 4 * kParents;  // + barriers, TMEM slot, scratch, per-parent maxima and flags
+constexpr int kKC = 32;           // K chunk
+constexpr int kAHalf = 128 * kKC * 2;    // 8 KB: one FP16 split of an A chunk
+constexpr int kBHalf = kCols * kKC * 2;  // 8 KB
+constexpr int kBandBuf = 2 * kAHalf + 2 * kBHalf;  // A hi, lo, B hi, lo
+constexpr int kSmem = 2 * kBandBuf + 256 + 4 * kParents;  // + barriers, TMEM slot, scratch, per-parent maxima and flags
 constexpr int kErrBand = 121;
 // Largest level (samples of all clusters and RHS) that k_tc_band leaves to the
 // SIMT M2M, by the times of all levels with and without: 78848 samples 31.2 / 34.0
 // us, 142336 51.9 / 52.2, 180224 41.3 / 40.9, 293568 95.3 / 93.4, 360448 39.5 / 32.7.
 // k_tc_m2m and k_tc_l2l beat the SIMT kernels at every size from 6656 samples on.
 constexpr int64_t kBandDirect = 140000;
+
+// A ring's real and imaginary row of one 8-sample group, the 16-byte core-matrix rows
+// at o and o + 16 of the hi and lo operand.  Every other group stores the second row
+// first: the eight lanes of a store phase then cover all banks.
+__device__ __forceinline__ void store_rows(char *hi, char *lo, uint32_t o, bool flip, const uint32_t (&hr)[4],
+                                           const uint32_t (&hm)[4], const uint32_t (&lr)[4], const uint32_t (&lm)[4]) {
+  uint32_t h[2][4], l[2][4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    h[0][k] = flip ? hm[k] : hr[k];
+    h[1][k] = flip ? hr[k] : hm[k];
+    l[0][k] = flip ? lm[k] : lr[k];
+    l[1][k] = flip ? lr[k] : lm[k];
+  }
+  const uint32_t o0 = o + (flip ? 16 : 0), o1 = o + (flip ? 0 : 16);
+  st_shared_v4(hi + o0, h[0]);
+  st_shared_v4(hi + o1, h[1]);
+  st_shared_v4(lo + o0, l[0]);
+  st_shared_v4(lo + o1, l[1]);
+}
 
 struct BandArgs {
   const float2 *src;  // child-level multipoles (level base)
@@ -86,46 +107,39 @@ __device__ __forceinline__ RingRef ring_ref(const BandArgs &A, int bx, int ring)
   return r;
 }
 
-// Eight consecutive window samples kk0 .. kk0+7 of a ring (zero outside).
-__device__ __forceinline__ void ring_load8(const BandArgs &A, const RingRef &r, int kk0, int kw0, float2 *v) {
-  int j0;
-  if (kw0 < 0) {
-    j0 = kk0;
-  } else {
-    j0 = (kw0 + kk0) % A.ns_in;  // the window may be longer than the ring; weights past it are zero
-  }
-  if (r.p && !(j0 & 1) && j0 + 8 <= A.ns_in) {  // eight samples inside the ring, 16-byte aligned
-    const float4 *q4 = (const float4 *)(r.p + j0);
+// Eight consecutive window samples kk0 .. kk0+7 of a ring (zero outside).  Window
+// starts and rings are multiples of four samples, so each half lies inside the ring
+// or past its end as a whole.
+__device__ __forceinline__ void ring_load8(const BandArgs &A, const RingRef &r, int kk0, int kw0, float2 (&v)[8]) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float4 t = q4[k];
-      v[2 * k] = make_float2(t.x, t.y);
-      v[2 * k + 1] = make_float2(t.z, t.w);
-    }
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    int j = j0 + k;
+  for (int h = 0; h < 2; h++) {
+    int j = kk0 + 4 * h;
     bool ok = r.p != nullptr;
-    if (kw0 < 0) {
+    if (kw0 < 0)
       ok = ok && j < A.ns_in;
-    } else if (j >= A.ns_in) {
-      j -= A.ns_in;
-    }
-    float2 x = make_float2(0.f, 0.f);
-    if (ok) x = r.p[j];
-    v[k] = x;
+    else
+      j = (kw0 + j) % A.ns_in;  // the window may be longer than the ring; weights past it are zero
+    const float4 *p = (const float4 *)(r.p + j);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = ok ? p[0] : zero, b = ok ? p[1] : zero;
+    v[4 * h] = make_float2(a.x, a.y);
+    v[4 * h + 1] = make_float2(a.z, a.w);
+    v[4 * h + 2] = make_float2(b.x, b.y);
+    v[4 * h + 3] = make_float2(b.z, b.w);
   }
 }
 
+// A CTA takes 128 parent samples of 16 parents and walks its K window in chunks of 32
+// through two buffers: while the tensor core multiplies one chunk, the next one's
+// weights arrive by a bulk copy and its samples, read a chunk ahead into registers,
+// are split into the other buffer.  (Chunks of 64 through one buffer, every step
+// waiting for the one before: M2M of
+// 1024 x 1024 x 64, all levels, 564 us, this 514; x 16 171 / 155.)
 __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   extern __shared__ __align__(1024) char sm[];
-  char *ahi = sm, *bhi = sm + 2 * kAHalf, *blo = bhi + kBHalf;
-  uint64_t *abar = (uint64_t *)(blo + kBHalf);
-  uint64_t *mbar = abar + 1;
-  uint32_t *tslot = (uint32_t *)(abar + 2);
-  float *fscr = (float *)(abar + 3);  // [8]
+  uint64_t *abar = (uint64_t *)(sm + 2 * kBandBuf);  // [2] weights landed
+  uint64_t *mbar = abar + 2;                         // [2] buffer's MMAs complete
+  uint32_t *tslot = (uint32_t *)(abar + 4);
+  float *fscr = (float *)(abar + 5);  // [8]
   unsigned *pmax = (unsigned *)(abar + 16);  // [kParents] output maxima (FP32 bits)
   const int bx = blockIdx.x + grid_wait();
   if (threadIdx.x < kParents) pmax[threadIdx.x] = 0u;
@@ -141,6 +155,12 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   const int mt = blockIdx.y, m0 = mt * 128;
   const int kw0 = A.kw0[mt], nch = A.nchunk[mt];
   const uint8_t *Achunks = A.A + (size_t)A.chunk0[mt] * 2 * kAHalf;
+  // the thread's ring and 8-sample group of every chunk
+  static_assert(4 * kParents * (kKC / 8) == 256, "one group per thread");
+  const int rg = (threadIdx.x & 3) | ((threadIdx.x >> 4) << 2), g8 = (threadIdx.x >> 2) & 3;
+  const RingRef ring = ring_ref(A, bx, rg);
+  float2 v[8];
+  ring_load8(A, ring, g8 * 8, kw0, v);
 
   // power-of-two scale from the input level's maximum over the CTA's RHS
   // (written by the kernel that produced that level)
@@ -152,8 +172,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   }
   if (lane == 0) fscr[warp] = mx;
   if (threadIdx.x == 0) {
-    mbar_init(abar, 1);
-    mbar_init(mbar, 1);
+    for (int i = 0; i < 4; i++) mbar_init(abar + i, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tslot, kCols);
@@ -169,57 +188,49 @@ __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   bool ok = true;
 
   for (int ch = 0; ch < nch; ch++) {
+    const int b = ch & 1;
+    char *buf = sm + b * kBandBuf, *bhi = buf + 2 * kAHalf, *blo = bhi + kBHalf;
+    if (ch >= 2) ok = mbar_wait(mbar + b, ((ch >> 1) - 1) & 1, A.err, kErrBand) && ok;
     if (threadIdx.x == 0) {
-      mbar_expect_tx(abar, 2 * kAHalf);
-      bulk_g2s(ahi, Achunks + (size_t)ch * 2 * kAHalf, 2 * kAHalf, abar);
+      mbar_expect_tx(abar + b, 2 * kAHalf);
+      bulk_g2s(buf, Achunks + (size_t)ch * 2 * kAHalf, 2 * kAHalf, abar + b);
     }
-    // B chunk: ring r gives rows 2r (re) and 2r + 1 (im); item = (ring, 8-sample group)
-#pragma unroll 2
-    for (int it = threadIdx.x; it < 4 * kParents * (kKC / 8); it += blockDim.x) {
-      const int r = it >> 3, g8 = it & 7;
-      __align__(16) __half hr[8], lr[8], hi8[8], li8[8];
-      float2 v[8];
-      ring_load8(A, ring_ref(A, bx, r), ch * kKC + g8 * 8, kw0, v);
+    // ring rg gives B rows 2 rg (re) and 2 rg + 1 (im)
+    uint32_t hr[4], lr[4], hm[4], lm[4];
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        split_f16(v[k].x * s, hr[k], lr[k]);
-        split_f16(v[k].y * s, hi8[k], li8[k]);
-      }
-      const int n0 = 2 * r, n1 = 2 * r + 1;
-      const int o0 = ((n0 >> 3) * (kKC / 8) + g8) * 128 + (n0 & 7) * 16;
-      const int o1 = ((n1 >> 3) * (kKC / 8) + g8) * 128 + (n1 & 7) * 16;
-      *(uint4 *)(bhi + o0) = *(uint4 *)hr;
-      *(uint4 *)(blo + o0) = *(uint4 *)lr;
-      *(uint4 *)(bhi + o1) = *(uint4 *)hi8;
-      *(uint4 *)(blo + o1) = *(uint4 *)li8;
+    for (int k = 0; k < 4; k++) {
+      split2u(v[2 * k].x * s, v[2 * k + 1].x * s, hr[k], lr[k]);
+      split2u(v[2 * k].y * s, v[2 * k + 1].y * s, hm[k], lm[k]);
     }
+    store_rows(bhi, blo, ((rg >> 2) * (kKC / 8) + g8) * 128 + (rg & 3) * 32, g8 & 1, hr, hm, lr, lm);
+    if (ch + 1 < nch) ring_load8(A, ring, (ch + 1) * kKC + g8 * 8, kw0, v);  // in flight under the MMAs
     fence_proxy_async();
     __syncthreads();
     if (warp == 0) {
-      const bool aok = mbar_wait(abar, ch & 1, A.err, kErrBand);
+      const bool aok = mbar_wait(abar + b, (ch >> 1) & 1, A.err, kErrBand);
       tc_fence_after();
       if (__all_sync(0xffffffffu, aok)) {
-        const uint64_t ah = smem_desc(sbase, 128, (kKC / 8) * 128);
-        const uint64_t al = smem_desc(sbase + kAHalf, 128, (kKC / 8) * 128);
-        const uint64_t bh = smem_desc(sbase + 2 * kAHalf, 128, (kKC / 8) * 128);
-        const uint64_t bl = smem_desc(sbase + 2 * kAHalf + kBHalf, 128, (kKC / 8) * 128);
+        const uint32_t base = sbase + b * kBandBuf;
+        const uint64_t ah = smem_desc(base, 128, (kKC / 8) * 128);
+        const uint64_t al = smem_desc(base + kAHalf, 128, (kKC / 8) * 128);
+        const uint64_t bh = smem_desc(base + 2 * kAHalf, 128, (kKC / 8) * 128);
+        const uint64_t bl = smem_desc(base + 2 * kAHalf + kBHalf, 128, (kKC / 8) * 128);
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < kKC / 16; ks++) {
             const uint32_t k = ks * 256;
-            mma_f16(tmem, desc_add(ah, k), desc_add(bh, k), idesc, (ch | ks) ? 1 : 0);
-            mma_f16(tmem, desc_add(ah, k), desc_add(bl, k), idesc, 1);
+            mma_f16(tmem, desc_add(ah, k), desc_add(bl, k), idesc, (ch | ks) ? 1 : 0);
             mma_f16(tmem, desc_add(al, k), desc_add(bh, k), idesc, 1);
+            mma_f16(tmem, desc_add(ah, k), desc_add(bh, k), idesc, 1);
           }
         }
       }
       __syncwarp();
-      if (elect_one()) mma_commit(mbar);
+      if (elect_one()) mma_commit(mbar + b);
       __syncwarp();
     }
-    ok = mbar_wait(mbar, ch & 1, A.err, kErrBand) && ok;
-    __syncthreads();
   }
+  for (int ch = max(0, nch - 2); ch < nch; ch++) ok = mbar_wait(mbar + (ch & 1), (ch >> 1) & 1, A.err, kErrBand) && ok;
 
   // ---- epilogue ----
   tc_fence_after();
@@ -391,11 +402,7 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_l2l(L2lArgs A) {
             split2u(re0, re1, hr[i], lr[i]);
             split2u(im0, im1, hm[i], lm[i]);
           }
-          const uint32_t o = (uint32_t)cm * 128 + q * 32;
-          st_shared_v4(bhi + o, hr);
-          st_shared_v4(bhi + o + 16, hm);
-          st_shared_v4(blo + o, lr);
-          st_shared_v4(blo + o + 16, lm);
+          store_rows(bhi, blo, (uint32_t)cm * 128 + q * 32, cm & 1, hr, hm, lr, lm);
         }
       }
       fence_proxy_async();
@@ -608,11 +615,7 @@ __global__ void __launch_bounds__(R::threads, 1) k_tc_m2m(M2mArgs A) {
             split2u(z.x * s, z.z * s, hr[i], lr[i]);
             split2u(z.y * s, z.w * s, hm[i], lm[i]);
           }
-          const uint32_t o = (uint32_t)cm * 128 + q * 32;
-          st_shared_v4(bhi + o, hr);
-          st_shared_v4(bhi + o + 16, hm);
-          st_shared_v4(blo + o, lr);
-          st_shared_v4(blo + o + 16, lm);
+          store_rows(bhi, blo, (uint32_t)cm * 128 + q * 32, cm & 1, hr, hm, lr, lm);
         }
       }
       fence_proxy_async();
@@ -917,6 +920,8 @@ static isg_status build_transition(isg_ctx *c, Transition &T, int ns_out, int ns
       len = ns_in - best_gap;
     }
     const bool whole = len >= ns_in - 8;
+    len += start & 3;  // ring_load8 reads quads
+    start &= ~3;
     kw0[mt] = whole ? -1 : start;
     const int span = whole ? ns_in : len;
     nch[mt] = (span + kKC - 1) / kKC;
