@@ -510,9 +510,13 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
 // locals by M2L's, each lowered until both products carry the same power of
 // two.  Two accumulator sets (256 columns each) alternate between
 // items, so an item's epilogue runs under the next item's MMAs.
+// Shared memory bounds the large items: the MMAs read 12 KB for their 128 cycles, and
+// tensor loads, weight stages and converters come on top.  Both operand kinds are
+// written at the halo's pitch of 10 leaves and read in an order that keeps a phase's
+// lanes on different banks: 1024 x 1024 x 64 929 -> 883 us, 256 x 256 x 64 94.1 -> 89.6
+// (L2P stages at a pitch of 8 leaves were 4-way conflicts).
 constexpr int kNpKC = 4;                                       // 8-real K-chunks per A-stage
 constexpr int kNpHaloSplit = kHR * kNpKC * kHC * 16;           // 21760: one FP16 split of a halo K-group
-constexpr int kNpL2pSplit = kPair * kTY * kNpKC * kTX * 16;    // 16384: one FP16 split of an L2P stage
 constexpr int kNpBuf = 2 * kNpHaloSplit;                       // 43520: an operand (hi, lo) or a staged A-stage
 constexpr int kNpHaloBytes = kHR * kHC * 32 * 4;               // 43520: a halo K-group as FP32
 constexpr int kNpL2pBytes = kPair * kTY * kTX * 32 * 4;        // 32768: an L2P stage as FP32
@@ -532,7 +536,7 @@ struct NpSmem {
   static constexpr int total = dscr + 2 * kNpEpiWarps * 3 * 8;
 };
 static_assert(kNpBuf % 128 == 0 && NpSmem::o % 128 == 0, "tensor-load destinations are 128-byte aligned");
-static_assert(kNpHaloBytes <= kNpBuf && kNpL2pBytes <= kNpBuf && 2 * kNpL2pSplit <= kNpBuf, "buffer sizes");
+static_assert(kNpHaloBytes <= kNpBuf && kNpL2pBytes <= kNpBuf, "buffer sizes");
 static_assert(NpSmem::total <= 227 * 1024, "shared memory of one CTA");
 
 // A-stage a of an item: returns 0 (halo K-group a, a < 4) or 1 (L2P stage
@@ -720,9 +724,9 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         int idx;
         const int kind = np_stage(a, A.nl2p, idx);
         const uint32_t obase = sbase + NpSmem::o + i * kNpBuf;
-        const uint32_t lbo = kind == 0 ? kHC * 16 : kTX * 16;  // K-adjacent core matrices
+        constexpr uint32_t lbo = kHC * 16;  // K-adjacent core matrices
         const uint64_t dh0 = smem_desc(obase, lbo, kNpKC * lbo);
-        const uint64_t dl0 = smem_desc(obase + (kind == 0 ? kNpHaloSplit : kNpL2pSplit), lbo, kNpKC * lbo);
+        const uint64_t dl0 = smem_desc(obase + kNpHaloSplit, lbo, kNpKC * lbo);
         const int nq = kind == 0 ? 9 : 1;
         for (int q = 0; q < nq; q++, kb++) {
           const int b = kb % kNpNB;
@@ -769,37 +773,26 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         const bool ok = mbar_wait_or(sfull + i, (ka / kNpNS) & 1, abort, A.err, kErrNp) &&
                         mbar_wait_or(ofree + o, ((ka / kNpNO) & 1) ^ 1, abort, A.err, kErrNp);
         const float4 *st = (const float4 *)(sm + NpSmem::s + i * kNpBuf);
-        char *hi = sm + NpSmem::o + o * kNpBuf;
+        char *hi = sm + NpSmem::o + o * kNpBuf, *lo = hi + kNpHaloSplit;
         int idx;
-        if (np_stage(a, A.nl2p, idx) == 0) {
-          char *lo = hi + kNpHaloSplit;
-          for (int e = ct; e < (TR + 2) * kHC * kNpKC && ok; e += kNpConv) {
-            const int c = e & 3, hc = (e >> 2) % kHC, hr = (e >> 2) / kHC;
-            const float4 a0 = st[2 * e], a1 = st[2 * e + 1];  // staging offset ((hr * 10 + hc) * 32 + 8 c) reals
-            const float si = A.mode == IN_CONJ ? -s1 : s1;    // the imaginary parts' sign
-            uint32_t h[4], l[4];
-            split2u(a0.x * s1, a0.y * si, h[0], l[0]);
-            split2u(a0.z * s1, a0.w * si, h[1], l[1]);
-            split2u(a1.x * s1, a1.y * si, h[2], l[2]);
-            split2u(a1.z * s1, a1.w * si, h[3], l[3]);
-            const int off = ((hr * kNpKC + c) * kHC + hc) * 16;
-            st_shared_v4(hi + off, h);
-            st_shared_v4(lo + off, l);
-          }
-        } else {
-          char *lo = hi + kNpL2pSplit;
-          for (int e = ct; e < TR * kTX * kNpKC && ok; e += kNpConv) {
-            const int c = e & 3, col = (e >> 2) & (kTX - 1), row = e >> 5;
-            const float4 a0 = st[2 * e], a1 = st[2 * e + 1];  // staging offset ((row * 8 + col) * 32 + 8 c) reals
-            uint32_t h[4], l[4];
-            split2u(a0.x * s2, a0.y * s2, h[0], l[0]);
-            split2u(a0.z * s2, a0.w * s2, h[1], l[1]);
-            split2u(a1.x * s2, a1.y * s2, h[2], l[2]);
-            split2u(a1.z * s2, a1.w * s2, h[3], l[3]);
-            const int off = ((row * kNpKC + c) * kTX + col) * 16;
-            st_shared_v4(hi + off, h);
-            st_shared_v4(lo + off, l);
-          }
+        const bool halo = np_stage(a, A.nl2p, idx) == 0;
+        const int cols = halo ? kHC : kTX, units = (halo ? TR + 2 : TR) * cols * kNpKC;
+        const float sr = halo ? s1 : s2, si = halo && A.mode == IN_CONJ ? -s1 : sr;  // the imaginary parts' sign
+        for (int e = ct; e < units && ok; e += kNpConv) {
+          const int c = e & 3, row = halo ? (e >> 2) / kHC : (e >> 2) / kTX, col = (e >> 2) - row * cols;
+          // staging offset ((row * cols + col) * 32 + 8 c) reals; every other leaf reads its
+          // second half first, so that the 8 lanes of a load phase cover all banks
+          const int f = (e >> 2) & 1;
+          const float4 x0 = st[2 * e + f], x1 = st[2 * e + 1 - f];
+          const float4 a0 = f ? x1 : x0, a1 = f ? x0 : x1;
+          uint32_t h[4], l[4];
+          split2u(a0.x * sr, a0.y * si, h[0], l[0]);
+          split2u(a0.z * sr, a0.w * si, h[1], l[1]);
+          split2u(a1.x * sr, a1.y * si, h[2], l[2]);
+          split2u(a1.z * sr, a1.w * si, h[3], l[3]);
+          const int off = ((row * kNpKC + c) * kHC + col) * 16;  // the pitch of 10 leaves keeps the banks apart
+          st_shared_v4(hi + off, h);
+          st_shared_v4(lo + off, l);
         }
         fence_proxy_async();
         named_sync(1, kNpConv);

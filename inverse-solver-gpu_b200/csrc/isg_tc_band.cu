@@ -6,11 +6,10 @@
 // Output samples are tiled by 128 (the MMA M); for each tile the weights are
 // restricted to the circular window of input samples its rows touch (a few
 // dozen more than 128 x the rate ratio), precomputed on the host as FP16 hi/lo
-// K-chunks of 64 in the core-matrix layout and brought in by bulk copies.  The
+// K-chunks of 32 in the core-matrix layout and brought in by bulk copies.  The
 // CTA's 128 MMA columns are 16 parents x 4 children x (re, im) of one level of
 // one or more RHS (64 KB of shared memory and 128 TMEM columns, so three CTAs
-// share an SM: each CTA's load, MMA and epilogue phases run one after another,
-// and the SM overlaps them across CTAs); ring values are split into FP16
+// share an SM); ring values are split into FP16
 // hi/lo after a power-of-two scale per CTA (3 products, FP32 accumulation in
 // TMEM).  The child shift
 // phases are folded into the epilogue (sum over the four children), exactly as
@@ -132,8 +131,8 @@ __device__ __forceinline__ void ring_load8(const BandArgs &A, const RingRef &r, 
 // through two buffers: while the tensor core multiplies one chunk, the next one's
 // weights arrive by a bulk copy and its samples, read a chunk ahead into registers,
 // are split into the other buffer.  (Chunks of 64 through one buffer, every step
-// waiting for the one before: M2M of
-// 1024 x 1024 x 64, all levels, 564 us, this 514; x 16 171 / 155.)
+// waiting for the one before: M2M of 1024 x 1024 x 64, all levels, 564 us, this 514;
+// x 16 171 / 155.)
 __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   extern __shared__ __align__(1024) char sm[];
   uint64_t *abar = (uint64_t *)(sm + 2 * kBandBuf);  // [2] weights landed
