@@ -1034,13 +1034,14 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
 #pragma unroll
       for (int r = 0; r < kP2mPer; r++) {
         const int u = threadIdx.x + r * kP2mConv;
-        const int m = ((u >> 7) << 3) | (u & 7), c = (u >> 3) & 15;
+        const int m = ((u >> 7) << 3) | (u & 7), c = ((u >> 3) & 15) ^ (u & 7);
 #pragma unroll
         for (int p = 0; p < 4; p++) v[r][p] = make_float2(0.f, 0.f);
         if (u < kP2mUnits && leaf0 + m < A.nleaves) {
-          // odd leaves read their two halves in the other order: the 16-byte loads of a
-          // warp then fall on 8 distinct bank groups
-          const int odd = m & 1;
+          // the 8 leaves of a load phase, 512 bytes apart, take 8 different chunks, the
+          // upper four of them their second half first: all banks, no conflict (with one
+          // chunk for all, 4-way: P2M of 1024 x 1024 x 64 258 us, this 237)
+          const int odd = (c >> 2) & 1;
           const float4 x0 = zst[m * 32 + 2 * c + odd], x1 = zst[m * 32 + 2 * c + 1 - odd];
           const float4 a0 = odd ? x1 : x0, a1 = odd ? x0 : x1;
           v[r][0] = make_float2(a0.x, a0.y);
@@ -1067,11 +1068,12 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
         for (int r = 0; r < kP2mPer; r++) {
           const int u = threadIdx.x + r * kP2mConv;
           if (u >= kP2mUnits) continue;
+          const int off = (u >> 7) * 2048 + (((u >> 3) & 15) ^ (u & 7)) * 128 + (u & 7) * 16;
           uint32_t h[4], l[4];
 #pragma unroll
           for (int p = 0; p < 4; p++) split2u(v[r][p].x * s, v[r][p].y * si, h[p], l[p]);
-          st_shared_v4(ahi + u * 16, h);  // u * 16 = (m >> 3) * 2048 + c * 128 + (m & 7) * 16
-          st_shared_v4(alo + u * 16, l);
+          st_shared_v4(ahi + off, h);
+          st_shared_v4(alo + off, l);
         }
       }
       if (threadIdx.x == 0) sval[b] = s;
