@@ -513,7 +513,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16(Args g) {
   const bool rowmajor = g.sCn == 1 && g.mode != 2;
   float *tile = reinterpret_cast<float *>(sm) + warp * (32 * 17);
   for (int c0 = 16 * half; c0 < g.nt; c0 += 32) {
-    __syncwarp();
     float d[16];
     tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)c0, d);
     if (rowmajor) {

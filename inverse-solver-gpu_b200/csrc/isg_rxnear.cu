@@ -362,14 +362,12 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
     for (int w = blockIdx.x; w < A.nitems; w += gridDim.x, it++) {
       const int set = it % nset;
       const bool ok = mbar_wait_or(tfull + set, (it / nset) & 1, abort, A.err, kErrRx);
-      __syncwarp();
       tc_fence_after();
       const int row = (w % A.mt) * 128 + 32 * qd + lane;
       const bool live = ok && row < A.mvalid;
       float2 *out = A.out + (size_t)(w / A.mt) * A.split_stride + (live && A.out_perm ? A.out_perm[row] : row);
       const uint32_t t0 = tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(set * 256);
       for (int j0 = 0; j0 < R; j0 += 16) {
-        __syncwarp();
         float dre[16], dre2[16], dim1[16], dim2[16];
         tmem_ld16(t0 + (uint32_t)j0, dre);
         tmem_ld16(t0 + (uint32_t)(R + j0), dre2);

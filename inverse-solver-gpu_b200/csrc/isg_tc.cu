@@ -61,7 +61,7 @@ __device__ __forceinline__ int loader_id() {
   const int w = threadIdx.x >> 5;
   return w == 0 ? threadIdx.x : threadIdx.x - 32;
 }
-__device__ __forceinline__ void loaders_bar() { asm volatile("bar.sync 1, %0;\n" ::"n"(kLoaders)); }
+__device__ __forceinline__ void loaders_bar() { named_sync(1, kLoaders); }
 
 // max over the loader threads (named barrier 1)
 __device__ float loaders_max(float v, float *scratch) {
@@ -821,7 +821,6 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       np_scales(A, rhs, s1, s2, p);
       const float inv = 1.f / p;
       const bool ok = mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNp);
-      __syncwarp();  // the lanes leave the wait one by one; the TMEM loads are .aligned
       tc_fence_after();
       const size_t rbase = (size_t)rhs * A.U;
       const float *gf = A.g ? (const float *)(A.g + rhs * A.gstride) : nullptr;

@@ -103,9 +103,10 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes
 }
 
 // ---- tcgen05 ----
-// Allocation and release are .aligned: the whole warp executes them together, so
-// the warp converges first (the thread that set up the barriers just before is one
-// of it, and the compiler may otherwise carry its branch on into the allocation).
+// TMEM allocation, release and loads and the named barriers are .aligned: the whole
+// warp executes them together, so each wrapper converges the warp first (lanes leave
+// a wait one by one, a lane may come out of a branch of its own just before, and the
+// compiler may otherwise carry that branch on into the instruction).
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {
   __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(dst_smem)),
@@ -170,6 +171,7 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 // 16 consecutive FP32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
@@ -183,6 +185,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
 // 8 consecutive FP32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
   uint32_t r[8];
+  __syncwarp();
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
@@ -194,6 +197,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
 // 32 consecutive FP32 columns of this thread's TMEM lane (one wait).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
   uint32_t r[32];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
       "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
@@ -246,6 +250,7 @@ constexpr int kPipeThreads = 512;
 
 // Named barrier 1..15 (0 is __syncthreads) over `count` threads.
 __device__ __forceinline__ void named_sync(int id, int count) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
 
