@@ -232,10 +232,10 @@ __global__ void __launch_bounds__(kRxThreads, 1) k_rx_gemm(RxGemmArgs A) {
       int kb0, kb1;
       blocks(w, kb0, kb1);
       const int set = it % nset;
-      ok = mbar_wait_or(tfree + set, ((it / nset) & 1) ^ 1, abort, A.err, kErrRx);
+      const bool ready = mbar_wait_or(tfree + set, ((it / nset) & 1) ^ 1, abort, A.err, kErrRx);
       for (int kb = kb0; kb < kb1; kb++, ka++) {
         const int i = ka % kRxNA, b = ka & 1;
-        ok = __all_sync(0xffffffffu, ok && mbar_wait_or(afull + i, (ka / kRxNA) & 1, abort, A.err, kErrRx) &&
+        ok = __all_sync(0xffffffffu, ready && mbar_wait_or(afull + i, (ka / kRxNA) & 1, abort, A.err, kErrRx) &&
                                          mbar_wait_or(bfull + b, (ka >> 1) & 1, abort, A.err, kErrRx));
         if (!ok) break;
         tc_fence_after();

@@ -710,17 +710,18 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
   } else if (warp == 2) {
     // ---- MMA issue (the warp waits, one elected lane issues): D[128 target
     // reals][8 TR leaves of the item] += weights (A, M = 128) x data (B, N = 8 TR):
-    // each weight stage is 2 K-steps x 3 split products ----
+    // each weight stage is 2 K-steps x 3 split products.  A wait that expires may do so in
+    // some lanes only, so the warp votes once per weight stage and branches on the vote ----
     const uint32_t idesc = idesc_f16_f32(128, kTX * TR), sbase = smem_u32(sm);
     int ka = 0, kb = 0, it = 0;
     bool ok = true;
     for (int w = first; w < A.nitems && ok; w = next_item(w), it++) {
       const int set = it & 1;
       const uint32_t d = tmem + (uint32_t)(set * 256);
-      ok = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNp);
+      bool ready = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNp);
       for (int a = 0; a < na && ok; a++, ka++) {
         const int i = ka % kNpNO;
-        ok = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNp);
+        ready = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNp) && ready;
         int idx;
         const int kind = np_stage(a, A.nl2p, idx);
         const uint32_t obase = sbase + NpSmem::o + i * kNpBuf;
@@ -730,7 +731,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         const int nq = kind == 0 ? 9 : 1;
         for (int q = 0; q < nq; q++, kb++) {
           const int b = kb % kNpNB;
-          ok = __all_sync(0xffffffffu, ok && mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNp));
+          ok = __all_sync(0xffffffffu, mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNp) && ready);
           if (!ok) break;
           tc_fence_after();
           const uint32_t bb = sbase + NpSmem::b + b * kStageBytes;
@@ -820,7 +821,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       float s1, s2, p;
       np_scales(A, rhs, s1, s2, p);
       const float inv = 1.f / p;
-      const bool ok = mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNp);
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNp));
       tc_fence_after();
       const size_t rbase = (size_t)rhs * A.U;
       const float *gf = A.g ? (const float *)(A.g + rhs * A.gstride) : nullptr;

@@ -29,3 +29,45 @@ def test_aligned_instructions_converge_the_warp_first():
                 bad.append(f"{os.path.basename(path)}:{code.count(chr(10), 0, m.start()) + 1}")
     assert found >= 8
     assert not bad, bad
+
+
+def _role(code, at):
+    """The text of the innermost block around `at` that an `if (warp == ...` opens."""
+    depth, start = 0, at
+    while start > 0:
+        start -= 1
+        if code[start] == "}":
+            depth += 1
+        elif code[start] == "{":
+            depth -= 1
+            if depth < 0:
+                head = code[max(code.rfind(c, 0, start) for c in ";{}") + 1:start]
+                if re.search(r"if\s*\(warp == ", head):
+                    break
+                depth = 0
+    depth, end = 0, start
+    while True:
+        depth += {"{": 1, "}": -1}.get(code[end], 0)
+        end += 1
+        if depth == 0:
+            return code[start:end]
+
+
+def test_mma_warps_branch_on_votes():
+    """elect.sync and votes take the whole warp.  A bounded wait can expire in some lanes and
+    not in others, so in a warp that elects a lane no branch or loop depends on a wait's own
+    result, only on a vote over it."""
+    roles, bad = set(), []
+    for path in SOURCES:
+        code = _code(path)
+        for m in re.finditer(r"if \(elect_one\(\)\)", code):
+            role = _role(code, m.start())
+            if role in roles:
+                continue
+            roles.add(role)
+            own = r"\b(?:%s)\b" % "|".join(re.findall(r"(\w+) = mbar_wait(?:_or)?\(", role) + ["mbar_wait_or", "mbar_wait"])
+            voted = re.sub(r"__all_sync\(0xffffffffu, \w+\)", "vote", role)
+            bad += [(os.path.basename(path), head) for head in re.findall(r"(?:if|while) \([^\n]*|for \([^\n]*", voted)
+                    if re.search(own, head)]
+    assert len(roles) == 6
+    assert not bad, bad
