@@ -609,8 +609,8 @@ __global__ void __launch_bounds__(64 * TY, TX == 8 ? 0 : 2) k_near(
     const float2 *__restrict__ dot_a, double *__restrict__ part, int nleaf, int U, int tiles_x, int tiles_total) {
   constexpr int kHalo = (TY + 2) * (TX + 2), kThreads = 64 * TY;
   constexpr int kStages = near_stages(TX), kRows = near_rows(TX);
-  if (inactive(active, blockIdx.y + grid_wait())) return;
-  const int rhs = blockIdx.y;
+  const int rhs = blockIdx.y + grid_wait();
+  if (inactive(active, rhs)) return;
   extern __shared__ __align__(16) float2 sm[];
   float2 *ring = sm;                              // [kStages][kRows][64]
   float2 *hx = ring + kStages * kRows * kBB;      // [kHalo leaves][64]

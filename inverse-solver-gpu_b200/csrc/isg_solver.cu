@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256) k_update_xr(const RhsState *st, const int
                                                    const float2 *__restrict__ p, const float2 *__restrict__ s,
                                                    const float2 *__restrict__ t, int U, double *part, int *count) {
   const int rhs = blockIdx.y + grid_wait();
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *count = 0;  // k_fin_iter counts the active RHS
+  if (blockIdx.x == 0 && rhs == 0 && threadIdx.x == 0) *count = 0;  // k_fin_iter counts the active RHS
   if (inactive(active, rhs)) return;
   const float2 a = f2(ld2(st[rhs].alpha)), o = f2(ld2(st[rhs].omega));
   const size_t base = (size_t)rhs * U;

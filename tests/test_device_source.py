@@ -71,3 +71,22 @@ def test_mma_warps_branch_on_votes():
                     if re.search(own, head)]
     assert len(roles) == 6
     assert not bad, bad
+
+
+def test_waits_for_the_kernel_before_reach_every_index():
+    """Read-only loads may be moved ahead of griddepcontrol.wait unless their address depends
+    on it: the block index that grid_wait()'s zero goes into is not read again without it."""
+    kernels, bad = 0, []
+    for path in SOURCES:
+        code = _code(path)
+        starts = [m.start() for m in re.finditer(r"__global__", code)] + [len(code)]
+        for a, b in zip(starts, starts[1:]):
+            body = code[a:b]
+            if "grid_wait()" not in body:
+                continue
+            kernels += 1
+            index = re.search(r"(blockIdx\.[xyz]) \+ grid_wait\(\)", body)
+            if not index or body.count(index.group(1)) != 1:
+                bad.append((os.path.basename(path), body[body.index("(", 40) - 40:][:60]))
+    assert kernels >= 20
+    assert not bad, bad
