@@ -208,6 +208,9 @@ int near_blocks_per_rhs(const DevPlan &P, int nrhs);
 size_t near_partials(const DevPlan &P, int max_rhs);
 // Samples of a level over all its clusters and a batch.
 int64_t level_outputs(const DevPlan &P, int lvl, int nrhs);
+// Whether launch_l2l takes the tiled kernel (and with it the level's l2l_cols).
+bool l2l_tiled(const DevPlan &P, int lvl, int nrhs);
+constexpr int kL2lCols = 64;  // its columns per block unless tuned
 void launch_near(const DevPlan &P, const NearArgs &A, cudaStream_t st);
 void launch_rx_interp(const DevPlan &P, const float2 *mul, float2 *rx, int nrhs, cudaStream_t st);
 void launch_rx_anterp(const DevPlan &P, const float2 *rx, float2 *loc, int nrhs, float2 scale, cudaStream_t st);

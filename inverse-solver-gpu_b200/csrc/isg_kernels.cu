@@ -932,10 +932,12 @@ void launch_m2l(const DevPlan &P, int lvl, const float2 *mul, float2 *loc, int n
   }
 }
 
+bool l2l_tiled(const DevPlan &P, int lvl, int nrhs) { return level_outputs(P, lvl, nrhs) > kL2lDirect; }
+
 void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *active, cudaStream_t st) {
   const DevLevel &c = P.lv[lvl], &p = P.lv[lvl - 1];
   const int64_t out = level_outputs(P, lvl, nrhs);
-  if (out <= kL2lDirect) {
+  if (!l2l_tiled(P, lvl, nrhs)) {
     const int C = out <= kL2lSingle ? 1 : 4, samples = 4 * p.n * p.n * c.ns / C;
     const DirectArgs D{loc + p.off, loc + c.off, P.mp, p.n, p.ns, c.ns, c.awidth, c.afirst, c.aw,
                        C == 1 ? p.shl : p.shlT, active};
@@ -943,7 +945,7 @@ void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *act
     launch(C == 1 ? k_l2l_direct<1> : k_l2l_direct<4>, dim3((samples + 127) / 128, nrhs), 128, 0, st, D);
     return;
   }
-  const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : 64;
+  const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : kL2lCols;
   const TileArgs A = tile_args(loc, loc, P.mp, p.off, c.off, p.n, p.ns, c.ns, nrhs, c.at, p.shlT, cap, active);
   const TileSmem L(c.at.wmax, A.cols + 1, c.at.out, A.cols, 4 * A.cols, (size_t)4 * c.at.out * (A.cols + 1), true);
   const size_t smem = L.total * sizeof(float2);

@@ -60,6 +60,10 @@ isg_status isg_autotune(isg_ctx *c, int nrhs, int engine, isg_stream stream) {
   }
   for (int i = 3; i < P.L; i++) {  // L2L into level i
     DevLevel &d = P.lv[i];
+    if (!l2l_tiled(P, i, nrhs)) {  // the direct kernel has no columns: larger batches keep the built-in ones
+      d.l2l_cols = kL2lCols;
+      continue;
+    }
     int best = 0;
     float tbest = FLT_MAX;
     for (int cols : {32, 64}) {

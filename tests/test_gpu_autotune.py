@@ -30,3 +30,12 @@ def test_autotune_keeps_the_operator(engine):
     assert np.linalg.norm(after - before) / np.linalg.norm(before) < 1e-5
     info = s.bicgs(torch.zeros_like(x), g, x, tol=1e-5, engine=engine)
     assert all(i["status"] == 0 and 0 <= i["true_residual"] <= 1e-5 for i in info)
+
+
+def test_levels_of_the_direct_l2l_keep_the_built_in_columns():
+    """Up to 600000 outputs a level L2L has no columns per block to choose: a tuned context
+    keeps the built-in 64 for the larger batches that do."""
+    s = isg.Solver(6, numrx=16, max_rhs=8, device=0)
+    s.setup_gpu()
+    for nrhs in (1, 2, 4):
+        assert s.autotune(nrhs, isg.ENGINE_SIMT)["l2l_cols"][3:] == [64, 64, 64]
