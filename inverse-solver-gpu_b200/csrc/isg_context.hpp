@@ -45,7 +45,7 @@ struct isg_ctx {
   float2 *wg = nullptr;                   // [R][U] contrast in blocked order
   float2 *vr = nullptr, *vrt = nullptr, *vp = nullptr, *vv = nullptr, *vs = nullptr, *vt = nullptr;
   float2 *vgx = nullptr;  // [R][U] g times the next matvec's input, written by the update kernels
-  unsigned *levmax = nullptr;  // [R][kLevStride] per-level max |re|, |im| of the multipoles (FP32 bits)
+  unsigned *levmax = nullptr;  // [R][kLevStride] per-level max |re|, |im| of the multipoles; slot kInMaxSlot: the input's
   unsigned *locmax = nullptr;  // levmax + kMaxLevels: the same for the locals (written by M2L)
   double *part = nullptr;  // FP64 partial records [RHS][block][4]
   isg::RhsState *state = nullptr;  // [R]

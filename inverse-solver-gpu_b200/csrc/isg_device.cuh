@@ -9,8 +9,8 @@
 namespace isg {
 
 constexpr int kMaxLevels = 12;
-// Per RHS: the maxima of the multipoles' levels, then of the locals' (FP32 bits).
-constexpr int kLevStride = 2 * kMaxLevels;
+// Per RHS: the maxima of the multipoles' levels, of the locals' and of the input (FP32 bits).
+constexpr int kInMaxSlot = 2 * kMaxLevels, kLevStride = kInMaxSlot + 1;
 constexpr int kBox = 8;
 constexpr int kBB = 64;  // pixels per leaf
 // Kernels put one RHS per grid row (gridDim.y or .z), so no batch may exceed this.
@@ -199,7 +199,7 @@ struct NearArgs {
   double *part = nullptr;         // [R][nblocks][4]
   const float2 *x_epi = nullptr;  // x of the `x - ...` epilogue when in.x already holds g x (else in.x)
   const unsigned *locmax = nullptr;  // tensor engine: per-RHS level maxima of the locals, written by M2L
-  const unsigned *inmax = nullptr;   // tensor engine: [R][kLevStride] whose slot kMaxLevels - 1 holds the input's
+  const unsigned *inmax = nullptr;   // tensor engine: [R][kLevStride] whose slot kInMaxSlot holds the input's
                                      // maximum per RHS, written by the tensor-core P2M of the same matvec
 };
 // FP64 partial records per RHS that launch_near writes for a batch of nrhs, and

@@ -524,7 +524,6 @@ constexpr int kNpNS = 2, kNpNO = 2, kNpNB = 3;                 // staging, opera
 constexpr int kNpConvWarp0 = 3, kNpConvWarps = 4, kNpEpiWarp0 = 7, kNpEpiWarps = 8;
 constexpr int kNpThreads = 32 * (kNpEpiWarp0 + kNpEpiWarps);  // 480
 constexpr int kNpConv = 32 * kNpConvWarps, kNpEpi = 32 * kNpEpiWarps;
-constexpr int kInMaxSlot = kMaxLevels - 1;                     // levmax slot of P2M's input maximum
 constexpr int kErrNp = 121;
 struct NpSmem {
   static constexpr int s = 0;                                  // kNpNS FP32 staging buffers
@@ -1060,7 +1059,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
       for (int k = 0; k < kP2mConvWarps; k++) m2 = fmaxf(m2, fscr[k]);
       const float s = pow2_scale(m2), si = A.conj ? -s : s;
       // the input's maximum per RHS: the near-field kernel's scale for the same input
-      if (threadIdx.x == 0 && fok && m2 > 0.f && A.lvl < kInMaxSlot)
+      if (threadIdx.x == 0 && fok && m2 > 0.f)
         atomicMax(&A.levmax[(w / A.tiles) * kLevStride + kInMaxSlot], __float_as_uint(m2));
       char *ahi = sm + P2mPipeSmem::a(b), *alo = ahi + kP2mA;
       if (fok) {
@@ -1374,7 +1373,7 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
   const TcPlan &T = *c->tc;
   const float2 *loc_leaf = N.loc + P.lv[P.L - 1].off;
   if (N.in.mode == IN_G || !N.inmax || !N.locmax || !T.nearNp || P.ns_leaf % 4 || P.ns_leaf > 4 * kLocChunksMax || P.mp % 2 ||
-      !aligned16(loc_leaf) || P.L - 1 >= kInMaxSlot)
+      !aligned16(loc_leaf))
     return false;
   const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return false;

@@ -31,3 +31,26 @@ def test_large_grid_solves(level):
         print("level", level, "engine", eng, "iterations", [i["iterations"] for i in info])
     d = torch.linalg.vector_norm(xs[isg.ENGINE_TENSOR] - xs[isg.ENGINE_SIMT]) / torch.linalg.vector_norm(xs[isg.ENGINE_SIMT])
     assert d.item() < 1e-4, d.item()
+
+
+def test_operator_on_the_deepest_tree():
+    """16384 x 16384 pixels, 12 levels, the most a context takes: the tensor engine's forward
+    and adjoint operators against the plain engine's (split products of 2^-22 a term against
+    FP32's 2^-24), and a solve of a weak contrast whose inner products come from the near
+    field's records."""
+    import torch
+    s = isg.Solver(12, numrx=8, max_rhs=1, device=0)
+    s.setup_gpu()
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(12)
+    x = torch.complex(*(torch.randn(s.numunk, generator=gen, device="cuda") for _ in range(2)))
+    g = (0.01 * torch.rand(s.numunk, generator=gen, device="cuda")).to(torch.complex64)
+    for herm in (False, True):
+        a = s.matvec(x, g, hermitian=herm, order=isg.ORDER_BLOCKED, engine=isg.ENGINE_TENSOR)
+        b = s.matvec(x, g, hermitian=herm, order=isg.ORDER_BLOCKED)
+        a -= x
+        b -= x
+        assert torch.linalg.norm(a - b) <= 1e-5 * torch.linalg.norm(b)
+    u = torch.zeros_like(x)
+    info = s.bicgs(u, g, x, tol=1e-4, order=isg.ORDER_BLOCKED, engine=isg.ENGINE_TENSOR)
+    assert info[0]["status"] == 0 and info[0]["true_residual"] <= 1e-4, info
