@@ -9,14 +9,12 @@
 // the FP16 range, and summing hi*hi + hi*lo + lo*hi (the lo*lo term is below
 // FP32 rounding).
 //
-// Near-field CTA: a tile of 16 x 8 leaves of one RHS.  Its 18 x 10 halo of
-// leaves is stored once in shared memory in the K-major core-matrix layout
-// [halo row][16-byte K chunk][halo column], so the operand of each of the nine
-// neighbour slots is the same halo seen through a descriptor shifted by one
-// halo row / column.  The weights (9 slots x 128 x 128 reals, then the
-// L2P basis) stream through a 4-deep ring of 16 KB stages filled by bulk
-// async copies.  Warp 1 is the copy producer, thread 0 issues the MMAs, the
-// other warps load and convert operands and all warps run the epilogue.
+// Near-field CTA: 8, 16 or 32 x 8 leaves of one RHS.  Its halo of leaves is stored
+// in shared memory in the K-major core-matrix layout [halo row][16-byte K chunk]
+// [halo column], so the operand of each of the nine neighbour slots is the same
+// halo seen through a descriptor shifted by one halo row / column.  The weights (9
+// slots x 128 x 128 reals, then the L2P basis) stream through a ring of 16 KB stages
+// filled by bulk async copies.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -33,457 +31,15 @@ namespace {
 
 using namespace tc;
 
-constexpr int kTY = 16, kTX = 8;                 // leaves per tile (one 128-row MMA)
-constexpr int kPair = 2;                         // tiles per CTA, stacked in y, sharing every weight stage
-constexpr int kHR = kPair * kTY + 2, kHC = kTX + 2;  // 34 x 10 halo of the pair
-constexpr int kLboA = kHC * 16;                  // 160
-constexpr int kSboA = 16 * kLboA;                // 2560 (one halo row: 16 K-chunks)
-constexpr int kRegion = kHR * kSboA;             // 87040 bytes per FP16 split
+constexpr int kTX = 8, kTRMax = 32;              // leaf columns and most leaf rows of a near-field item
+constexpr int kHR = kTRMax + 2, kHC = kTX + 2;   // its 34 x 10 halo
 constexpr int kStageBytes = 16384;               // hi [128 x 32] + lo [128 x 32]
 constexpr int kStageHalf = 8192;
-constexpr int kNB = 3;                           // ring depth
 constexpr int kNearStages = 36;                  // 9 slots x 4 K-chunks of 32 reals
-constexpr int kLocChunksMax = 20;                // K chunks (8 reals each) of the L2P operand
-constexpr int kSboL = kLocChunksMax * 128;       // 2560
-constexpr int kL2pTile = 16 * kSboL;             // 40960: one tile's L2P operand per split
-constexpr int kLoaders = 224;                    // warps 0, 2..7
-constexpr int kErrNearFull = 101, kErrNearEmpty = 102, kErrNearDone = 103, kErrP2m = 111;
-
-struct NearSmem {
-  static constexpr int hi = 0, lo = kRegion, stages = 2 * kRegion, bars = stages + kNB * kStageBytes;
-  static constexpr int misc = bars + 16 * 8;
-  static constexpr int total = misc + 256;
-};
-static_assert(kPair * kL2pTile <= kRegion, "the L2P operands reuse the halo region");
-static_assert(kPair * 128 * 66 * 8 <= 2 * kRegion, "the epilogue tiles reuse the halo region");
-
-__device__ __forceinline__ int loader_id() {
-  const int w = threadIdx.x >> 5;
-  return w == 0 ? threadIdx.x : threadIdx.x - 32;
-}
-__device__ __forceinline__ void loaders_bar() { named_sync(1, kLoaders); }
-
-// max over the loader threads (named barrier 1)
-__device__ float loaders_max(float v, float *scratch) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) scratch[w] = v;
-  loaders_bar();
-  float m = 0.f;
-  for (int q = 0; q < 8; q++)
-    if (q != 1) m = fmaxf(m, scratch[q]);
-  loaders_bar();
-  return m;
-}
-
+constexpr int kLeafSampMax = 80;                 // samples of a leaf ring
+constexpr int kErrNear = 101, kErrP2m = 111;
 
 __device__ __forceinline__ float cabs1(float2 v) { return fmaxf(fabsf(v.x), fabsf(v.y)); }
-
-// Stores 4 complex values as one 16-byte chunk of hi and one of lo.
-__device__ __forceinline__ void store_chunk(char *smem, int off, const float2 *v, float s) {
-  __align__(16) __half h[8], l[8];
-#pragma unroll
-  for (int p = 0; p < 4; p++) {
-    split_f16(v[p].x * s, h[2 * p], l[2 * p]);
-    split_f16(v[p].y * s, h[2 * p + 1], l[2 * p + 1]);
-  }
-  *(uint4 *)(smem + NearSmem::hi + off) = *(uint4 *)h;
-  *(uint4 *)(smem + NearSmem::lo + off) = *(uint4 *)l;
-}
-
-struct TcNearArgs {
-  const float2 *x, *g;  // operator input (transformed by mode)
-  const float2 *xe;     // x of the `x - ...` epilogue
-  int64_t gstride;
-  int mode;
-  const int *active;
-  const float2 *loc_leaf;  // per-RHS stride mp
-  size_t mp;
-  int ns;
-  const uint8_t *B;  // stages: 36 near + nl2p basis
-  int nl2p;          // L2P stages
-  float inv_w, inv_b;  // 1 / weight scales
-  float2 *y;
-  int epi, red;
-  const float2 *dot_a;
-  double *part;
-  int nleaf, U, tiles_x, tiles;
-  int loc_vec;  // leaf locals can be copied in 16-byte chunks (ns % 4 == 0, aligned)
-  int pair;     // tiles per CTA: kPair, or 1 when the launch is too small to fill the GPU
-  const unsigned *locmax;  // when set: [R][kLevStride] maxima of the locals (written by M2L), the L2P scale
-  int lvl_leaf;
-  int tma_x;    // the halo comes by two tensor loads (map tmx)
-  int tma_loc;  // the leaf locals come by tensor loads (map tml)
-  int *err;
-};
-
-// tmx views the input as [RHS][leaf row][4-pixel chunk][leaf column][8 floats]
-// and tml the leaf locals as [RHS][leaf row][4-sample chunk][leaf column][8
-// floats]: a box of either lands in the staging layout below (first 16 bytes
-// of every chunk in the hi slots, the second 16 in the lo slots).
-__global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_constant__ CUtensorMap tmx,
-                                                    const __grid_constant__ CUtensorMap tml) {
-  extern __shared__ __align__(1024) char sm[];
-  const int rhs = blockIdx.y;
-  if (A.active && !A.active[rhs]) return;
-  uint64_t *full = (uint64_t *)(sm + NearSmem::bars);
-  uint64_t *empty = full + kNB;
-  uint64_t *done = empty + kNB;
-  uint64_t *hbar = done + 1, *lbar = done + 2;  // halo, leaf locals landed
-  uint32_t *tslot = (uint32_t *)(sm + NearSmem::misc);
-  float *fscr = (float *)(sm + NearSmem::misc + 16);      // [8]
-  float *scales = (float *)(sm + NearSmem::misc + 48);    // [2]
-  double *dscr = (double *)(sm + NearSmem::misc + 64);    // [8][3]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pair = blockIdx.x;
-  const int pty = pair / A.tiles_x, ptx = pair % A.tiles_x;
-  const int ty0 = pty * A.pair * kTY, tx0 = ptx * kTX;
-  const int tiles_y = (A.nleaf + kTY - 1) / kTY;
-  const int ntile = min(A.pair, tiles_y - pty * A.pair);
-  const size_t rbase = (size_t)rhs * A.U;
-  const float2 *gr = A.g ? A.g + rhs * A.gstride : nullptr;
-  const int nstages = kNearStages + A.nl2p;
-
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < kNB; b++) {
-      mbar_init(&full[b], 1);
-      mbar_init(&empty[b], 1);
-    }
-    mbar_init(done, 1);
-    mbar_init(hbar, 1);
-    mbar_init(lbar, 1);
-    fence_mbar_init();
-  }
-  if (warp == 0) tmem_alloc(tslot, 512);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tslot;  // near field of tile u in columns [128 u, +128), L2P in [256 + 128 u, +128)
-
-  // ---- halo of the input: every thread stages x as FP32 with cp.async where its
-  // FP16 halves will go (first two pixels of a 4-pixel chunk in the hi slot,
-  // last two in the lo slot); the loaders then take its max (and conjugate) in
-  // place, and convert to hi/lo once the pair's scale is known ----
-  // (halo row, 4-pixel chunk, halo column): consecutive items are consecutive
-  // 16-byte slots, free of bank conflicts
-  const int kItems = (A.pair * kTY + 2) * kHC * 16;
-  if (threadIdx.x == 32) {
-    // the epilogue's x and dot vector rows of the pair, into L2 while the MMAs run
-    const uint32_t run = (uint32_t)min(kTX, A.nleaf - tx0) * kBB * 8;
-    for (int r = 0; r < ntile * kTY; r++) {
-      const int ly = ty0 + r;
-      if (ly >= A.nleaf) break;
-      const size_t at = rbase + (size_t)(ly * A.nleaf + tx0) * kBB;
-      if (A.epi == EPI_FWD || A.epi == EPI_ADJ || A.red == RED_TS) bulk_prefetch_l2(A.xe + at, run);
-      if (A.red == RED_DOT) bulk_prefetch_l2(A.dot_a + at, run);
-    }
-  }
-  if (A.tma_x) {
-    // two tensor loads: pixels 0, 1 of every chunk to the hi slots, 2, 3 to the lo slots
-    if (threadIdx.x == 0) {
-      mbar_expect_tx(hbar, 2 * kItems * 16);
-      tma_load_5d(sm + NearSmem::hi, &tmx, 0, tx0 - 1, 0, ty0 - 1, rhs, hbar);
-      tma_load_5d(sm + NearSmem::lo, &tmx, 4, tx0 - 1, 0, ty0 - 1, rhs, hbar);
-    }
-    mbar_wait(hbar, 0, A.err, kErrNearFull);
-  } else {
-    for (int it = threadIdx.x; it < kItems; it += blockDim.x) {
-      const int hc = it % kHC, c = (it / kHC) & 15, hr = it / (kHC * 16);
-      const int ly = ty0 - 1 + hr, lx = tx0 - 1 + hc;
-      const bool in = ly >= 0 && ly < A.nleaf && lx >= 0 && lx < A.nleaf;
-      const size_t i = in ? (size_t)(ly * A.nleaf + lx) * kBB + 4 * c : 0;
-      const int off = hr * kSboA + c * kLboA + hc * 16;
-      cp_async16z(sm + NearSmem::hi + off, A.x + rbase + i, in);
-      cp_async16z(sm + NearSmem::lo + off, A.x + rbase + i + 2, in);
-    }
-    cp_async_wait_all();
-  }
-  __syncthreads();
-
-  if (warp == 1) {
-    // ---- producer: weight stages through the ring ----
-    if (lane == 0) {
-      for (int t = 0; t < nstages; t++) {
-        const int b = t % kNB;
-        if (t >= kNB && !mbar_wait(&empty[b], ((t / kNB) - 1) & 1, A.err, kErrNearEmpty)) break;
-        mbar_expect_tx(&full[b], kStageBytes);
-        bulk_g2s(sm + NearSmem::stages + b * kStageBytes, A.B + (size_t)t * kStageBytes, kStageBytes, &full[b]);
-      }
-    }
-  } else {
-    const int li = loader_id();
-    float mx = 0.f;
-#pragma unroll 8
-    for (int it = li; it < kItems; it += kLoaders) {
-      const int hc = it % kHC, ck = (it / kHC) & 15, hr = it / (kHC * 16);
-      const int off = hr * kSboA + ck * kLboA + hc * 16;
-      float4 *ph = (float4 *)(sm + NearSmem::hi + off), *pl = (float4 *)(sm + NearSmem::lo + off);
-      const float4 a0 = *ph, a1 = *pl;
-      const float c = A.mode == IN_CONJ ? -1.f : 1.f;
-      const float2 v0 = make_float2(a0.x, c * a0.y), v1 = make_float2(a0.z, c * a0.w);
-      const float2 v2 = make_float2(a1.x, c * a1.y), v3 = make_float2(a1.z, c * a1.w);
-      mx = fmaxf(mx, fmaxf(fmaxf(cabs1(v0), cabs1(v1)), fmaxf(cabs1(v2), cabs1(v3))));
-      *ph = make_float4(v0.x, v0.y, v1.x, v1.y);
-      *pl = make_float4(v2.x, v2.y, v3.x, v3.y);
-    }
-    const float s1 = pow2_scale(loaders_max(mx, fscr));
-    for (int it = li; it < kItems; it += kLoaders) {
-      const int hc = it % kHC, c = (it / kHC) & 15, hr = it / (kHC * 16);
-      const int off = hr * kSboA + c * kLboA + hc * 16;
-      const float4 q0 = *(const float4 *)(sm + NearSmem::hi + off), q1 = *(const float4 *)(sm + NearSmem::lo + off);
-      const float2 v[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
-                           make_float2(q1.z, q1.w)};
-      store_chunk(sm, off, v, s1);
-    }
-    if (li == 0) scales[0] = s1;
-    fence_proxy_async();
-    loaders_bar();
-
-    // ---- MMA issue: every weight stage serves both tiles of the pair ----
-    const uint32_t idesc = idesc_f16_f32(128, 128);
-    const uint32_t sbase = smem_u32(sm);
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      const uint64_t ah0 = smem_desc(sbase + NearSmem::hi, kLboA, kSboA);
-      const uint64_t al0 = smem_desc(sbase + NearSmem::lo, kLboA, kSboA);
-      const uint64_t bh0 = smem_desc(sbase + NearSmem::stages, 128, 512);
-      const uint64_t bl0 = smem_desc(sbase + NearSmem::stages + kStageHalf, 128, 512);
-      for (int t = 0; t < kNearStages; t++) {
-        const int b = t % kNB;
-        if (!mbar_wait(&full[b], (t / kNB) & 1, A.err, kErrNearFull)) break;
-        const int s = t >> 2, c = t & 3, dr = s / 3 - 1, dc = s % 3 - 1;
-#pragma unroll
-        for (int ks = 0; ks < 2; ks++) {
-          const uint32_t boff = b * kStageBytes + ks * 256;
-          for (int u = 0; u < ntile; u++) {
-            const uint32_t aoff = (u * kTY + 1 + dr) * kSboA + (1 + dc) * 16 + (uint32_t)(c * 4 + ks * 2) * kLboA;
-            const uint32_t d = tmem + 128 * u;
-            mma_f16(d, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, (t | ks) ? 1 : 0);
-            mma_f16(d, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, 1);
-            mma_f16(d, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
-          }
-        }
-        mma_commit(&empty[b]);
-      }
-      mma_commit(done);
-    }
-
-    // ---- L2P operands: the tiles' leaf locals, staged with cp.async into the
-    // halo region once the near-field MMAs are done, then scaled and converted ----
-    const int nchunk = (A.ns + 3) / 4;
-    const bool vec_ok = A.loc_vec != 0;
-    const int kL = ntile * 128 * kLocChunksMax;
-    const float2 *lr = A.loc_leaf + (size_t)rhs * A.mp;
-    const bool near_ok = mbar_wait(done, 0, A.err, kErrNearDone);
-    float s2 = 1.f;
-    if (near_ok && A.tma_loc) {
-      // one tensor load per tile and slot: samples 0, 1 of every chunk to hi, 2, 3 to lo
-      if (li == 0) {
-        mbar_expect_tx(lbar, ntile * 2 * kL2pTile);
-        for (int u = 0; u < ntile; u++) {
-          tma_load_5d(sm + NearSmem::hi + u * kL2pTile, &tml, 0, tx0, 0, ty0 + u * kTY, rhs, lbar);
-          tma_load_5d(sm + NearSmem::lo + u * kL2pTile, &tml, 4, tx0, 0, ty0 + u * kTY, rhs, lbar);
-        }
-      }
-      mbar_wait(lbar, 0, A.err, kErrNearFull);
-    }
-    if (near_ok) {
-      for (int it = li; it < kL && !A.tma_loc; it += kLoaders) {
-        // (tile, row group, chunk, row in group): consecutive 16-byte slots
-        const int m7 = it & 7, c = (it >> 3) % kLocChunksMax, mg = (it >> 3) / kLocChunksMax;
-        const int u = mg >> 4, m = ((mg & 15) << 3) | m7;
-        const int ly = ty0 + u * kTY + m / kTX, lx = tx0 + m % kTX;
-        const bool valid = c < nchunk && ly < A.nleaf && lx < A.nleaf;
-        const int off = u * kL2pTile + (m >> 3) * kSboL + c * 128 + (m & 7) * 16;
-        const float2 *src = lr + (valid ? (size_t)(ly * A.nleaf + lx) * A.ns + 4 * c : 0);
-        if (vec_ok) {
-          cp_async16z(sm + NearSmem::hi + off, src, valid);
-          cp_async16z(sm + NearSmem::lo + off, src + 2, valid);
-        } else {
-          float2 v[4];
-#pragma unroll
-          for (int p = 0; p < 4; p++) v[p] = (valid && 4 * c + p < A.ns) ? src[p] : make_float2(0.f, 0.f);
-          *(float4 *)(sm + NearSmem::hi + off) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-          *(float4 *)(sm + NearSmem::lo + off) = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
-        }
-      }
-      cp_async_wait_all();
-      loaders_bar();
-      if (A.locmax) {  // the leaf level's maximum per RHS, from M2L
-        s2 = pow2_scale(__uint_as_float(A.locmax[rhs * kLevStride + A.lvl_leaf]));
-      } else {
-        float mx2 = 0.f;
-        for (int it = li; it < kL; it += kLoaders) {
-          // (tile, row group, chunk, row in group): consecutive 16-byte slots
-          const int m7 = it & 7, c = (it >> 3) % kLocChunksMax, mg = (it >> 3) / kLocChunksMax;
-          const int u = mg >> 4, m = ((mg & 15) << 3) | m7;
-          const int off = u * kL2pTile + (m >> 3) * kSboL + c * 128 + (m & 7) * 16;
-          const float4 q0 = *(const float4 *)(sm + NearSmem::hi + off),
-                       q1 = *(const float4 *)(sm + NearSmem::lo + off);
-          mx2 = fmaxf(mx2, fmaxf(fmaxf(fabsf(q0.x), fabsf(q0.y)), fmaxf(fabsf(q0.z), fabsf(q0.w))));
-          mx2 = fmaxf(mx2, fmaxf(fmaxf(fabsf(q1.x), fabsf(q1.y)), fmaxf(fabsf(q1.z), fabsf(q1.w))));
-        }
-        s2 = pow2_scale(loaders_max(mx2, fscr));
-      }
-      for (int it = li; it < kL; it += kLoaders) {
-        // (tile, row group, chunk, row in group): consecutive 16-byte slots
-        const int m7 = it & 7, c = (it >> 3) % kLocChunksMax, mg = (it >> 3) / kLocChunksMax;
-        const int u = mg >> 4, m = ((mg & 15) << 3) | m7;
-        const int off = u * kL2pTile + (m >> 3) * kSboL + c * 128 + (m & 7) * 16;
-        const float4 q0 = *(const float4 *)(sm + NearSmem::hi + off), q1 = *(const float4 *)(sm + NearSmem::lo + off);
-        const float2 v[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
-                             make_float2(q1.z, q1.w)};
-        store_chunk(sm, off, v, s2);
-      }
-    } else {
-      loaders_bar();  // keeps the named-barrier count of the loaders the same on this path
-      if (!A.locmax) (void)loaders_max(0.f, fscr);
-    }
-    if (li == 0) scales[1] = s2;
-    fence_proxy_async();
-    loaders_bar();
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      const uint64_t ah0 = smem_desc(sbase + NearSmem::hi, 128, kSboL);
-      const uint64_t al0 = smem_desc(sbase + NearSmem::lo, 128, kSboL);
-      const uint64_t bh0 = smem_desc(sbase + NearSmem::stages, 128, 512);
-      const uint64_t bl0 = smem_desc(sbase + NearSmem::stages + kStageHalf, 128, 512);
-      for (int t = kNearStages; t < nstages; t++) {
-        const int b = t % kNB;
-        if (!mbar_wait(&full[b], (t / kNB) & 1, A.err, kErrNearFull)) break;
-        const int c = t - kNearStages;
-#pragma unroll
-        for (int ks = 0; ks < 2; ks++) {
-          const uint32_t boff = b * kStageBytes + ks * 256;
-          for (int u = 0; u < ntile; u++) {
-            const uint32_t aoff = u * kL2pTile + (uint32_t)(c * 4 + ks * 2) * 128;
-            const uint32_t d = tmem + 256 + 128 * u;
-            mma_f16(d, desc_add(ah0, aoff), desc_add(bh0, boff), idesc, (c | ks) ? 1 : 0);
-            mma_f16(d, desc_add(ah0, aoff), desc_add(bl0, boff), idesc, 1);
-            mma_f16(d, desc_add(al0, aoff), desc_add(bh0, boff), idesc, 1);
-          }
-        }
-        mma_commit(&empty[b]);
-      }
-      mma_commit(done);
-    }
-  }
-
-  // ---- epilogue (all warps), in two passes per tile: (1) each thread takes its
-  // leaf's 32 pixels out of TMEM (near field and L2P, scaled back) into a padded
-  // shared tile [leaf][66 float2] in the halo region, free once the L2P MMAs are
-  // done; (2) each warp then takes one leaf at a time, so x, the dot vector and
-  // y move as 512 contiguous bytes per warp access ----
-  constexpr int kOutLd = 66;  // float2 per leaf row: 16-byte aligned rows, 2-way bank spread
-  const int q = warp & 3, hh = warp >> 2;
-  const int m = 32 * q + lane;
-  const bool need_x = A.epi == EPI_FWD || A.epi == EPI_ADJ || A.red == RED_TS;
-  const bool ok = mbar_wait(done, 1, A.err, kErrNearDone);
-  __syncthreads();
-  tc_fence_after();
-  const float inv1 = A.inv_w / scales[0], inv2 = A.inv_b / scales[1];
-  for (int u = 0; u < ntile; u++) {
-    float2 *ot = (float2 *)(sm + NearSmem::hi) + (size_t)u * 128 * kOutLd;
-#pragma unroll
-    for (int ch = 0; ch < 4; ch++) {
-      const int col = 64 * hh + 16 * ch;
-      float d1[16], d2[16];
-      tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + 128 * u + col, d1);
-      tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + 256 + 128 * u + col, d2);
-#pragma unroll
-      for (int p = 0; p < 8; p++)
-        ot[m * kOutLd + col / 2 + p] =
-            make_float2(d1[2 * p] * inv1 + d2[2 * p] * inv2, d1[2 * p + 1] * inv1 + d2[2 * p + 1] * inv2);
-    }
-  }
-  __syncthreads();
-  for (int u = 0; u < ntile; u++) {
-    const float2 *ot = (const float2 *)(sm + NearSmem::hi) + (size_t)u * 128 * kOutLd;
-    double r0 = 0, r1 = 0, r2 = 0;
-    // every load of the tile first (one round trip), then the arithmetic and stores
-    float4 xv[16], av[16];
-    size_t idx[16];
-    bool live[16];
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      const int e = threadIdx.x + 256 * r, lm = e >> 5, pp = e & 31;  // leaf, pixel pair
-      const int ly = ty0 + u * kTY + lm / kTX, lx = tx0 + lm % kTX;
-      live[r] = ok && ly < A.nleaf && lx < A.nleaf;
-      idx[r] = live[r] ? rbase + (size_t)(ly * A.nleaf + lx) * kBB + 2 * pp : rbase;
-      xv[r] = (need_x && live[r]) ? *(const float4 *)(A.xe + idx[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      av[r] = (A.red == RED_DOT && live[r]) ? *(const float4 *)(A.dot_a + idx[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      if (!live[r]) continue;
-      const int e = threadIdx.x + 256 * r, lm = e >> 5, pp = e & 31;
-      const size_t i = idx[r];
-      const float4 ov = *(const float4 *)(ot + lm * kOutLd + 2 * pp);
-      float2 o[2] = {make_float2(ov.x, ov.y), make_float2(ov.z, ov.w)};
-      const float2 xin[2] = {make_float2(xv[r].x, xv[r].y), make_float2(xv[r].z, xv[r].w)};
-      if (A.epi == EPI_FWD) {
-        o[0] = csub(xin[0], o[0]);
-        o[1] = csub(xin[1], o[1]);
-      } else if (A.epi == EPI_ADJ) {
-        const float4 gv = *(const float4 *)(gr + (i - rbase));
-        o[0] = csub(xin[0], cconj(cmul(make_float2(gv.x, gv.y), o[0])));
-        o[1] = csub(xin[1], cconj(cmul(make_float2(gv.z, gv.w), o[1])));
-      } else if (A.epi == EPI_CONJ) {
-        o[0] = cconj(o[0]);
-        o[1] = cconj(o[1]);
-      }
-      *(float4 *)(A.y + i) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
-      if (A.red == RED_DOT) {
-        const float2 a0 = make_float2(av[r].x, av[r].y), a1 = make_float2(av[r].z, av[r].w);
-        r0 += (double)a0.x * o[0].x + (double)a0.y * o[0].y + (double)a1.x * o[1].x + (double)a1.y * o[1].y;
-        r1 += (double)a0.x * o[0].y - (double)a0.y * o[0].x + (double)a1.x * o[1].y - (double)a1.y * o[1].x;
-      } else if (A.red == RED_TS) {
-#pragma unroll
-        for (int e2 = 0; e2 < 2; e2++) {
-          r0 += (double)o[e2].x * xin[e2].x + (double)o[e2].y * xin[e2].y;
-          r1 += (double)o[e2].x * xin[e2].y - (double)o[e2].y * xin[e2].x;
-          r2 += (double)o[e2].x * o[e2].x + (double)o[e2].y * o[e2].y;
-        }
-      }
-    }
-    if (A.red != RED_NONE) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        r0 += __shfl_xor_sync(0xffffffffu, r0, o);
-        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
-        r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-      }
-      if (lane == 0) {
-        dscr[warp * 3 + 0] = r0;
-        dscr[warp * 3 + 1] = r1;
-        dscr[warp * 3 + 2] = r2;
-      }
-    }
-    __syncthreads();
-    if (A.red != RED_NONE && threadIdx.x == 0) {
-      double s0 = 0, s1v = 0, s2v = 0;
-      for (int w2 = 0; w2 < 8; w2++) {
-        s0 += dscr[w2 * 3 + 0];
-        s1v += dscr[w2 * 3 + 1];
-        s2v += dscr[w2 * 3 + 2];
-      }
-      // one record per 8 x 8 leaves: the tile's sum in its first, zero in its second
-      const int rows8 = (A.nleaf + 7) / 8, r0 = (ty0 + u * kTY) / 8;
-      for (int r = r0; r < min(rows8, r0 + kTY / 8); r++) {
-        double *p = A.part + (((size_t)rhs * rows8 + r) * A.tiles_x + ptx) * 4;
-        p[0] = r == r0 ? s0 : 0;
-        p[1] = r == r0 ? s1v : 0;
-        p[2] = r == r0 ? s2v : 0;
-        p[3] = 0;
-      }
-    }
-    __syncthreads();  // dscr is reused by the next tile
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
-}
 
 // ---- near field + L2P, persistent and pipelined ----
 // Items are TR x 8 leaves of one RHS (TR = 32, or 16 or 8 where 32 would leave
@@ -502,7 +58,7 @@ __global__ void __launch_bounds__(256, 1) k_tc_near(TcNearArgs A, const __grid_c
 // weight ring fit in shared memory and the roles overlap:
 //   warp 0      tensor loads of the A-stages (4-D maps, no multicast)
 //   warp 1      bulk copies of the weight stages
-//   warp 2      MMA issue (one thread)
+//   warp 2      MMA issue (one elected lane)
 //   warps 3..6  A-stage conversion to FP16 hi/lo
 //   warps 7..14 epilogue, two per TMEM lane quarter (an item's upper and lower leaf rows)
 // Near field and L2P accumulate into one TMEM accumulator per item: the input
@@ -519,12 +75,11 @@ constexpr int kNpKC = 4;                                       // 8-real K-chunk
 constexpr int kNpHaloSplit = kHR * kNpKC * kHC * 16;           // 21760: one FP16 split of a halo K-group
 constexpr int kNpBuf = 2 * kNpHaloSplit;                       // 43520: an operand (hi, lo) or a staged A-stage
 constexpr int kNpHaloBytes = kHR * kHC * 32 * 4;               // 43520: a halo K-group as FP32
-constexpr int kNpL2pBytes = kPair * kTY * kTX * 32 * 4;        // 32768: an L2P stage as FP32
+constexpr int kNpL2pBytes = kTRMax * kTX * 32 * 4;             // 32768: an L2P stage as FP32
 constexpr int kNpNS = 2, kNpNO = 2, kNpNB = 3;                 // staging, operand buffers, weight ring depth
 constexpr int kNpConvWarp0 = 3, kNpConvWarps = 4, kNpEpiWarp0 = 7, kNpEpiWarps = 8;
 constexpr int kNpThreads = 32 * (kNpEpiWarp0 + kNpEpiWarps);  // 480
 constexpr int kNpConv = 32 * kNpConvWarps, kNpEpi = 32 * kNpEpiWarps;
-constexpr int kErrNp = 121;
 struct NpSmem {
   static constexpr int s = 0;                                  // kNpNS FP32 staging buffers
   static constexpr int o = kNpNS * kNpBuf;                     // kNpNO FP16 hi/lo operand buffers
@@ -543,14 +98,9 @@ static_assert(NpSmem::total <= 227 * 1024, "shared memory of one CTA");
 // rounds each step against the running sum, and interleaving the L2P terms
 // into the near-field sum measured 2x the operator error (5.5e-6 against
 // 2.5e-6 relative to FP64 on random inputs).
-__host__ __device__ inline int np_stage(int a, int nl2p, int &idx) {
-  (void)nl2p;
-  if (a < 4) {
-    idx = a;
-    return 0;
-  }
-  idx = a - 4;
-  return 1;
+__host__ __device__ inline int np_stage(int a, int &idx) {
+  idx = a < 4 ? a : a - 4;
+  return a < 4 ? 0 : 1;
 }
 
 // A dot product's terms over one epilogue chunk at FP32 instruction cost:
@@ -577,7 +127,7 @@ struct Acc32 {
   }
 };
 
-struct TcNearPipeArgs {
+struct TcNearArgs {
   const float2 *x, *g;  // operator input (transformed by mode)
   const float2 *xe;     // x of the `x - ...` epilogue
   int64_t gstride;
@@ -598,7 +148,7 @@ struct TcNearPipeArgs {
 
 // The item's operand scales: input s1 and locals s2 lowered to a common product scale p = s1 sw = s2 sb.
 // A zero maximum (an all-zero input or locals) leaves the other operand's scale alone.
-__device__ __forceinline__ void np_scales(const TcNearPipeArgs &A, int rhs, float &s1, float &s2, float &p) {
+__device__ __forceinline__ void np_scales(const TcNearArgs &A, int rhs, float &s1, float &s2, float &p) {
   const float mx = __uint_as_float(A.levmax[rhs * kLevStride + kInMaxSlot]);
   const float ml = __uint_as_float(A.locmax[rhs * kLevStride + A.lvl_leaf]);
   const float a = mx > 0.f ? pow2_scale(mx) * A.sw : INFINITY;
@@ -610,7 +160,7 @@ __device__ __forceinline__ void np_scales(const TcNearPipeArgs &A, int rhs, floa
 }
 
 template <int TR>
-__global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A, const __grid_constant__ CUtensorMap tmh,
+__global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearArgs A, const __grid_constant__ CUtensorMap tmh,
                                                                 const __grid_constant__ CUtensorMap tml) {
   extern __shared__ __align__(1024) char sm[];
   uint64_t *sfull = (uint64_t *)(sm + NpSmem::bars);  // staging landed / read out
@@ -671,10 +221,10 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         }
         for (int a = 0; a < na; a++, ka++) {
           const int i = ka % kNpNS;
-          if (!mbar_wait_or(sfree + i, ((ka / kNpNS) & 1) ^ 1, abort, A.err, kErrNp)) break;
+          if (!mbar_wait_or(sfree + i, ((ka / kNpNS) & 1) ^ 1, abort, A.err, kErrNear)) break;
           char *dst = sm + NpSmem::s + i * kNpBuf;
           int idx;
-          if (np_stage(a, A.nl2p, idx) == 0) {
+          if (np_stage(a, idx) == 0) {
             mbar_expect_tx(sfull + i, halo_bytes);
             tma_load_4d(dst, &tmh, 32 * idx, tx0 - 1, ty0 - 1, rhs, sfull + i);
           } else {
@@ -686,7 +236,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       // every load issued has landed before the CTA exits (bounded waits)
       for (int j = 1; j <= kNpNS && j <= ka; j++) {
         const int kk = ka - j;
-        mbar_wait(sfull + kk % kNpNS, (kk / kNpNS) & 1, A.err, kErrNp);
+        mbar_wait(sfull + kk % kNpNS, (kk / kNpNS) & 1, A.err, kErrNear);
       }
     }
   } else if (warp == 1) {
@@ -696,14 +246,14 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       for (int w = first; w < A.nitems && !*abort; w = next_item(w)) {
         for (int t = 0; t < nb; t++, kb++) {
           const int b = kb % kNpNB;
-          if (!mbar_wait_or(bempty + b, ((kb / kNpNB) & 1) ^ 1, abort, A.err, kErrNp)) break;
+          if (!mbar_wait_or(bempty + b, ((kb / kNpNB) & 1) ^ 1, abort, A.err, kErrNear)) break;
           mbar_expect_tx(bfull + b, kStageBytes);
           bulk_g2s(sm + NpSmem::b + b * kStageBytes, A.B + (size_t)t * kStageBytes, kStageBytes, bfull + b);
         }
       }
       for (int j = 1; j <= kNpNB && j <= kb; j++) {
         const int kk = kb - j;
-        mbar_wait(bfull + kk % kNpNB, (kk / kNpNB) & 1, A.err, kErrNp);
+        mbar_wait(bfull + kk % kNpNB, (kk / kNpNB) & 1, A.err, kErrNear);
       }
     }
   } else if (warp == 2) {
@@ -717,12 +267,12 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     for (int w = first; w < A.nitems && ok; w = next_item(w), it++) {
       const int set = it & 1;
       const uint32_t d = tmem + (uint32_t)(set * 256);
-      bool ready = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNp);
+      bool ready = mbar_wait_or(tfree + set, ((it >> 1) & 1) ^ 1, abort, A.err, kErrNear);
       for (int a = 0; a < na && ok; a++, ka++) {
         const int i = ka % kNpNO;
-        ready = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNp) && ready;
+        ready = mbar_wait_or(ofull + i, (ka / kNpNO) & 1, abort, A.err, kErrNear) && ready;
         int idx;
-        const int kind = np_stage(a, A.nl2p, idx);
+        const int kind = np_stage(a, idx);
         const uint32_t obase = sbase + NpSmem::o + i * kNpBuf;
         constexpr uint32_t lbo = kHC * 16;  // K-adjacent core matrices
         const uint64_t dh0 = smem_desc(obase, lbo, kNpKC * lbo);
@@ -730,7 +280,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
         const int nq = kind == 0 ? 9 : 1;
         for (int q = 0; q < nq; q++, kb++) {
           const int b = kb % kNpNB;
-          ok = __all_sync(0xffffffffu, mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNp) && ready);
+          ok = __all_sync(0xffffffffu, mbar_wait_or(bfull + b, (kb / kNpNB) & 1, abort, A.err, kErrNear) && ready);
           if (!ok) break;
           tc_fence_after();
           const uint32_t bb = sbase + NpSmem::b + b * kStageBytes;
@@ -758,7 +308,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
     // every MMA issued is complete before the CTA frees TMEM (bounded wait)
     if (elect_one()) mma_commit(mdone);
     __syncwarp();
-    mbar_wait(mdone, 0, A.err, kErrNp);
+    mbar_wait(mdone, 0, A.err, kErrNear);
   } else if (warp < kNpEpiWarp0) {
     // ---- converters: a staged FP32 A-stage becomes the FP16 hi/lo operand.  One
     // unit is a 4-complex chunk (32 bytes) of one leaf: staging [row][col][32 reals]
@@ -770,12 +320,12 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       np_scales(A, w / A.ppr, s1, s2, p);
       for (int a = 0; a < na; a++, ka++) {
         const int i = ka % kNpNS, o = ka % kNpNO;
-        const bool ok = mbar_wait_or(sfull + i, (ka / kNpNS) & 1, abort, A.err, kErrNp) &&
-                        mbar_wait_or(ofree + o, ((ka / kNpNO) & 1) ^ 1, abort, A.err, kErrNp);
+        const bool ok = mbar_wait_or(sfull + i, (ka / kNpNS) & 1, abort, A.err, kErrNear) &&
+                        mbar_wait_or(ofree + o, ((ka / kNpNO) & 1) ^ 1, abort, A.err, kErrNear);
         const float4 *st = (const float4 *)(sm + NpSmem::s + i * kNpBuf);
         char *hi = sm + NpSmem::o + o * kNpBuf, *lo = hi + kNpHaloSplit;
         int idx;
-        const bool halo = np_stage(a, A.nl2p, idx) == 0;
+        const bool halo = np_stage(a, idx) == 0;
         const int cols = halo ? kHC : kTX, units = (halo ? TR + 2 : TR) * cols * kNpKC;
         const float sr = halo ? s1 : s2, si = halo && A.mode == IN_CONJ ? -s1 : sr;  // the imaginary parts' sign
         for (int e = ct; e < units && ok; e += kNpConv) {
@@ -820,7 +370,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearPipeArgs A
       float s1, s2, p;
       np_scales(A, rhs, s1, s2, p);
       const float inv = 1.f / p;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNp));
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNear));
       tc_fence_after();
       const size_t rbase = (size_t)rhs * A.U;
       const float *gf = A.g ? (const float *)(A.g + rhs * A.gstride) : nullptr;
@@ -1202,17 +752,15 @@ void pack_stage(std::vector<uint8_t> &buf, size_t at, int nrows, int k0, double 
 }  // namespace
 
 struct TcPlan {
-  uint8_t *nearB = nullptr;
-  uint8_t *nearNp = nullptr;  // the same stages in the pipelined kernel's A-stage order
+  uint8_t *nearB = nullptr;  // weight stages in the near field's A-stage order
   int nl2p = 0;
-  float inv_w = 1, inv_b = 1;
   float sw = 1, sb = 1;
   uint8_t *p2mB = nullptr;
   int npad = 0, p2m_stage = 0;
   float inv_c = 1;
   int *err = nullptr;
   bool ok = false;
-  int near_pair = 0;  // tiles per near-field CTA picked by isg_autotune (0: built-in choice)
+  int near_pair = 0;  // near-field items picked by isg_autotune: of 16 leaf rows times this at most (0: 32)
 };
 
 bool tc_available(const isg_ctx *c) { return c->tc && c->tc->ok; }
@@ -1226,124 +774,6 @@ int tc_near_pair(const isg_ctx *c) { return tc_available(c) ? c->tc->near_pair :
 int *isg_ctx::tc_err_flag() const { return tc ? tc->err : nullptr; }
 
 namespace isg {
-
-isg_status tc_setup(isg_ctx *c) {
-  int dev = 0, major = 0, minor = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
-  cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
-  const HostTables &T = c->T;
-  const int ns = T.nsamp[T.L - 1];
-  c->tc = new TcPlan();
-  TcPlan &P = *c->tc;
-  if (major != 10 || ns > 4 * kLocChunksMax || T.nleaf < 1) return ISG_OK;  // engine unavailable, SIMT remains
-  // near field: real embedding of near[slot][t][b]; row n = 2t + d, K = 2b + e
-  auto wreal = [&](int s, int n, int k) {
-    const cd w = T.near[((size_t)s * kBB + n / 2) * kBB + k / 2];
-    const int d = n & 1, e = k & 1;
-    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
-  };
-  auto breal = [&](int n, int k) {
-    if (k / 2 >= ns) return 0.0;
-    const cd w = T.basis[(size_t)(n / 2) * ns + k / 2];
-    const int d = n & 1, e = k & 1;
-    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
-  };
-  double mw = 0, mb = 0, mc = 0;
-  for (const cd &v : T.near) mw = std::max(mw, std::max(std::abs(v.real()), std::abs(v.imag())));
-  for (const cd &v : T.basis) mb = std::max(mb, std::max(std::abs(v.real()), std::abs(v.imag())));
-  for (const cd &v : T.coeff) mc = std::max(mc, std::max(std::abs(v.real()), std::abs(v.imag())));
-  const double sw = pow2_scale_host(mw), sb = pow2_scale_host(mb), sc = pow2_scale_host(mc);
-  const int kl = ((2 * ns + 31) / 32) * 32;  // L2P K padded to whole stages
-  P.nl2p = kl / 32;
-  std::vector<uint8_t> nb((size_t)(kNearStages + P.nl2p) * kStageBytes, 0);
-  for (int t = 0; t < kNearStages; t++)
-    pack_stage(nb, (size_t)t * kStageBytes, 128, (t & 3) * 32, sw, [&](int n, int k) { return wreal(t >> 2, n, k); });
-  for (int c2 = 0; c2 < P.nl2p; c2++)
-    pack_stage(nb, (size_t)(kNearStages + c2) * kStageBytes, 128, c2 * 32, sb, breal);
-  P.inv_w = (float)(1.0 / sw);
-  P.inv_b = (float)(1.0 / sb);
-  P.sw = (float)sw;
-  P.sb = (float)sb;
-  // pipelined kernel: per A-stage, a halo K-group's nine slots or one L2P stage
-  std::vector<uint8_t> np((size_t)(kNearStages + P.nl2p) * kStageBytes, 0);
-  {
-    size_t t = 0;
-    for (int a = 0; a < 4 + P.nl2p; a++) {
-      int idx;
-      if (np_stage(a, P.nl2p, idx) == 0) {
-        for (int q = 0; q < 9; q++, t++)
-          pack_stage(np, t * kStageBytes, 128, idx * 32, sw, [&](int n, int k) { return wreal(q, n, k); });
-      } else {
-        pack_stage(np, (t++) * kStageBytes, 128, idx * 32, sb, breal);
-      }
-    }
-  }
-  // P2M: row n = 2k + d over samples (padded to a multiple of 16), K = 2 pixel + e
-  P.npad = ((2 * ns + 15) / 16) * 16;
-  P.p2m_stage = P.npad * 32 * 2 * 2;
-  auto creal = [&](int n, int k) {
-    if (n / 2 >= ns) return 0.0;
-    const cd w = T.coeff[(size_t)(n / 2) * kBB + k / 2];
-    const int d = n & 1, e = k & 1;
-    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
-  };
-  std::vector<uint8_t> pb((size_t)4 * P.p2m_stage, 0);
-  for (int c2 = 0; c2 < 4; c2++) pack_stage(pb, (size_t)c2 * P.p2m_stage, P.npad, c2 * 32, sc, creal);
-  P.inv_c = (float)(1.0 / sc);
-  isg_status e;
-  if ((e = cuda_check(c, cudaMalloc(&P.nearB, nb.size()), "tc alloc")) != ISG_OK) return e;
-  if ((e = cuda_check(c, cudaMalloc(&P.nearNp, np.size()), "tc alloc")) != ISG_OK) return e;
-  if ((e = cuda_check(c, cudaMalloc(&P.p2mB, pb.size()), "tc alloc")) != ISG_OK) return e;
-  if ((e = cuda_check(c, cudaMalloc(&P.err, sizeof(int)), "tc alloc")) != ISG_OK) return e;
-  cudaMemcpy(P.nearB, nb.data(), nb.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(P.nearNp, np.data(), np.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(P.p2mB, pb.data(), pb.size(), cudaMemcpyHostToDevice);
-  cudaMemset(P.err, 0, sizeof(int));
-  cudaFuncSetAttribute(k_tc_near, cudaFuncAttributeMaxDynamicSharedMemorySize, NearSmem::total);
-  for (auto k : {k_tc_near_pipe<8>, k_tc_near_pipe<16>, k_tc_near_pipe<32>})
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, NpSmem::total);
-  cudaFuncSetAttribute(k_tc_p2m_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)P2mPipeSmem::total(P.p2m_stage));
-  if ((e = cuda_check(c, cudaGetLastError(), "tc setup")) != ISG_OK) return e;
-  P.ok = true;
-  return ISG_OK;
-}
-
-void tc_destroy(isg_ctx *c) {
-  if (!c->tc) return;
-  cudaFree(c->tc->nearB);
-  cudaFree(c->tc->nearNp);
-  cudaFree(c->tc->p2mB);
-  cudaFree(c->tc->err);
-  delete c->tc;
-  c->tc = nullptr;
-}
-
-int tc_near_blocks(const isg_ctx *c) {
-  const int n8 = (c->P.nleaf + 7) / 8;
-  return n8 * n8;
-}
-
-// Leaf rows per item of the pipelined near field: 32 (the most MMA columns, so
-// each weight stage serves 256 leaves), unless 16 or 8 rows still give every
-// item an SM of its own or the grid is no higher than that: the launch is then
-// as long as one item, whose time falls with its rows.
-static int np_rows(const DevPlan &P, int nrhs, int sms) {
-  const int cols = (P.nleaf + kTX - 1) / kTX;
-  for (int tr : {8, 16})
-    if (tr >= P.nleaf || (int64_t)cols * ((P.nleaf + tr - 1) / tr) * nrhs <= sms) return tr;
-  return 32;
-}
-
-int tc_error(isg_ctx *c) {
-  if (!tc_available(c)) return 0;
-  int h = 0;
-  cudaMemcpy(&h, c->tc->err, sizeof(int), cudaMemcpyDeviceToHost);
-  return h;
-}
-
-static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry-point query, so
 // that the library does not link the driver library (it still loads where
@@ -1363,28 +793,140 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// The pipelined near-field kernel; returns false (launching nothing) when the
-// call does not meet its conditions: the input plain or conjugated (not still
-// without its contrast), P2M's input maximum known (N.inmax), leaf
-// rings of a multiple of 4 samples (<= 80), 16-byte aligned vectors and both
-// tensor maps encoded.
-static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_status *e) {
+isg_status tc_setup(isg_ctx *c) {
+  int dev = 0, major = 0, minor = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+  cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
+  const HostTables &T = c->T;
+  const int ns = T.nsamp[T.L - 1];
+  c->tc = new TcPlan();
+  TcPlan &P = *c->tc;
+  if (major != 10 || ns > kLeafSampMax || !tensor_map_encoder()) return ISG_OK;  // engine unavailable, SIMT remains
+  // near field: real embedding of near[slot][t][b]; row n = 2t + d, K = 2b + e
+  auto wreal = [&](int s, int n, int k) {
+    const cd w = T.near[((size_t)s * kBB + n / 2) * kBB + k / 2];
+    const int d = n & 1, e = k & 1;
+    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
+  };
+  auto breal = [&](int n, int k) {
+    if (k / 2 >= ns) return 0.0;
+    const cd w = T.basis[(size_t)(n / 2) * ns + k / 2];
+    const int d = n & 1, e = k & 1;
+    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
+  };
+  double mw = 0, mb = 0, mc = 0;
+  for (const cd &v : T.near) mw = std::max(mw, std::max(std::abs(v.real()), std::abs(v.imag())));
+  for (const cd &v : T.basis) mb = std::max(mb, std::max(std::abs(v.real()), std::abs(v.imag())));
+  for (const cd &v : T.coeff) mc = std::max(mc, std::max(std::abs(v.real()), std::abs(v.imag())));
+  const double sw = pow2_scale_host(mw), sb = pow2_scale_host(mb), sc = pow2_scale_host(mc);
+  const int kl = ((2 * ns + 31) / 32) * 32;  // L2P K padded to whole stages
+  P.nl2p = kl / 32;
+  P.sw = (float)sw;
+  P.sb = (float)sb;
+  // near field: per A-stage, a halo K-group's nine slots or one L2P stage
+  std::vector<uint8_t> nb((size_t)(kNearStages + P.nl2p) * kStageBytes, 0);
+  {
+    size_t t = 0;
+    for (int a = 0; a < 4 + P.nl2p; a++) {
+      int idx;
+      if (np_stage(a, idx) == 0) {
+        for (int q = 0; q < 9; q++, t++)
+          pack_stage(nb, t * kStageBytes, 128, idx * 32, sw, [&](int n, int k) { return wreal(q, n, k); });
+      } else {
+        pack_stage(nb, (t++) * kStageBytes, 128, idx * 32, sb, breal);
+      }
+    }
+  }
+  // P2M: row n = 2k + d over samples (padded to a multiple of 16), K = 2 pixel + e
+  P.npad = ((2 * ns + 15) / 16) * 16;
+  P.p2m_stage = P.npad * 32 * 2 * 2;
+  auto creal = [&](int n, int k) {
+    if (n / 2 >= ns) return 0.0;
+    const cd w = T.coeff[(size_t)(n / 2) * kBB + k / 2];
+    const int d = n & 1, e = k & 1;
+    return d == 0 ? (e == 0 ? w.real() : -w.imag()) : (e == 0 ? w.imag() : w.real());
+  };
+  std::vector<uint8_t> pb((size_t)4 * P.p2m_stage, 0);
+  for (int c2 = 0; c2 < 4; c2++) pack_stage(pb, (size_t)c2 * P.p2m_stage, P.npad, c2 * 32, sc, creal);
+  P.inv_c = (float)(1.0 / sc);
+  isg_status e;
+  if ((e = cuda_check(c, cudaMalloc(&P.nearB, nb.size()), "tc alloc")) != ISG_OK) return e;
+  if ((e = cuda_check(c, cudaMalloc(&P.p2mB, pb.size()), "tc alloc")) != ISG_OK) return e;
+  if ((e = cuda_check(c, cudaMalloc(&P.err, sizeof(int)), "tc alloc")) != ISG_OK) return e;
+  cudaMemcpy(P.nearB, nb.data(), nb.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(P.p2mB, pb.data(), pb.size(), cudaMemcpyHostToDevice);
+  cudaMemset(P.err, 0, sizeof(int));
+  for (auto k : {k_tc_near_pipe<8>, k_tc_near_pipe<16>, k_tc_near_pipe<32>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, NpSmem::total);
+  cudaFuncSetAttribute(k_tc_p2m_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)P2mPipeSmem::total(P.p2m_stage));
+  if ((e = cuda_check(c, cudaGetLastError(), "tc setup")) != ISG_OK) return e;
+  P.ok = true;
+  return ISG_OK;
+}
+
+void tc_destroy(isg_ctx *c) {
+  if (!c->tc) return;
+  cudaFree(c->tc->nearB);
+  cudaFree(c->tc->p2mB);
+  cudaFree(c->tc->err);
+  delete c->tc;
+  c->tc = nullptr;
+}
+
+int tc_near_blocks(const isg_ctx *c) {
+  const int n8 = (c->P.nleaf + 7) / 8;
+  return n8 * n8;
+}
+
+// Leaf rows per item of the pipelined near field: 32 (the most MMA columns, so
+// each weight stage serves 256 leaves), unless 16 or 8 rows still give every
+// item an SM of its own or the grid is no higher than that: the launch is then
+// as long as one item, whose time falls with its rows.
+static int np_rows(const DevPlan &P, int nrhs, int sms, int cap) {
+  const int cols = (P.nleaf + kTX - 1) / kTX;
+  for (int tr : {8, 16})
+    if (tr >= cap || tr >= P.nleaf || (int64_t)cols * ((P.nleaf + tr - 1) / tr) * nrhs <= sms) return tr;
+  return kTRMax;
+}
+
+int tc_error(isg_ctx *c) {
+  if (!tc_available(c)) return 0;
+  int h = 0;
+  cudaMemcpy(&h, c->tc->err, sizeof(int), cudaMemcpyDeviceToHost);
+  return h;
+}
+
+static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
+
+static int device_sms(const isg_ctx *c) {
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
+  return sms;
+}
+
+bool tc_near_tall(const isg_ctx *c, int nrhs) { return np_rows(c->P, nrhs, device_sms(c), kTRMax) == kTRMax; }
+
+// The input is plain or conjugated (callers form g x first, run_matvec); its
+// maximum and the locals' are known (P2M and M2L of the same matvec).  Leaf rings are
+// multiples of 4 samples, so every row that the tensor maps address is 16-byte aligned.
+isg_status tc_near(isg_ctx *c, const NearArgs &N, cudaStream_t st) {
   const DevPlan &P = c->P;
   const TcPlan &T = *c->tc;
   const float2 *loc_leaf = N.loc + P.lv[P.L - 1].off;
-  if (N.in.mode == IN_G || !N.inmax || !N.locmax || !T.nearNp || P.ns_leaf % 4 || P.ns_leaf > 4 * kLocChunksMax || P.mp % 2 ||
-      !aligned16(loc_leaf))
-    return false;
-  const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-  if (!encode) return false;
-  TcNearPipeArgs A;
+  if (!aligned16(N.in.x) || (N.x_epi && !aligned16(N.x_epi)) || (N.in.g && !aligned16(N.in.g)) || !aligned16(N.y) ||
+      (N.dot_a && !aligned16(N.dot_a)) || (N.in.gstride % 2) || N.epi == EPI_L2P_ONLY || N.in.mode == IN_G ||
+      !N.inmax || !N.locmax)
+    return ISG_UNSUPPORTED;
+  TcNearArgs A;
   A.x = N.in.x;
   A.xe = N.x_epi ? N.x_epi : N.in.x;
   A.g = N.in.g;
   A.gstride = N.in.gstride;
   A.mode = N.in.mode;
   A.active = N.in.active;
-  A.B = T.nearNp;
+  A.B = T.nearB;
   A.nl2p = T.nl2p;
   A.sw = T.sw;
   A.sb = T.sb;
@@ -1398,9 +940,9 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
   A.part = N.part;
   A.nleaf = P.nleaf;
   A.U = P.U;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
-  const int tr = np_rows(P, N.in.nrhs, sms);
+  const int sms = device_sms(c);
+  const bool tuned = T.near_pair > 0 && 4 * N.in.nrhs >= P.tuned_nrhs;
+  const int tr = np_rows(P, N.in.nrhs, sms, tuned ? 16 * T.near_pair : kTRMax);
   A.tiles_x = (P.nleaf + kTX - 1) / kTX;
   A.ppr = A.tiles_x * ((P.nleaf + tr - 1) / tr);
   A.nitems = A.ppr * N.in.nrhs;
@@ -1419,92 +961,19 @@ static bool tc_near_pipe(isg_ctx *c, const NearArgs &N, cudaStream_t st, isg_sta
                             (cuuint64_t)N.in.nrhs};
   const cuuint64_t ls[3] = {(cuuint64_t)P.ns_leaf * 8, (cuuint64_t)P.nleaf * P.ns_leaf * 8, (cuuint64_t)P.mp * 8};
   const cuuint32_t lb[4] = {32, (cuuint32_t)kTX, (cuuint32_t)tr, 1};
+  const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (encode(&tmh, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)A.x, hd, hs, hb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
       encode(&tml, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)loc_leaf, ld, ls, lb, one,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+    c->err = "near field: a tensor map was refused";
+    return ISG_CUDA_ERROR;
+  }
   count_launch();
   launch(tr == 32 ? k_tc_near_pipe<32> : tr == 16 ? k_tc_near_pipe<16> : k_tc_near_pipe<8>, std::min(A.nitems, sms),
          kNpThreads, NpSmem::total, st, A, tmh, tml);
-  *e = cuda_check(c, cudaGetLastError(), "tc near launch");
-  return true;
-}
-
-isg_status tc_near(isg_ctx *c, const NearArgs &N, cudaStream_t st) {
-  const DevPlan &P = c->P;
-  const TcPlan &T = *c->tc;
-  if (!aligned16(N.in.x) || (N.x_epi && !aligned16(N.x_epi)) || (N.in.g && !aligned16(N.in.g)) || !aligned16(N.y) ||
-      (N.dot_a && !aligned16(N.dot_a)) ||
-      (N.in.gstride % 2) || N.epi == EPI_L2P_ONLY)
-    return ISG_UNSUPPORTED;
-  isg_status pe = ISG_OK;
-  if (tc_near_pipe(c, N, st, &pe)) return pe;
-  TcNearArgs A;
-  A.x = N.in.x;
-  A.xe = N.x_epi ? N.x_epi : N.in.x;
-  A.g = N.in.g;
-  A.gstride = N.in.gstride;
-  A.mode = N.in.mode;
-  A.active = N.in.active;
-  A.loc_leaf = N.loc + P.lv[P.L - 1].off;
-  A.mp = P.mp;
-  A.ns = P.ns_leaf;
-  A.B = T.nearB;
-  A.nl2p = T.nl2p;
-  A.inv_w = T.inv_w;
-  A.inv_b = T.inv_b;
-  A.y = N.y;
-  A.epi = N.epi;
-  A.red = N.red;
-  A.dot_a = N.dot_a;
-  A.part = N.part;
-  A.nleaf = P.nleaf;
-  A.U = P.U;
-  A.tiles_x = (P.nleaf + kTX - 1) / kTX;
-  const int tiles_y = (P.nleaf + kTY - 1) / kTY;
-  A.tiles = A.tiles_x * tiles_y;
-  A.loc_vec = (P.ns_leaf % 4 == 0) && aligned16(A.loc_leaf) && (P.mp % 2 == 0);
-  A.err = T.err;
-  A.locmax = N.locmax;
-  A.lvl_leaf = P.L - 1;
-  count_launch();
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->opts.device);
-  A.pair = (A.tiles * N.in.nrhs >= 2 * kPair * sms) ? kPair : 1;
-  if (T.near_pair > 0 && 4 * N.in.nrhs >= P.tuned_nrhs) A.pair = std::min(T.near_pair, kPair);
-  const int pairs = A.tiles_x * ((tiles_y + A.pair - 1) / A.pair);
-  // tensor maps (see k_tc_near); a map that does not encode keeps its 16-byte copies
-  CUtensorMap tmx, tml;
-  memset(&tmx, 0, sizeof(tmx));
-  memset(&tml, 0, sizeof(tml));
-  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-  const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-  A.tma_x = 0;
-  if (encode) {
-    const cuuint64_t dims[5] = {8, (cuuint64_t)P.nleaf, 16, (cuuint64_t)P.nleaf, (cuuint64_t)N.in.nrhs};
-    const cuuint64_t strides[4] = {(cuuint64_t)kBB * 8, 32, (cuuint64_t)P.nleaf * kBB * 8, (cuuint64_t)P.U * 8};
-    const cuuint32_t box[5] = {4, (cuuint32_t)kHC, 16, (cuuint32_t)(A.pair * kTY + 2), 1};
-    A.tma_x = encode(&tmx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, (void *)A.x, dims, strides, box, one,
-                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                     CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  }
-  A.tma_loc = 0;
-  if (A.loc_vec && encode) {
-    const cuuint64_t dims[5] = {8, (cuuint64_t)P.nleaf, (cuuint64_t)(P.ns_leaf / 4), (cuuint64_t)P.nleaf,
-                                (cuuint64_t)N.in.nrhs};
-    const cuuint64_t strides[4] = {(cuuint64_t)P.ns_leaf * 8, 32, (cuuint64_t)P.nleaf * P.ns_leaf * 8,
-                                   (cuuint64_t)P.mp * 8};
-    const cuuint32_t box[5] = {4, (cuuint32_t)kTX, (cuuint32_t)kLocChunksMax, (cuuint32_t)kTY, 1};
-    A.tma_loc = P.ns_leaf / 4 <= kLocChunksMax &&
-                encode(&tml, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, (void *)A.loc_leaf, dims, strides,
-                                       box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                       CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  }
-  k_tc_near<<<dim3(pairs, N.in.nrhs), 256, NearSmem::total, st>>>(A, tmx, tml);
   return cuda_check(c, cudaGetLastError(), "tc near launch");
 }
 

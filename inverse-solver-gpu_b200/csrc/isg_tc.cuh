@@ -56,12 +56,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// 16-byte asynchronous global -> shared copy; zero-fills when !valid.
-__device__ __forceinline__ void cp_async16z(void *smem, const void *gmem, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem),
-               "r"(valid ? 16 : 0));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
 
@@ -71,18 +65,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                    smem_u32(dst)),
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
-}
-
-// Tiled 5-D tensor load global -> shared (no multicast), completion counted on
-// an mbarrier.  c0 is the innermost coordinate; it must address a 16-byte
-// boundary.  Coordinates outside the tensor read as zero.
-__device__ __forceinline__ void tma_load_5d(void *dst, const void *tmap, int c0, int c1, int c2, int c3, int c4,
-                                            uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
-      "[%7];\n" ::"r"(smem_u32(dst)),
-      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
-      : "memory");
 }
 
 // Tiled 4-D tensor load global -> shared (no multicast); c0 (innermost) must
@@ -246,8 +228,6 @@ __device__ __forceinline__ void st_shared_v4(void *p, const uint32_t (&v)[4]) {
                : "memory");
 }
 
-constexpr int kPipeThreads = 512;
-
 // Named barrier 1..15 (0 is __syncthreads) over `count` threads.
 __device__ __forceinline__ void named_sync(int id, int count) {
   __syncwarp();
@@ -273,13 +253,6 @@ struct PipeRoles {
   static constexpr int conv_warps = CONV, mma_warp = CONV, epi_warp0 = CONV + 1;
   static constexpr int threads = 32 * (CONV + 1 + EPI), conv = 32 * CONV, epi = 32 * EPI, epi_groups = EPI / 4;
 };
-
-constexpr int kPipeConvWarps = 11;  // warps 0..10
-constexpr int kPipeMmaWarp = 11;    // warp 11
-constexpr int kPipeEpiWarp0 = 12;   // warps 12..15, one per TMEM lane quarter
-constexpr int kPipeConv = 32 * kPipeConvWarps;
-constexpr int kPipeEpi = kPipeThreads - 32 * kPipeEpiWarp0;
-constexpr int kPipeEpiGroups = kPipeEpi / 128;  // column groups of the accumulator
 
 // Barrier slots: A, zfull[2], bfull[2], bfree[2], tfull[2], tfree[2]; then
 // the TMEM base and the abort flag.

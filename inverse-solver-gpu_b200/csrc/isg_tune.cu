@@ -2,8 +2,8 @@
 // kernels on this context's own buffers and keeps the fastest per level.
 //   M2L   sibling-group rows per thread          1, 2, 4, ..., 64
 //   L2L   columns (RHS x parent) per tile block  32, 64
-//   M2M   columns per tile block (SIMT path)     32, 64
-//   near  16x8-leaf tiles per tensor-core CTA    1, 2
+//   M2M   columns per block (SIMT path)          32, 64
+//   near  16-row halves of a near-field item (tensor engine)  1, 2
 // Every candidate computes the same outputs in the same order per output, so
 // the choice changes only the time.  The shapes apply to launches of at least
 // a quarter of the tuned batch; smaller batches keep the built-in choices.
@@ -94,12 +94,17 @@ isg_status isg_autotune(isg_ctx *c, int nrhs, int engine, isg_stream stream) {
     A.epi = EPI_G;
     A.red = RED_NONE;
     A.part = c->part;
-    int best = 0;
+    A.inmax = c->levmax;
+    A.locmax = c->locmax;
+    int best = 2;
     float tbest = FLT_MAX;
-    for (int pair : {1, 2}) {
-      tc_set_near_pair(c, pair);
-      const float t = time_launch(st, e0, e1, [&] { tc_near(c, A, st); });
-      if (t < tbest) tbest = t, best = pair;
+    tc_set_near_pair(c, 0);
+    if (tc_near_tall(c, nrhs)) {  // smaller launches take 16 or 8 rows whatever the choice
+      for (int pair : {2, 1}) {
+        tc_set_near_pair(c, pair);
+        const float t = time_launch(st, e0, e1, [&] { tc_near(c, A, st); });
+        if (t < tbest) tbest = t, best = pair;
+      }
     }
     tc_set_near_pair(c, best);
   }

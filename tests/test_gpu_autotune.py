@@ -1,7 +1,6 @@
 """The launch-shape autotuner: it picks one of the candidate shapes per level,
-and the operator's output does not depend on the choice (same complex64
-kernels, per-output order unchanged; 1e-5 relative for the tensor engine,
-whose per-CTA FP16 scale depends on how many tiles a CTA holds)."""
+and the operator's output does not depend on the choice (the same terms of every
+output in the same order)."""
 import numpy as np
 import pytest
 
@@ -39,3 +38,18 @@ def test_levels_of_the_direct_l2l_keep_the_built_in_columns():
     s.setup_gpu()
     for nrhs in (1, 2, 4):
         assert s.autotune(nrhs, isg.ENGINE_SIMT)["l2l_cols"][3:] == [64, 64, 64]
+
+
+def test_tuned_near_field_items_apply_to_the_operator():
+    """The tuner times the near-field kernel that the operator launches: where the launch's
+    items are small in any case the choice stays 2, and tuning leaves every bit alone."""
+    import torch
+    s = isg.Solver(7, numrx=16, max_rhs=12, device=0)
+    s.setup_gpu()
+    x = torch.randn(12, s.numunk, dtype=torch.complex64, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    g = torch.full((s.numunk,), 0.3, dtype=torch.complex64, device="cuda")
+    before = s.matvec(x, g, engine=isg.ENGINE_TENSOR)
+    for nrhs in (1, 2, 4):  # 64 and 128 items of 8 rows, 128 of 16: one per SM
+        assert s.autotune(nrhs, isg.ENGINE_TENSOR)["near_pair"] == 2
+    s.autotune(12, isg.ENGINE_TENSOR)
+    assert torch.equal(s.matvec(x, g, engine=isg.ENGINE_TENSOR), before)
