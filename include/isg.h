@@ -265,8 +265,8 @@ isg_status isg_dbim(isg_ctx *ctx, int ntx, const void *inc, const void *mes, con
 /* ---- measurement ---- */
 /* Number of CUDA kernels this library has launched in the process so far. */
 int64_t isg_kernel_launches(void);
-/* Runs the forward matvec `reps` times on nrhs internal test vectors and writes
- * the mean device time in ms of each stage: [0] P2M, [1] M2M (all levels),
+/* Runs the forward matvec `reps` times on nrhs random internal test vectors and
+ * writes the mean device time in ms of each stage: [0] P2M, [1] M2M (all levels),
  * [2] M2L+L2L (all levels), [3] L2P+near field, [4] whole matvec. */
 isg_status isg_time_stages(isg_ctx *ctx, int nrhs, int engine, int reps, double *ms_out);
 

@@ -677,34 +677,38 @@ isg_status isg_time_stages(isg_ctx *c, int nrhs, int engine, int reps, double *m
   cudaStream_t st = c->stream;
   const DevPlan &P = c->P;
   const size_t n = (size_t)nrhs * P.U;
-  cudaMemsetAsync(c->wx, 0, n * sizeof(float2), st);
-  cudaMemsetAsync(c->wg, 0, (size_t)P.U * sizeof(float2), st);
+  // the buffers of a forward solve's matvec, with values: on zeros the tensor cores and
+  // the arithmetic draw less power, and the clocks are higher than any solve sees
+  launch_fill_uniform(c->vp, n, 1, st);
+  launch_fill_uniform(c->vgx, n, 2, st);
+  launch_fill_uniform(c->vrt, n, 3, st);
+  launch_fill_uniform(c->wg, (size_t)P.U, 4, st);
   cudaEvent_t ev[5];
   for (auto &v : ev) cudaEventCreate(&v);
   double acc[5] = {0, 0, 0, 0, 0};
   BatchArgs B;
-  B.x = c->wx;
+  B.x = c->vp;
   B.g = c->wg;
   B.mode = IN_G;
   B.nrhs = nrhs;
   NearArgs A;
   A.in = B;
   A.loc = c->loc;
-  A.y = c->wy;
+  A.y = c->vv;
   A.epi = EPI_FWD;
   A.red = RED_DOT;
-  A.dot_a = c->wx;
+  A.dot_a = c->vrt;
   A.part = c->part;
   const bool tc = engine == ISG_ENGINE_TENSOR;
   if (tc) {
-    // as in a forward tensor-engine solve: the vector updates already formed g x
-    // (wx stands in for it), so P2M and the near field read it plainly and the
-    // epilogue takes x separately
+    // the vector updates already formed g x, so P2M and the near field read it plainly
+    // and the epilogue takes x separately
+    B.x = c->vgx;
     B.g = nullptr;
     B.gstride = 0;
     B.mode = IN_PLAIN;
     A.in = B;
-    A.x_epi = c->wx;
+    A.x_epi = c->vp;
     A.locmax = c->locmax;
     A.inmax = c->levmax;
   }

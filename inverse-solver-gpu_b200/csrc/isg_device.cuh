@@ -220,6 +220,8 @@ void launch_permute_g(const int *perm, const float2 *in, float2 *out, const floa
 // gx = g x per RHS (16-byte aligned vectors, even gstride)
 void launch_gmul(const float2 *x, const float2 *g, int64_t gstride, float2 *gx, int U, int nrhs, const int *active,
                  cudaStream_t st);
+// v: n values with parts uniform in [-1, 1), from the seed alone (test vectors of the timers)
+void launch_fill_uniform(float2 *v, size_t n, unsigned seed, cudaStream_t st);
 void launch_permute(const int *perm, const float2 *in, float2 *out, int U, int nrhs, bool gather, cudaStream_t st);
 
 }  // namespace isg

@@ -834,6 +834,17 @@ __global__ void k_gmul(const float2 *__restrict__ x, const float2 *__restrict__ 
   }
 }
 
+// v[i] from a hash of the seed and i (the 64-bit finaliser of SplitMix64)
+__global__ void k_fill_uniform(float2 *v, size_t n, unsigned seed) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    uint64_t z = ((uint64_t)seed << 40) + (i + 1) * 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    v[i] = make_float2((int)(z >> 32) * 0x1p-31f, (int)z * 0x1p-31f);
+  }
+}
+
 }  // namespace
 
 // Leaves per block and per thread of k_p2m.
@@ -1014,6 +1025,11 @@ void launch_permute_g(const int *perm, const float2 *in, float2 *out, const floa
                       int U, int nrhs, cudaStream_t st) {
   count_launch();
   launch(k_permute_g, dim3(std::min((U + 255) / 256, 1184), nrhs), 256, 0, st, perm, in, out, g, gstride, gx, U);
+}
+
+void launch_fill_uniform(float2 *v, size_t n, unsigned seed, cudaStream_t st) {
+  count_launch();
+  k_fill_uniform<<<1184, 256, 0, st>>>(v, n, seed);
 }
 
 void launch_gmul(const float2 *x, const float2 *g, int64_t gstride, float2 *gx, int U, int nrhs, const int *active,

@@ -46,6 +46,13 @@ isg_status isg_autotune(isg_ctx *c, int nrhs, int engine, isg_stream stream) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
+  BatchArgs B;  // test vectors of a matvec, up to the multipoles
+  B.x = c->wx;
+  B.mode = IN_PLAIN;
+  B.nrhs = nrhs;
+  launch_fill_uniform(c->wx, (size_t)nrhs * P.U, 1, st);
+  launch_p2m(P, B, c->mul, st);
+  for (int i = P.L - 2; i >= 2; i--) launch_m2m(P, i, c->mul, nrhs, nullptr, st);
   for (int i = 2; i < P.L; i++) {  // M2L, accumulating from level 3 on as in the matvec
     DevLevel &d = P.lv[i];
     int best = 0;
@@ -86,9 +93,7 @@ isg_status isg_autotune(isg_ctx *c, int nrhs, int engine, isg_stream stream) {
   }
   if (engine == ISG_ENGINE_TENSOR && tc_available(c)) {
     NearArgs A;
-    A.in.x = c->wx;
-    A.in.nrhs = nrhs;
-    A.in.mode = IN_PLAIN;
+    A.in = B;
     A.loc = c->loc;
     A.y = c->wy;
     A.epi = EPI_G;
