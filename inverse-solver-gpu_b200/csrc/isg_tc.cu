@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearArgs A, co
       float s1, s2, p;
       np_scales(A, rhs, s1, s2, p);
       const float inv = 1.f / p;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNear));
+      // a lane whose wait expired writes nothing, but takes part in the shuffles below
+      const bool ok = mbar_wait_or(tfull + set, (it >> 1) & 1, abort, A.err, kErrNear);
       tc_fence_after();
       const size_t rbase = (size_t)rhs * A.U;
       const float *gf = A.g ? (const float *)(A.g + rhs * A.gstride) : nullptr;
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearArgs A, co
           live = 0;
 #pragma unroll
           for (int j = 0; j < 8; j++) {
-            const bool lv = ok && lyb + ch < A.nleaf && tx0 + j < A.nleaf;
+            const bool lv = lyb + ch < A.nleaf && tx0 + j < A.nleaf;
             live |= lv ? 1u << j : 0u;
             const int fi = fidx(ch, j);
             xv[j] = (need_x && lv) ? xr[fi] : 0.f;
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(kNpThreads, 1) k_tc_near_pipe(TcNearArgs A, co
             } else if (A.epi == EPI_CONJ) {
               v = odd ? -o : o;
             }
-            yr[fidx(ch, j)] = v;
+            if (ok) yr[fidx(ch, j)] = v;
             if (A.red == RED_DOT) {  // conj(a) y
               const float vp = __shfl_xor_sync(0xffffffffu, v, 1);
               q0.add_prod(j, av[j], v);
