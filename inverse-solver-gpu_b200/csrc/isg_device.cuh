@@ -78,8 +78,8 @@ struct DevPlan {
 // 256 x 9 adjoint 147 -> 115 us, a 128 x 128 x 32 iteration 249 -> 229).  Every such
 // kernel calls grid_wait() before it touches anything an earlier kernel wrote or
 // reads: it returns once the kernel before, which waited in its turn, has finished.
-// The result is 0 and goes into the block index, so that no load that depends on it
-// can move ahead.  No kernel lets the next one in earlier (griddepcontrol.launch_
+// The result is 0 and goes into the block index (or the pointers, k_near), so that no
+// load that depends on it can move ahead.  No kernel lets the next one in earlier (griddepcontrol.launch_
 // dependents): blocks that wait beside a large M2L slow it down (M2L + L2L at 1024 x
 // 1024 x 64 1368 -> 1575 us).
 __device__ __forceinline__ int grid_wait() {

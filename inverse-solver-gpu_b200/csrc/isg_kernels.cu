@@ -609,7 +609,10 @@ __global__ void __launch_bounds__(64 * TY, TX == 8 ? 0 : 2) k_near(
     const float2 *__restrict__ dot_a, double *__restrict__ part, int nleaf, int U, int tiles_x, int tiles_total) {
   constexpr int kHalo = (TY + 2) * (TX + 2), kThreads = 64 * TY;
   constexpr int kStages = near_stages(TX), kRows = near_rows(TX);
-  const int rhs = blockIdx.y + grid_wait();
+  // the wait's zero goes into the pointers: in the index it costs registers that 4 x 8 leaves
+  // do not have (1024 x 1024 x 64 8136 us, 128 x 128 x 32 92; so 7987 and 88)
+  const int rhs = blockIdx.y, z = grid_wait();
+  x += z, g += z, active += z, loc_leaf += z, dot_a += z;
   if (inactive(active, rhs)) return;
   extern __shared__ __align__(16) float2 sm[];
   float2 *ring = sm;                              // [kStages][kRows][64]

@@ -73,9 +73,10 @@ def test_mma_warps_branch_on_votes():
     assert not bad, bad
 
 
-def test_waits_for_the_kernel_before_reach_every_index():
+def test_waits_for_the_kernel_before_reach_every_address():
     """Read-only loads may be moved ahead of griddepcontrol.wait unless their address depends
-    on it: the block index that grid_wait()'s zero goes into is not read again without it."""
+    on it: grid_wait()'s zero goes into the block index, which is not read again without it,
+    or into every pointer to what an earlier kernel may have written."""
     kernels, bad = 0, []
     for path in SOURCES:
         code = _code(path)
@@ -86,7 +87,12 @@ def test_waits_for_the_kernel_before_reach_every_index():
                 continue
             kernels += 1
             index = re.search(r"(blockIdx\.[xyz]) \+ grid_wait\(\)", body)
-            if not index or body.count(index.group(1)) != 1:
-                bad.append((os.path.basename(path), body[body.index("(", 40) - 40:][:60]))
+            ok = index and body.count(index.group(1)) == 1
+            if not index and re.search(r"\bz = grid_wait\(\);", body):
+                args = re.findall(r"const (?:float2|int) \*__restrict__ (\w+)", body[:body.index("{")])
+                tables = {"nearW", "basisT"}
+                ok = len(args) > 2 and all(re.search(r"\b%s \+= z\b" % p, body) for p in args if p not in tables)
+            if not ok:
+                bad.append((os.path.basename(path), body[:body.index("{")][-60:]))
     assert kernels >= 20
     assert not bad, bad
