@@ -32,23 +32,23 @@ TOL = {False: dict(out=1e-4, loss=1e-4, grad=1e-3, block=1e-2),
        True: dict(out=3e-2, loss=3e-2, grad=5e-2, block=2e-1)}
 
 
-@pytest.mark.parametrize("tensor", [False, True])
-def test_fno_forward_loss_and_gradient_match_the_oracle(tensor):
+def _match_the_oracle(level, C, M, L, S, n, scale, tensor):
+    """Outputs, loss and gradient of n samples in batches of S against the FP64 oracle,
+    parameters normal with the given standard deviation."""
     from _oracle import Oracle
-    C, M, L, S = 4, 3, 2, 2
     t = TOL[tensor]
-    s = isg.Solver(3, numrx=16, max_rhs=4, device=0)  # 32 x 32 pixels
+    s = isg.Solver(level, numrx=16, max_rhs=4, device=0)
     s.setup_gpu()
-    orc = Oracle(3, numrx=16)
+    orc = Oracle(level, numrx=16)
     um = s.host_table("unkmap")
     s.fno_create(width=C, modes=M, layers=L, batch=S, seed=5, tensor=tensor)
     o = FnoOracle(N=s.side, C=C, M=M, L=L, k0=float(s.opts.k0))
     assert isg.lib().isg_fno_param_count(s._h) == o.nparam
     rng = np.random.default_rng(11)
-    p = rng.normal(0, 0.3, o.nparam).astype(np.float32)
+    p = rng.normal(0, scale, o.nparam).astype(np.float32)
     s.fno_set_params(p)
     assert np.array_equal(s.fno_params(0), p)
-    n, U = 3, s.numunk
+    U = s.numunk
     chi = np.stack([s.phantom(seed=40 + j, count=2, eps=(1.2, 1.8), tand_max=0.1) for j in range(n)])
     G = (2 * np.pi) ** 2 * chi
     B = np.stack([np.exp(1j * 2 * np.pi * rng.uniform() * np.arange(U) / U) for _ in range(n)])
@@ -71,6 +71,23 @@ def test_fno_forward_loss_and_gradient_match_the_oracle(tensor):
     # tree order is the same network on reordered vectors
     xt = s.fno_apply(cuda(s.raster_to_tree(G)), cuda(s.raster_to_tree(B)), order=isg.ORDER_TREE).cpu().numpy()
     assert rel(xt, s.raster_to_tree(x)) < 1e-6
+
+
+@pytest.mark.parametrize("tensor", [False, True])
+def test_fno_forward_loss_and_gradient_match_the_oracle(tensor):
+    _match_the_oracle(3, C=4, M=3, L=2, S=2, n=3, scale=0.3, tensor=tensor)  # 32 x 32 pixels
+
+
+# What larger grids and models reach: rows of the y transform staged in several passes, with a
+# remainder from 89 modes on, and its outputs in several blocks, the last one partly filled
+# (2 M^2 = 288 and 18432); bias sums and weight gradients split over the pixels; 136 KB of
+# weights and inputs in the mode mix.  The parameters keep a layer's gain near one (0.3 at
+# width 4), and every tolerance counts roundings, whatever the size.
+@pytest.mark.parametrize("level,C,M,L,S,n,tensor", [(5, 5, 12, 2, 2, 3, False), (5, 5, 12, 2, 2, 3, True),
+                                                     (6, 2, 96, 1, 2, 2, False), (4, 128, 3, 2, 3, 3, False),
+                                                     (4, 128, 3, 2, 3, 3, True)])
+def test_fno_large_shapes_match_the_oracle(level, C, M, L, S, n, tensor):
+    _match_the_oracle(level, C, M, L, S, n, scale=0.6 / C ** 0.5, tensor=tensor)
 
 
 @pytest.mark.parametrize("tensor", [False, True])
