@@ -48,7 +48,7 @@ def test_tensor_near_field_items_match_the_plain_engine(level, nrhs):
     x, g = _rand(nrhs, s.numunk, 4), _rand(nrhs, s.numunk, 5)
     for herm in (False, True):
         for gg in (g, g[0]):
-            for order in (isg.ORDER_TREE, isg.ORDER_BLOCKED):
+            for order in (isg.ORDER_TREE, isg.ORDER_BLOCKED, isg.ORDER_RASTER):
                 a = s.matvec(x, gg, hermitian=herm, order=order, engine=isg.ENGINE_TENSOR)
                 b = s.matvec(x, gg, hermitian=herm, order=order)
                 # 3xFP16 split products: 2^-22 per term against FP32's 2^-24, both over ~650 terms
