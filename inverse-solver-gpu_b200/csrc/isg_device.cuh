@@ -75,13 +75,13 @@ struct DevPlan {
 // Programmatic dependent launch.  The kernels of a matvec and of a BiCGSTAB
 // iteration are launched so that the next one's blocks come up as this one's leave:
 // launch, barrier set-up, TMEM allocation and static tables then overlap (a 256 x
-// 256 x 9 adjoint 147 -> 115 us, a 128 x 128 x 32 iteration 249 -> 229).  Every such
+// 256 x 9 adjoint 161 -> 130 us, a 128 x 128 x 32 iteration 249 -> 229).  Every such
 // kernel calls grid_wait() before it touches anything an earlier kernel wrote or
 // reads: it returns once the kernel before, which waited in its turn, has finished.
 // The result is 0 and goes into the block index (or the pointers, k_near), so that no
-// load that depends on it can move ahead.  No kernel lets the next one in earlier (griddepcontrol.launch_
-// dependents): blocks that wait beside a large M2L slow it down (M2L + L2L at 1024 x
-// 1024 x 64 1368 -> 1575 us).
+// load that depends on it can move ahead.  No kernel lets the next one in earlier
+// (griddepcontrol.launch_dependents): blocks that wait beside a large M2L slow it down
+// (M2L + L2L at 1024 x 1024 x 64 on zero vectors 1368 -> 1575 us).
 __device__ __forceinline__ int grid_wait() {
   int z;
   asm volatile("griddepcontrol.wait;\n mov.u32 %0, 0;\n" : "=r"(z)::"memory");

@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(kM2lThreads, NC == 1 ? 3 : 2) k_m2l(M2lArgs A)
 // worked out the ring's address.  Each thread then walks the window once with
 // its kTileOut x 4 accumulators live: the band weights (and the L2L shift
 // phases) are the same for every thread of the block, so each staged value
-// feeds 36 FMAs from registers.  Outputs go back through
-// shared memory so that every ring is written in runs of tb.out samples.
+// feeds 36 FMAs from registers.  Outputs go back through shared memory so that
+// every ring is written in runs of tb.out samples.
 struct TileArgs {
   const float2 *src;
   float2 *dst;
@@ -303,16 +303,16 @@ struct TileArgs {
 };
 
 // Shared-memory carve-up of one tiled block (float2 units, 16-byte aligned parts).
-// With dup, the weights are stored as (w, w) pairs and each shift phase s as
-// (s.x, s.x, -s.y, s.y), the operands of packed FP32 pair arithmetic.
+// The weights are stored as (w, w) pairs and each shift phase s as (s.x, s.x, -s.y,
+// s.y), the operands of packed FP32 pair arithmetic.
 struct TileSmem {
   size_t win, w, sh, src, dst, total;
-  __host__ __device__ TileSmem(int wmax, int ld, int out, int nsrc, int ndst, size_t out_tile, bool dup = false) {
+  __host__ __device__ TileSmem(int wmax, int ld, int out, int nsrc, int ndst, size_t out_tile) {
     auto up2 = [](size_t x) { return (x + 1) & ~(size_t)1; };
     win = 0;
     w = up2(((size_t)wmax * ld > out_tile ? (size_t)wmax * ld : out_tile));
-    sh = w + up2((size_t)wmax * out / (dup ? 1 : 2));
-    src = sh + (size_t)wmax * (dup ? 8 : 4);
+    sh = w + up2((size_t)wmax * out);
+    src = sh + (size_t)wmax * 8;
     dst = src + nsrc;
     total = dst + ndst;
   }
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(128) k_l2l_tile(TileArgs A) {
   const int cols = A.cols, TO = A.tb.out, tile = blockIdx.y, c0 = (blockIdx.x + grid_wait()) * cols;
   if (!any_active_column(A, c0)) return;
   const int a0 = A.tb.a0[tile], wl = A.tb.wl[tile], ld = cols + 1;
-  const TileSmem L(A.tb.wmax, ld, TO, cols, 4 * cols, (size_t)4 * TO * ld, true);
+  const TileSmem L(A.tb.wmax, ld, TO, cols, 4 * cols, (size_t)4 * TO * ld);
   const float2 **sp = (const float2 **)(sm + L.src);
   float2 **dp = (float2 **)(sm + L.dst);
   float4 *sw = (float4 *)(sm + L.w);   // [wl][TO / 2]: (w, w, w', w') pairs
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(128) k_l2l_tile(TileArgs A) {
 // and reads a parent's value once for four; the shifts of opposite children are
 // conjugates of each other.  On small launches the time is one thread's chain of
 // loads, which S = 1 and C = 1 keep shortest.  M2M of 1024 x 1024 x 16, all levels:
-// 450 us, tiled through shared memory 642; x 1: 62 / 94.
+// 463 us, tiled through shared memory 645; x 64: 1703 / 2429.
 struct DirectArgs {
   const float2 *src;  // input level, one RHS' block every mp elements
   float2 *dst;
@@ -961,7 +961,7 @@ void launch_l2l(const DevPlan &P, int lvl, float2 *loc, int nrhs, const int *act
   }
   const int cap = (c.l2l_cols > 0 && 4 * nrhs >= P.tuned_nrhs) ? c.l2l_cols : kL2lCols;
   const TileArgs A = tile_args(loc, loc, P.mp, p.off, c.off, p.n, p.ns, c.ns, nrhs, c.at, p.shlT, cap, active);
-  const TileSmem L(c.at.wmax, A.cols + 1, c.at.out, A.cols, 4 * A.cols, (size_t)4 * c.at.out * (A.cols + 1), true);
+  const TileSmem L(c.at.wmax, A.cols + 1, c.at.out, A.cols, 4 * A.cols, (size_t)4 * c.at.out * (A.cols + 1));
   const size_t smem = L.total * sizeof(float2);
   count_launch();
   launch(k_l2l_tile, dim3((A.ncols + A.cols - 1) / A.cols, c.at.tiles), A.cols * (c.at.out / kTileOut), smem, st, A);

@@ -69,7 +69,7 @@ __device__ __forceinline__ float cabs1(float2 v) { return fmaxf(fabsf(v.x), fabs
 // Shared memory bounds the large items: the MMAs read 12 KB for their 128 cycles, and
 // tensor loads, weight stages and converters come on top.  Both operand kinds are
 // written at the halo's pitch of 10 leaves and read in an order that keeps a phase's
-// lanes on different banks: 1024 x 1024 x 64 929 -> 883 us, 256 x 256 x 64 94.1 -> 89.6
+// lanes on different banks: 1024 x 1024 x 64 1185 -> 1086 us, 256 x 256 x 64 105.5 -> 101.5
 // (L2P stages at a pitch of 8 leaves were 4-way conflicts).
 constexpr int kNpKC = 4;                                       // 8-real K-chunks per A-stage
 constexpr int kNpHaloSplit = kHR * kNpKC * kHC * 16;           // 21760: one FP16 split of a halo K-group
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kP2mThreads, 1) k_tc_p2m_pipe(TcP2mArgs A) {
         if (u < kP2mUnits && leaf0 + m < A.nleaves) {
           // the 8 leaves of a load phase, 512 bytes apart, take 8 different chunks, the
           // upper four of them their second half first: all banks, no conflict (with one
-          // chunk for all, 4-way: P2M of 1024 x 1024 x 64 258 us, this 237)
+          // chunk for all, 4-way: P2M of 1024 x 1024 x 64 256 us, this 249)
           const int odd = (c >> 2) & 1;
           const float4 x0 = zst[m * 32 + 2 * c + odd], x1 = zst[m * 32 + 2 * c + 1 - odd];
           const float4 a0 = odd ? x1 : x0, a1 = odd ? x0 : x1;

@@ -19,13 +19,13 @@
 // levels whose rings have at most 128 samples (the leaves and their parents,
 // most of the tree's samples): persistent CTAs keep the level's whole
 // anterpolation matrix (128 child samples x the parent ring, FP16 hi/lo) in
-// shared memory and walk items of 32 (or 16) parents.  An item's parent rings
-// arrive by cp.async while the previous item is multiplied and written; each
+// shared memory and walk items of 32, 16 or 8 parents.  An item's parent rings
+// arrive by a bulk copy while the previous item is multiplied and written; each
 // CTA forms the four shifted copies shl[q][j] z[j] of every ring directly in
 // the FP16 hi/lo operand layout (256 MMA columns = 32 parents x 4 children x
 // re, im), and the epilogue writes each child ring from TMEM with the child
 // sample on the lane, so every store is coalesced.  Coarser levels keep the
-// SIMT tiled kernel.
+// SIMT kernels.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -79,7 +79,7 @@ struct BandArgs {
   size_t mp;
   int n_p, ns_in, ns_out;
   const float2 *shift;  // shiftmul of the parent level, [4][ns_p]
-  const uint8_t *A;     // K-chunks of this transition (hi then lo, 32 KB each)
+  const uint8_t *A;     // K-chunks of this transition (hi then lo, 16 KB each)
   const int *kw0, *nchunk, *chunk0;  // per M-tile: window start (-1: whole ring), chunks, first chunk
   float inv_a;
   int nparents, ncols;  // ncols = parents x RHS
@@ -131,8 +131,8 @@ __device__ __forceinline__ void ring_load8(const BandArgs &A, const RingRef &r, 
 // through two buffers: while the tensor core multiplies one chunk, the next one's
 // weights arrive by a bulk copy and its samples, read a chunk ahead into registers,
 // are split into the other buffer.  (Chunks of 64 through one buffer, every step
-// waiting for the one before: M2M of 1024 x 1024 x 64, all levels, 564 us, this 514;
-// x 16 171 / 155.)
+// waiting for the one before: M2M of 1024 x 1024 x 64, all levels, 590 us, this 537;
+// x 16 176 / 160.)
 __global__ void __launch_bounds__(256, 3) k_tc_band(BandArgs A) {
   extern __shared__ __align__(1024) char sm[];
   uint64_t *abar = (uint64_t *)(sm + 2 * kBandBuf);  // [2] weights landed
@@ -746,8 +746,8 @@ struct Transition {
   bool ok = false;
 };
 
-// Packs reals(row, k0 .. k0+63) of a [128 x K] block as FP16 hi then lo in the
-// K-major core-matrix layout (SBO = 8 chunks x 128 B, LBO = 128 B).
+// Packs reals(row, k0 .. k0+31) of a [128 x K] block as FP16 hi then lo in the
+// K-major core-matrix layout (SBO = 4 chunks x 128 B, LBO = 128 B).
 template <class F>
 void pack_chunk(std::vector<uint8_t> &buf, size_t at, int k0, double scale, F real_at) {
   __half *hi = (__half *)(buf.data() + at), *lo = (__half *)(buf.data() + at + kAHalf);
@@ -1096,7 +1096,7 @@ bool band_l2l(isg_ctx *c, int lvl, float2 *loc, int nrhs, const int *active, cud
   A.kc_magic = T.kc_magic;
   A.nparents = p.n * p.n;
   // fewer parents per item while the GPU has fewer items than SMs (L2L and M2L of
-  // 128 x 128 x 32: 36.4 us, L2L with the SIMT kernels 46.4)
+  // 128 x 128 x 32: 38.6 us, L2L with the SIMT kernels 47.0)
   A.ppi = T.ppi;
   while (A.ppi > 8 && A.nparents / A.ppi * nrhs < c->band->sms) A.ppi /= 2;
   A.A = T.A;
